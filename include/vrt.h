@@ -104,13 +104,14 @@ enum {
 /* Launch-shape knobs of the wavefront path tracer; 0 keeps the default. */
 typedef struct VrtTuning {
   int refill_min;             /* idle lanes of a warp that trigger a refill    */
-  int trace_blocks_per_sm;    /* persistent DDA blocks per SM (0 = max)        */
+  int trace_blocks_per_sm;    /* persistent DDA blocks (of 128 threads) per SM
+                                 (0 = max)                                     */
   int shade_blocks_per_sm;    /* shading kernel blocks per SM                  */
-  int trace_variant;          /* tracer variant: (DDA iterations per pass of the
-                                 warp bookkeeping, min blocks per SM) =
-                                 0: (8,5) default, 1: (6,5), 2: (6,4), 3: (4,4),
-                                 4: (2,1), 5: (1,1); 6, 7, 8: (8,5) with the
-                                 step loop unrolled 1, 2, 4 times (not 8)        */
+  int trace_variant;          /* tracer variant: (rounds of transitions per pass
+                                 of the warp bookkeeping, DDA steps per round,
+                                 min blocks per SM) = 0: (3,5,9) default,
+                                 1: (4,4,9), 2: (3,4,8), 3: (4,3,9), 4: (2,4,9),
+                                 5: (8,1,9), 6: (4,3,10), 7: (3,6,9), 8: (3,6,8) */
   int atrous_tile_rows;       /* a-trous output tile rows: 0 (default) or 8 = 8
                                  at every step, 16 = 16 at steps 1-2 and 8 at
                                  step 4                                          */

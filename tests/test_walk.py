@@ -1,0 +1,57 @@
+"""The queue tracer's brick -> voxel walk (csrc/dda_walk.cuh) against the
+per-thread nested loops (the path-trace megakernel, itself held to the CPU
+oracle by the parity tests): the same frame through both, at the grid sizes
+where the walk's packed words change shape -- one brick, grids whose side is no
+power of two, and a grid of more than 128^3 bricks, which takes the tracer's
+wide form -- and from cameras that start outside the world, on voxel edges and
+that look along an axis.  Images and counters must be equal bit for bit.
+"""
+import math
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx(vrt):
+    c = vrt.Context(0)
+    yield c
+    c.close()
+
+
+def _world(vrt, ctx, n):
+    """Boxes of voxels over an empty grid (built by edits, so that the largest grid needs no host world)."""
+    sc = vrt.Scene(ctx, np.zeros(n ** 3, np.uint32), n)
+    rng = np.random.default_rng(n)
+    sc.edit_box(0, 0, 0, n - 1, max(n // 16 - 1, 0), n - 1, 0x0080A0C0)          # floor
+    for _ in range(40):
+        lo = rng.integers(0, n, 3)
+        hi = np.minimum(lo + rng.integers(0, max(n // 8, 2), 3), n - 1)
+        sc.edit_box(*map(int, lo), *map(int, hi), int(rng.integers(1, 1 << 32)))
+    return sc
+
+
+@pytest.mark.parametrize("n", [8, 24, 104, 1024, 1032])
+def test_walk_matches_nested_loops(vrt, ctx, n):
+    W, H = 96, 61
+    sc = _world(vrt, ctx, n)
+    ext = n / 16.0
+    poses = [vrt.CameraPose((ext * 0.5, ext * 0.6, ext * 0.4), 0.3, -0.2),       # inside
+             vrt.CameraPose((-0.7 * ext, ext * 1.5, -0.4 * ext), 0.8, -0.5),     # outside, looking in
+             vrt.CameraPose((ext * 0.5, ext * 0.5, ext * 0.25), 0.0, 0.0),       # on a voxel edge, along +z
+             vrt.CameraPose((ext * 0.5, ext, ext * 0.5), 0.0, -math.pi / 2)]     # on the top face, straight down
+    wave = vrt.Session(ctx, sc, W, H, keep_radiance_f32=True)
+    mega = vrt.Session(ctx, sc, W, H, keep_radiance_f32=True, path_kernel="megakernel")
+    for k, pose in enumerate(poses):
+        u = vrt.make_uniforms(pose, None, vrt.Lighting(), 11 + k, 3, 0, W, H)
+        for s in (wave, mega):
+            s.set_timing(True)
+            s.frame(u)
+        a, b = wave.stats(), mega.stats()
+        assert (a.rays, a.dda_outer, a.dda_inner, a.voxel_reads) == (b.rays, b.dda_outer, b.dda_inner, b.voxel_reads)
+        assert np.array_equal(wave.radiance_f32().view(np.uint32), mega.radiance_f32().view(np.uint32))
+        assert np.array_equal(wave.gbuffer().view(np.uint32), mega.gbuffer().view(np.uint32))
+    for o in (wave, mega, sc):
+        o.close()

@@ -17,6 +17,7 @@ namespace vrt {
 
 static_assert(sizeof(JobDev) == sizeof(JobHost), "job table layouts differ");
 static_assert(offsetof(JobDev, S) == offsetof(JobHost, vox), "job table layouts differ");
+static_assert(offsetof(JobDev, S.mw) == offsetof(JobHost, mw), "job table layouts differ");
 static_assert(offsetof(JobDev, out) == offsetof(JobHost, rad16), "job table layouts differ");
 static_assert(offsetof(JobDev, W) == offsetof(JobHost, W), "job table layouts differ");
 static_assert(offsetof(JobDev, acc_prev) == offsetof(JobHost, acc_prev), "job table layouts differ");
@@ -123,7 +124,7 @@ __global__ void __launch_bounds__(256) k_b_present(MultiJob J, uint32_t P, const
   jd.ldr[lp] = present_pixel(jd.u.params1[2], il, __ldg(jd.out.alb8 + lp), lut);
 }
 
-cudaError_t launch_batch_frame(const void* d_jobs, const uint32_t* d_firsts, int n, uint32_t P, int waves,
+cudaError_t launch_batch_frame(const void* d_jobs, const uint32_t* d_firsts, int n, int max_bg, uint32_t P, int waves,
                                const WavefrontBufs& wb, const WavefrontTuning& tune, unsigned long long* stats,
                                cudaStream_t st, uint32_t* launches, const float* present_lut, const CacheLaunch* cls,
                                int ncl, const AtrousTiles* at) {
@@ -132,10 +133,11 @@ cudaError_t launch_batch_frame(const void* d_jobs, const uint32_t* d_firsts, int
   J.firsts = d_firsts;
   J.n = n;
   J.cache_jobs = ncl;
+  J.max_bg = max_bg;
   // tail wave: as tuned; automatic (-1) = wave 2 when every job is cache-assisted (only the
   // training paths remain after the first bounce), else never
   const int tail = tune.tail_wave >= 0 ? tune.tail_wave : (ncl > 0 && ncl == n ? 2 : 0);
-  cudaError_t e = wf_launch_frame(J, P, waves, 0, wb, tune, stats, st, launches, nullptr, 0, nullptr, n, tail);
+  cudaError_t e = wf_launch_frame(J, P, waves, wb, tune, stats, st, launches, nullptr, 0, nullptr, n, tail);
   if (e != cudaSuccess) return e;
   // the cache jobs' inference, resolve and training, all jobs per launch
   if (ncl > 0 && (e = launch_cache_post(J, wf_view(wb), cls, ncl, stats, st, launches)) != cudaSuccess) return e;

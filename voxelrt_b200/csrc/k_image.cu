@@ -144,7 +144,7 @@ __global__ void __launch_bounds__(256) k_present_check(const float* __restrict__
 
 // ---------------------------------------------------------------------------
 // Brick build (scene.js:411-433): one block per brick, one warp per mask
-// word.  Word w holds bits 32w..32w+31 = lz = w/2, ly = 4(w&1) + lane/8,
+// word (the masks are laid out over the padded grid).  Word w holds bits 32w..32w+31 = lz = w/2, ly = 4(w&1) + lane/8,
 // lx = lane%8, so a warp ballot over "voxel != 0" is the word itself.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(512) k_build_bricks(const uint32_t* __restrict__ vox, int N, int BG,
@@ -160,17 +160,29 @@ __global__ void __launch_bounds__(512) k_build_bricks(const uint32_t* __restrict
   const uint32_t v = vox[x + y * N + z * (size_t)N * N];
   const uint32_t word = __ballot_sync(0xffffffffu, v != 0u);
   const size_t bi = (size_t)bx + (size_t)by * BG + (size_t)bz * BG * BG;
-  if (lane == 0) masks[bi * 16 + w] = word;
+  const size_t ci = (size_t)(bx + 1) + (size_t)(BG + 2) * ((size_t)(by + 1) + (size_t)(BG + 2) * (bz + 1));
+  if (lane == 0) masks[ci * 16 + w] = word;
   const int occ = __syncthreads_or(word != 0u);
   if (threadIdx.x == 0) bricks[bi] = occ ? 1u : 0u;
 }
 
-// Occupancy bitmap: bit bi = bricks[bi] != 0.
-__global__ void k_build_bits(const uint32_t* __restrict__ bricks, int nb, uint32_t* __restrict__ bits) {
+// Occupancy bitmaps: bit bi of bits = bricks[bi] != 0, and the same over the
+// grid padded by one cell on each side, whose border bits are set (pad).
+__global__ void k_build_bits(const uint32_t* __restrict__ bricks, int BG, uint32_t* __restrict__ bits,
+                             uint32_t* __restrict__ pad) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int nb = BG * BG * BG, P = BG + 2, np = P * P * P;
   const bool occ = i < nb && bricks[i] != 0u;
   const uint32_t word = __ballot_sync(0xffffffffu, occ);
   if ((threadIdx.x & 31) == 0 && i < ((nb + 31) & ~31)) bits[i >> 5] = word;
+  bool pocc = false;
+  if (i < np) {
+    const int x = i % P - 1, y = (i / P) % P - 1, z = i / (P * P) - 1;
+    pocc = x < 0 || y < 0 || z < 0 || x >= BG || y >= BG || z >= BG ||
+           bricks[(size_t)x + (size_t)BG * ((size_t)y + (size_t)BG * z)] != 0u;
+  }
+  const uint32_t pword = __ballot_sync(0xffffffffu, pocc);
+  if ((threadIdx.x & 31) == 0 && i < ((np + 31) & ~31)) pad[i >> 5] = pword;
 }
 
 __global__ void k_fill_box(uint32_t* __restrict__ vox, int N, int x0, int y0, int z0, int sx, int sy, int sz,
@@ -196,13 +208,13 @@ cudaError_t launch_build_bricks(const SceneDev& s, int bx0, int by0, int bz0, in
   const int nbx = bx1 - bx0 + 1, nby = by1 - by0 + 1, nbz = bz1 - bz0 + 1;
   if (nbx <= 0 || nby <= 0 || nbz <= 0) return cudaSuccess;
   const long nblocks = (long)nbx * nby * nbz;
-  k_build_bricks<<<(unsigned)nblocks, 512, 0, st>>>(s.vox, s.N, s.BG, s.bricks, s.masks, bx0, by0, bz0, nbx, nby);
+  k_build_bricks<<<(unsigned)nblocks, 512, 0, st>>>(s.vox, s.N, s.BG, s.bricks, s.cells + mask_word(s.BG), bx0, by0, bz0, nbx, nby);
   return cudaGetLastError();
 }
 
 cudaError_t launch_build_bits(const SceneDev& s, cudaStream_t st) {
-  const int nb = s.BG * s.BG * s.BG;
-  k_build_bits<<<(nb + 255) / 256, 256, 0, st>>>(s.bricks, nb, s.bits);
+  const int np = (s.BG + 2) * (s.BG + 2) * (s.BG + 2);
+  k_build_bits<<<(np + 255) / 256, 256, 0, st>>>(s.bricks, s.BG, s.bits, s.cells);
   return cudaGetLastError();
 }
 

@@ -1706,11 +1706,6 @@ static SingleJob restir_job(const SceneDev& s, const VrtUniforms& uu, float fcla
   return job;
 }
 
-static int occ_smem(const SceneDev& s) {
-  const int smem_occ = (int)(occ_words(s.BG) * sizeof(uint32_t));
-  return smem_occ <= (int)kMaxSmemOccBytes ? smem_occ : 0;
-}
-
 cudaError_t launch_restir_initial_wavefront(const SceneDev& s, const VrtUniforms& uu, float fclamp, int W, int H,
                                             const PathOut& out, const RestirBufs& rb, const WavefrontBufs& wb,
                                             const WavefrontTuning& tune, cudaStream_t st, uint32_t* launches,
@@ -1718,9 +1713,8 @@ cudaError_t launch_restir_initial_wavefront(const SceneDev& s, const VrtUniforms
   const SingleJob job = restir_job(s, uu, fclamp, W, H, out);
   const RestirWf r{(uint4*)rb.resA, (uint2*)rb.direct, (float4*)rb.scratch, W, H, nullptr, nullptr, nullptr, nullptr};
   const uint32_t P = (uint32_t)W * (uint32_t)H;
-  const int smem = occ_smem(s);
   unsigned long long* stats = out.stats;
-  return wf_run_waves(job, P, (int)job.u.params0[1] + 2, smem, wb, tune, stats, st, launches, trace_ev,
+  return wf_run_waves(job, P, (int)job.u.params0[1] + 2, wb, tune, stats, st, launches, trace_ev,
                       max_timed_waves, timed_waves, [&](const WfDev& b, int w, int sblocks) {
                         if (w == 0) k_wf_restir_primary<<<sblocks, 256, 0, st>>>(job, r, P, b, stats);
                         else k_wf_restir_wave<<<sblocks, 256, 0, st>>>(job, r, b, w);
@@ -1738,14 +1732,13 @@ cudaError_t launch_restir_unified_wavefront(const SceneDev& s, const VrtUniforms
   float4* sc = (float4*)rb.scratch;
   const RestirWf r{(uint4*)rb.resA, (uint2*)rb.direct, sc, W, H, sc + P, sc + 2 * (size_t)P, sc + 3 * (size_t)P,
                    sc + 4 * (size_t)P};
-  const int smem = occ_smem(s);
   // x1's three sequential rays, then one wave per estimateLo vertex
   auto shade = [&](const WfDev& b, int w, int sblocks) {
     if (w == 0) k_wf_unified_primary<<<sblocks, 256, 0, st>>>(R, r, P, b);
     else k_wf_unified_wave<<<sblocks, 256, 0, st>>>(R, r, b, w);
     return cudaGetLastError();
   };
-  return wf_run_waves<SingleJob, decltype(shade), true>(job, P, (int)job.u.params0[1] + 4, smem, wb, tune, out.stats,
+  return wf_run_waves<SingleJob, decltype(shade), true>(job, P, (int)job.u.params0[1] + 4, wb, tune, out.stats,
                                                         st, launches, trace_ev, max_timed_waves, timed_waves, shade);
 }
 
@@ -1784,14 +1777,9 @@ cudaError_t launch_restir_spatial_wavefront(const SceneDev& s, const VrtUniforms
   else k_restir_spatial_select<false><<<grid, 256, 0, st>>>(R, b, wave);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   const int sms = wf_sm_count();
-  const int smem = occ_smem(s);
-  const int refill = tune.refill_min > 0 ? tune.refill_min : 8;
-  if (smem > 0)
-    e = wf_dispatch_trace<SingleJob, true, true>(tune.trace_variant, job, smem, tune.trace_blocks_per_sm, sms, b, wave,
-                                                 0, refill, out.stats, st);
-  else
-    e = wf_dispatch_trace<SingleJob, false, true>(tune.trace_variant, job, 0, tune.trace_blocks_per_sm, sms, b, wave,
-                                                  0, refill, out.stats, st);
+  const int refill = tune.refill_min > 0 ? tune.refill_min : 12;
+  e = wf_dispatch_trace<SingleJob, true>(tune.trace_variant, job, tune.trace_blocks_per_sm, sms, b, wave, 0, refill,
+                                         out.stats, st);
   if (e != cudaSuccess) return e;
   k_restir_spatial_resolve<<<sms * 8, 256, 0, st>>>(R, b, wave);
   if (launches) *launches += 3;

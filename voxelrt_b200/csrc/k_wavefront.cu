@@ -23,6 +23,7 @@
 // The per-path arithmetic (RNG draws, shading, order of radiance sums) is
 // exactly the megakernel's, so results are bit-identical to it and to the
 // CPU oracle.
+#include "trace_kernel.cuh"
 #include "wavefront_core.cuh"
 #include <algorithm>
 #include <cstring>
@@ -58,7 +59,7 @@ void carve_wavefront(void* mem, size_t P, int max_waves, WavefrontBufs& wb, int 
 static SingleJob make_job(const SceneDev& s, const VrtUniforms& uu, float fclamp, int W, int H, const PathOut& out) {
   SingleJob job;
   std::memcpy(&job.u, &uu, sizeof(Uni));
-  job.S.vox = s.vox; job.S.masks = s.masks; job.S.bits = s.bits; job.S.N = s.N; job.S.BG = s.BG;
+  job.S = to_dscene(s);
   job.out.rad16 = (uint2*)out.rad16;
   job.out.rad32 = (float4*)out.rad32;
   job.out.alb8 = out.alb8;
@@ -78,13 +79,11 @@ cudaError_t launch_wavefront(const SceneDev& s, const VrtUniforms& uu, float fcl
   if (cache) job.cc = cache->cd;
   // cache-assisted frames run as many waves as their training paths need
   const int waves = (job.cc.on ? (int)job.cc.train_bounces : (int)job.u.params0[1]) + 2;
-  const int smem_occ = (int)(occ_words(s.BG) * sizeof(uint32_t));
-  const int smem = smem_occ <= 64 * 1024 ? smem_occ : 0;
   // cache frames: every path but the training paths ends at its first bounce
   // (wave 1), so by default the few paths left after it run to their end one
   // thread each
   const int tail = tune.tail_wave >= 0 ? tune.tail_wave : (job.cc.on ? 2 : 0);
-  cudaError_t e = wf_launch_frame(job, (uint32_t)(W * H), waves, smem, wb, tune, out.stats, st, launches, trace_ev,
+  cudaError_t e = wf_launch_frame(job, (uint32_t)(W * H), waves, wb, tune, out.stats, st, launches, trace_ev,
                                   max_timed_waves, timed_waves, 1, tail);
   if (e != cudaSuccess || !job.cc.on) return e;
   if (cache_ev && (e = cudaEventRecord(cache_ev[0], st)) != cudaSuccess) return e;

@@ -24,7 +24,9 @@ VRT_DI const uint32_t* stage_occupancy(const DScene& S, uint32_t* s_occ) {
 
 inline DScene to_dscene(const SceneDev& s) {
   DScene d;
-  d.vox = s.vox; d.masks = s.masks; d.bits = s.bits; d.N = s.N; d.BG = s.BG;
+  d.vox = s.vox; d.cells = s.cells; d.bits = s.bits; d.N = s.N; d.BG = s.BG;
+  d.rP = recip_pad(s.BG); d.rP2 = recip_pad2(s.BG);
+  d.mw = (uint32_t)mask_word(s.BG); d.pad = 0u;
   return d;
 }
 

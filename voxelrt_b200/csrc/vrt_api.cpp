@@ -254,7 +254,7 @@ static int scene_alloc(VrtCtx* ctx, int N, VrtScene** out) {
   const size_t nv = (size_t)N * N * N, nb = (size_t)s->dev.BG * s->dev.BG * s->dev.BG;
   int r = dev_alloc(ctx, (void**)&s->dev.vox, nv * 4, &s->bytes);
   if (!r) r = dev_alloc(ctx, (void**)&s->dev.bricks, nb * 4, &s->bytes);
-  if (!r) r = dev_alloc(ctx, (void**)&s->dev.masks, nb * 64, &s->bytes);
+  if (!r) r = dev_alloc(ctx, (void**)&s->dev.cells, cell_bytes(s->dev.BG), &s->bytes);
   if (!r) r = dev_alloc(ctx, (void**)&s->dev.bits, occ_words(s->dev.BG) * 4 + 128, &s->bytes);
   if (r) {
     std::string keep = g_err;
@@ -262,8 +262,31 @@ static int scene_alloc(VrtCtx* ctx, int N, VrtScene** out) {
     g_err = keep;
     return r;
   }
+  // full masks everywhere; building or uploading the bricks overwrites all but the border
+  const cudaError_t e = cudaMemsetAsync(s->dev.cells, 0xff, cell_bytes(s->dev.BG), ctx->stream);
+  if (e != cudaSuccess) {
+    vrt_scene_destroy(s);
+    return fail(VRT_ERR_CUDA, "scene: %s", cudaGetErrorString(e));
+  }
   *out = s;
   return VRT_OK;
+}
+
+// The reference's brickMasks (16 words per brick, BG^3 bricks) to or from the
+// interior of the scene's padded masks.
+static cudaError_t copy_masks(const SceneDev& s, uint32_t* host, cudaMemcpyKind kind, cudaStream_t st) {
+  const size_t BG = (size_t)s.BG, P = BG + 2;
+  cudaMemcpy3DParms p = {};
+  const cudaPitchedPtr h = make_cudaPitchedPtr(host, BG * 64, BG * 64, BG);
+  const cudaPitchedPtr d = make_cudaPitchedPtr(s.cells + mask_word(s.BG), P * 64, P * 64, P);
+  const cudaPos at = make_cudaPos(64, 1, 1);
+  const bool up = kind == cudaMemcpyHostToDevice;
+  p.srcPtr = up ? h : d;
+  p.dstPtr = up ? d : h;
+  (up ? p.dstPos : p.srcPos) = at;
+  p.extent = make_cudaExtent(BG * 64, BG, BG);
+  p.kind = kind;
+  return cudaMemcpy3DAsync(&p, st);
 }
 
 int vrt_scene_upload(VrtCtx* ctx, const uint32_t* voxels, int N, VrtScene** out) {
@@ -293,7 +316,7 @@ int vrt_scene_upload_prebuilt(VrtCtx* ctx, const uint32_t* voxels, const uint32_
   cudaStream_t st = ctx->stream;
   cudaError_t e = cudaMemcpyAsync(s->dev.vox, voxels, nv * 4, cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess) e = cudaMemcpyAsync(s->dev.bricks, bricks, nb * 4, cudaMemcpyHostToDevice, st);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(s->dev.masks, brick_masks, nb * 64, cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess) e = copy_masks(s->dev, const_cast<uint32_t*>(brick_masks), cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess) e = launch_build_bits(s->dev, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) {
@@ -328,7 +351,7 @@ int vrt_scene_read(VrtScene* s, uint32_t* voxels, uint32_t* bricks, uint32_t* ma
   cudaStream_t st = s->ctx->stream;
   if (voxels) CUDA_TRY(cudaMemcpyAsync(voxels, s->dev.vox, N * N * N * 4, cudaMemcpyDeviceToHost, st));
   if (bricks) CUDA_TRY(cudaMemcpyAsync(bricks, s->dev.bricks, nb * 4, cudaMemcpyDeviceToHost, st));
-  if (masks) CUDA_TRY(cudaMemcpyAsync(masks, s->dev.masks, nb * 64, cudaMemcpyDeviceToHost, st));
+  if (masks) CUDA_TRY(copy_masks(s->dev, masks, cudaMemcpyDeviceToHost, st));
   CUDA_TRY(cudaStreamSynchronize(st));
   return VRT_OK;
 }
@@ -341,7 +364,7 @@ int vrt_scene_destroy(VrtScene* s) {
   const size_t N = s->dev.N, nb = (size_t)s->dev.BG * s->dev.BG * s->dev.BG;
   dev_free(c, s->dev.vox, N * N * N * 4, &s->bytes);
   dev_free(c, s->dev.bricks, nb * 4, &s->bytes);
-  dev_free(c, s->dev.masks, nb * 64, &s->bytes);
+  dev_free(c, s->dev.cells, cell_bytes(s->dev.BG), &s->bytes);
   dev_free(c, s->dev.bits, occ_words(s->dev.BG) * 4 + 128, &s->bytes);
   const size_t cap = s->light_cap;
   dev_free(c, s->light_words, cap * 8, &s->bytes);
@@ -532,7 +555,7 @@ int vrt_session_set_tuning(VrtSession* s, const VrtTuning* t) {
       (t->atrous_tile_rows != 0 && t->atrous_tile_rows != 8 && t->atrous_tile_rows != 16) || t->tail_wave < -1 ||
       t->tail_wave > 64)
     return fail(VRT_ERR_INVALID, "tuning out of range");
-  s->tune.refill_min = t->refill_min ? t->refill_min : 8;
+  s->tune.refill_min = t->refill_min ? t->refill_min : 12;
   s->tune.trace_blocks_per_sm = t->trace_blocks_per_sm;
   s->tune.shade_blocks_per_sm = t->shade_blocks_per_sm ? t->shade_blocks_per_sm : 32;
   s->tune.trace_variant = t->trace_variant;
@@ -1063,6 +1086,7 @@ struct VrtBatch {
   int graph_waves = -1;
   WavefrontTuning graph_tune;
   uint64_t graph_cache_sig = 0;
+  bool graph_wide = false;        // captured with the tracer of scenes over kNarrowBG
   uint32_t graph_launches = 0;
   cudaEvent_t ev_start = nullptr, ev_end = nullptr, ev_upload = nullptr;
   bool uploaded = false;
@@ -1165,7 +1189,7 @@ int vrt_batch_set_tuning(VrtBatch* b, const VrtTuning* t) {
       (t->atrous_tile_rows != 0 && t->atrous_tile_rows != 8 && t->atrous_tile_rows != 16) || t->tail_wave < -1 ||
       t->tail_wave > 64)
     return fail(VRT_ERR_INVALID, "tuning out of range");
-  b->tune.refill_min = t->refill_min ? t->refill_min : 8;
+  b->tune.refill_min = t->refill_min ? t->refill_min : 12;
   b->tune.atrous_rows = t->atrous_tile_rows;
   b->tune.trace_blocks_per_sm = t->trace_blocks_per_sm;
   b->tune.shade_blocks_per_sm = t->shade_blocks_per_sm ? t->shade_blocks_per_sm : 32;
@@ -1212,6 +1236,8 @@ static int batch_frame_impl(VrtBatch* b, const int* idx, int m, const VrtUniform
   }
   const int waves = maxB + 2;
   if (waves + 1 > b->wf.max_waves) return fail(VRT_ERR_INVALID, "bounce count %d too large for a batch", maxB);
+  int max_bg = 0;
+  for (int i = 0; i < m; i++) max_bg = std::max(max_bg, ss[(size_t)i]->scene->dev.BG);
   if (int r = set_dev(b->ctx)) return r;
   cudaStream_t st = b->ctx->stream;
   // the staging tables may still be read by the previous frame's upload
@@ -1225,8 +1251,10 @@ static int batch_frame_impl(VrtBatch* b, const int* idx, int m, const VrtUniform
     std::memset(&j, 0, sizeof j);
     const int p = parity_of(s);
     j.u = u[i];
-    j.vox = s->scene->dev.vox; j.masks = s->scene->dev.masks; j.bits = s->scene->dev.bits;
+    j.vox = s->scene->dev.vox; j.cells = s->scene->dev.cells; j.bits = s->scene->dev.bits;
     j.N = s->scene->dev.N; j.BG = s->scene->dev.BG;
+    j.rP = recip_pad(j.BG); j.rP2 = recip_pad2(j.BG);
+    j.mw = (uint32_t)mask_word(j.BG);
     j.rad16 = s->rad16; j.rad32 = s->rad32; j.alb8 = s->alb8; j.gbuf = s->gbuf[p];
     j.W = s->W; j.H = s->H; j.first = first; j.fclamp = s->fclamp;
     j.acc_prev = s->accum[1 - p]; j.acc_cur = s->accum[p]; j.gbuf_prev = s->gbuf[1 - p];
@@ -1260,12 +1288,12 @@ static int batch_frame_impl(VrtBatch* b, const int* idx, int m, const VrtUniform
   b->launches = 0;
   if (graph) {
     if (!b->gexec || b->graph_waves != waves || !same_tuning(b->graph_tune, b->tune) ||
-        b->graph_cache_sig != cache_sig) {
+        b->graph_cache_sig != cache_sig || b->graph_wide != (max_bg > kNarrowBG)) {
       batch_drop_graph(b);
       cudaGraph_t graph = nullptr;
       CUDA_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed));
       uint32_t nl = 0;
-      cudaError_t e = launch_batch_frame(b->d_jobs, b->d_firsts, m, P, waves, b->wf, b->tune, b->stats, st, &nl,
+      cudaError_t e = launch_batch_frame(b->d_jobs, b->d_firsts, m, max_bg, P, waves, b->wf, b->tune, b->stats, st, &nl,
                                          b->ctx->present_lut, cls.data(), (int)cls.size(), &at);
       cudaError_t e2 = cudaStreamEndCapture(st, &graph);
       if (e != cudaSuccess || e2 != cudaSuccess) {
@@ -1281,12 +1309,13 @@ static int batch_frame_impl(VrtBatch* b, const int* idx, int m, const VrtUniform
       b->graph_waves = waves;
       b->graph_tune = b->tune;
       b->graph_cache_sig = cache_sig;
+      b->graph_wide = max_bg > kNarrowBG;
       b->graph_launches = nl;
     }
     b->launches = b->graph_launches;
     CUDA_TRY(cudaGraphLaunch(b->gexec, st));
   } else {
-    CUDA_TRY(launch_batch_frame(b->d_jobs, b->d_firsts, m, P, waves, b->wf, b->tune, b->stats, st, &b->launches,
+    CUDA_TRY(launch_batch_frame(b->d_jobs, b->d_firsts, m, max_bg, P, waves, b->wf, b->tune, b->stats, st, &b->launches,
                                 b->ctx->present_lut, cls.data(), (int)cls.size(), &at));
   }
   CUDA_TRY(cudaEventRecord(b->ev_end, st));

@@ -104,7 +104,10 @@ VRT_DI void sincos_(float x, float& s, float& c) {
 
 // Packed fp32 pairs (sm_100a's f32x2 arithmetic): each lane rounds exactly
 // as the scalar instruction would, so a pair of independent scalar
-// operations can run as one instruction without changing a bit.
+// operations can run as one instruction without changing a bit.  Except where
+// a product is an addend: the assembler fuses a packed multiply and a packed
+// add that consumes it into one rounding, .rn or not, so such a pair stays
+// scalar.
 VRT_DI float2 f2_mul(float2 a, float2 b) {
   float2 r;
   asm("{\n\t.reg .b64 a, b, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\t"
@@ -123,6 +126,13 @@ VRT_DI float2 f2_sub(float2 a, float2 b) {
   float2 r;
   asm("{\n\t.reg .b64 a, b, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\t"
       "sub.rn.f32x2 d, a, b;\n\tmov.b64 {%0, %1}, d;\n\t}"
+      : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return r;
+}
+VRT_DI float2 f2_add_rd(float2 a, float2 b) {   // rounded down
+  float2 r;
+  asm("{\n\t.reg .b64 a, b, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\t"
+      "add.rm.f32x2 d, a, b;\n\tmov.b64 {%0, %1}, d;\n\t}"
       : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
   return r;
 }
@@ -309,9 +319,15 @@ VRT_DI Mat unpack_material(uint32_t m) {
 // ---------------------------------------------------------------------------
 struct DScene {
   const uint32_t* __restrict__ vox;     // N^3 packed voxels
-  const uint32_t* __restrict__ masks;   // 16 words per brick
+  // Both levels' occupancy over the brick grid padded by one cell on each side
+  // (P = BG + 2 cells per axis, brick (x, y, z) at cell (x + 1, y + 1, z + 1)):
+  // 1 bit per cell (border cells: set), then from word mw on 16 mask words per
+  // cell (border cells: full).
+  const uint32_t* __restrict__ cells;
   const uint32_t* __restrict__ bits;    // 1 bit per brick: bricks[bi] != 0
   int N, BG;
+  uint32_t rP, rP2;                     // 2^32 / P and 2^32 / P^2 rounded up (dda_walk.cuh)
+  uint32_t mw, pad;
 };
 
 struct DHit {
@@ -428,6 +444,8 @@ VRT_DI DHit trace(const DScene& S, const uint32_t* occ, F3 roW, F3 rd, float max
   const F3 tDeltaB = absInv * 8.0f;
   F3 tMaxB = ((f3((float)bx, (float)by, (float)bz) + stepGE) * 8.0f - ro) * invRd;
 
+  const int P = BG + 2;                                       // the padded grid's side
+  const uint32_t* __restrict__ mask0 = S.cells + (S.mw + 16u * (uint32_t)(1 + P + P * P));   // brick (0, 0, 0)
   const int outerMax = 3 * BG + 2;
   for (int iter = 0; iter < outerMax; iter++) {
     if (t > tExit) break;
@@ -442,7 +460,7 @@ VRT_DI DHit trace(const DScene& S, const uint32_t* occ, F3 roW, F3 rd, float max
       F3 tMaxV = ((f3((float)vx, (float)vy, (float)vz) + stepGE) - ro) * invRd;
       float tCur = t;
       int vax = ax;
-      const uint32_t* __restrict__ bm = S.masks + (size_t)bi * 16u;
+      const uint32_t* __restrict__ bm = mask0 + (uint32_t)(bx + P * (by + P * bz)) * 16u;
       for (int j = 0; j < 3 * kBrick; j++) {
         if (kCount) cnt.inner++;
         const uint32_t bit = (uint32_t)((vx - mnx) + (vy - mny) * 8 + (vz - mnz) * 64);

@@ -7,16 +7,31 @@
 namespace vrt {
 
 // Device-resident scene: packed voxels, per-brick words and masks, plus the
-// 1-bit-per-brick occupancy bitmap the traversal stages in shared memory.
+// 1-bit-per-brick occupancy bitmap the per-thread traversal stages in shared
+// memory and the padded one the queue tracer walks (dda_walk.cuh).
 struct SceneDev {
   uint32_t* vox = nullptr;     // N^3
   uint32_t* bricks = nullptr;  // BG^3
-  uint32_t* masks = nullptr;   // 16 * BG^3
+  uint32_t* cells = nullptr;   // the padded bitmap and, from word mask_word(BG) on, the padded masks
   uint32_t* bits = nullptr;    // ceil(BG^3 / 32)
   int N = 0, BG = 0;
 };
 
 inline size_t occ_words(int BG) { return ((size_t)BG * BG * BG + 31) / 32; }
+// Largest brick grid side of the queue tracer's narrow form (dda_walk.cuh).
+constexpr int kNarrowBG = 128;
+// Words of the padded bitmap: one bit per cell of the (BG + 2)^3 grid, a border of one cell on
+// each side of the brick grid, whose bits are set.
+inline size_t pad_words(int BG) { return ((size_t)(BG + 2) * (BG + 2) * (BG + 2) + 31) / 32; }
+// The padded masks (16 words per cell) follow on a 64-byte boundary.
+inline size_t mask_word(int BG) { return (pad_words(BG) + 15) / 16 * 16; }
+inline size_t cell_bytes(int BG) {
+  return mask_word(BG) * 4 + (size_t)(BG + 2) * (BG + 2) * (BG + 2) * 64;
+}
+// 2^32 / d rounded up: with umulhi, the quotient of an index below 2^32 / d or one more.
+inline uint32_t recip_up(uint32_t d) { return (uint32_t)((1ull << 32) / d + 1ull); }
+inline uint32_t recip_pad(int BG) { return recip_up((uint32_t)BG + 2u); }
+inline uint32_t recip_pad2(int BG) { return recip_up((uint32_t)(BG + 2) * (uint32_t)(BG + 2)); }
 
 // Per-frame counters written by the path kernel (u64 each).
 enum StatSlot {
@@ -77,12 +92,11 @@ struct CacheDev {
 
 // Launch-shape knobs of the wavefront tracer (chosen by the autotuner).
 struct WavefrontTuning {
-  int refill_min = 8;           // idle lanes that trigger a warp refill
+  int refill_min = 12;          // idle lanes that trigger a warp refill
   int trace_blocks_per_sm = 0;  // 0 = occupancy maximum
   int shade_blocks_per_sm = 32;
-  int trace_variant = 0;        // (DDA iterations per warp-bookkeeping pass, min blocks/SM):
-                                // 0: (8, 5)  1: (6, 5)  2: (6, 4)  3: (4, 4)  4: (2, 1)  5: (1, 1);
-                                // 6, 7, 8: (8, 5) with the step loop unrolled 1, 2, 4 times
+  int trace_variant = 0;        // shape of the tracer (wf_dispatch_trace): (transition rounds per
+                                // warp-bookkeeping pass, steps per round, min blocks/SM)
   int atrous_rows = 0;          // a-trous output tile rows: 0 or 8 = 8 at all steps, 16 = 16 at steps 1-2 and 8 at step 4
   int tail_wave = -1;           // first wave whose paths finish one thread each (k_wf_tail); 0 = never;
                                 // -1 = automatic: wave 2 for cache-assisted frames (a session's, or a
@@ -94,9 +108,11 @@ struct WavefrontTuning {
 struct JobHost {
   VrtUniforms u;
   const uint32_t* vox;
-  const uint32_t* masks;
+  const uint32_t* cells;
   const uint32_t* bits;
   int N, BG;
+  uint32_t rP, rP2;         // recip_pad(BG), recip_pad2(BG)
+  uint32_t mw, spad;        // mask_word(BG)
   void* rad16;
   void* rad32;
   uint32_t* alb8;
@@ -146,7 +162,8 @@ struct CacheLaunch {
 // One batch frame over n jobs of P pixels in total: wavefront path trace
 // (waves = max bounces + 2), the cache jobs' post-wave work, temporal,
 // 3x a-trous, present.
-cudaError_t launch_batch_frame(const void* d_jobs, const uint32_t* d_firsts, int n, uint32_t P, int waves,
+// max_bg: the largest brick grid side of the jobs' scenes.
+cudaError_t launch_batch_frame(const void* d_jobs, const uint32_t* d_firsts, int n, int max_bg, uint32_t P, int waves,
                                const WavefrontBufs& wb, const WavefrontTuning& tune, unsigned long long* stats,
                                cudaStream_t st, uint32_t* launches, const float* present_lut,
                                const CacheLaunch* cls = nullptr, int ncl = 0, const AtrousTiles* at = nullptr);
@@ -235,6 +252,7 @@ cudaError_t launch_wavefront(const SceneDev& s, const VrtUniforms& u, float fcla
 
 cudaError_t launch_build_bricks(const SceneDev& s, int bx0, int by0, int bz0, int bx1, int by1, int bz1,
                                 cudaStream_t st);
+// Both occupancy bitmaps (plain and padded) from the brick words.
 cudaError_t launch_build_bits(const SceneDev& s, cudaStream_t st);
 cudaError_t launch_fill_box(const SceneDev& s, int x0, int y0, int z0, int x1, int y1, int z1, uint32_t value,
                             cudaStream_t st);

@@ -3,6 +3,7 @@
 // (k_batch.cu): path-state layout, block-aggregated queue appends, the flat
 // two-level DDA, and per-vertex shading.
 #pragma once
+#include "dda_walk.cuh"
 #include "vrt_device.cuh"
 #include "vrt_internal.h"
 #include <algorithm>
@@ -68,182 +69,6 @@ VRT_DI F3 hit_normal(int vax, F3 rd) {
 }
 
 // ---------------------------------------------------------------------------
-// Two-level DDA as one resumable iteration shared by both levels
-// (voxel.wgsl:73-153).  Each call performs
-//   [pending step at the current level] + [test of the current cell],
-// so lanes walking bricks and lanes walking voxels execute the same code.
-// Transitions reproduce the nested loops:
-//   brick test occupied  -> descend (entry voxel from t + 1e-4, next call
-//                           tests it without stepping)
-//   voxel test occupied  -> hit (voxel read, maxT check)
-//   voxel step leaves the brick, or 24 voxel tests done -> brick step pending
-// Steps use fma(|invRd|, scale, tMax), which equals the reference's
-// tMax + |invRd|*8 (brick) and tMax + |invRd| (voxel) bit for bit because
-// |invRd|*8 and |invRd|*1 are exact.
-// Counters follow the oracle: outer = brick iterations entered, inner =
-// voxel iterations entered, vreads = voxel words read.
-// ---------------------------------------------------------------------------
-enum : int { kLevelVoxel = 1, kPending = 2, kDone = 4, kHitCell = 8 };
-
-// Register layout: tm / (cx, cy, cz) / t / ax hold the current level's state
-// -- the brick level's tMaxB, brick cell, t and ax while walking bricks, the
-// voxel level's tMaxV, local cell, tCur and vax while walking voxels -- so the
-// step reads no level-selected operands; the brick level's tMax and cell are
-// saved in tmB / (bx, by, bz) on descent and restored when the voxel walk ends
-// (t and ax need no restore: the brick step that follows rewrites them).  The
-// step's scale (8 or 1) and the cells per axis (BG or 8, which is also the
-// stride of the test's bit index) are per-level registers, and only the
-// stepped coordinate is bounds-checked (the others did not move).  The entry axis left in ax after a miss is not meaningful; every
-// consumer reads it for hits only.  Against a layout with both levels' state
-// and per-operand level selects: 1.61 -> 1.48 ms of trace on the 1080p frame.
-struct FlatDDA {
-  F3 ro, invRd;
-  float maxT, tExit;
-  F3 tm, tmB;
-  int cx, cy, cz;               // current cell (brick, or voxel local to the brick)
-  int bx, by, bz;               // brick cell while walking voxels
-  int sx, sy, sz;
-  float t, sc;
-  int ext, ax, iter, j, state;   // ext: cells per axis of the current level (BG, or 8 in a brick)
-  uint32_t bi16;                // 16 x the brick index while walking voxels (its first mask word)
-  float tHit;
-  uint32_t mat;
-
-  VRT_DI bool done() const { return (state & kDone) != 0; }
-  VRT_DI int hit_axis() const { return ax; }
-
-  // Counters: brick iterations entered = iter at the end of the walk; voxel
-  // iterations = the sum of j over the bricks walked (added as each voxel
-  // walk ends), so the steps count nothing.
-  VRT_DI void finish(const DScene& S, DCount& c) {
-    tHit = -1.0f;
-    mat = 0u;
-    c.outer += (uint32_t)iter;
-    if (state & kHitCell) {
-      c.inner += (uint32_t)j;
-      const uint32_t vx = (uint32_t)(bx * kBrick + cx), vy = (uint32_t)(by * kBrick + cy),
-                     vz = (uint32_t)(bz * kBrick + cz);
-      mat = __ldg(S.vox + (vx + vy * (uint32_t)S.N + vz * (uint32_t)(S.N * S.N)));
-      c.vreads++;
-      if (!(t > maxT)) tHit = t * kVoxelSize;
-      else mat = 0u;
-    }
-  }
-
-  VRT_DI void init(const DScene& S, F3 roW, F3 rd, float maxTW) {
-    ro = roW * kInvVoxel;
-    maxT = maxTW * kInvVoxel;
-    const float sgx = rd.x >= 0.0f ? 1.0f : -1.0f;
-    const float sgy = rd.y >= 0.0f ? 1.0f : -1.0f;
-    const float sgz = rd.z >= 0.0f ? 1.0f : -1.0f;
-    invRd = f3(safe_inv(sgx, rd.x), safe_inv(sgy, rd.y), safe_inv(sgz, rd.z));
-    sx = rd.x > 0.0f ? 1 : (rd.x < 0.0f ? -1 : 0);
-    sy = rd.y > 0.0f ? 1 : (rd.y < 0.0f ? -1 : 0);
-    sz = rd.z > 0.0f ? 1 : (rd.z < 0.0f ? -1 : 0);
-    const F3 stepGE = f3(rd.x >= 0.0f ? 1.0f : 0.0f, rd.y >= 0.0f ? 1.0f : 0.0f, rd.z >= 0.0f ? 1.0f : 0.0f);
-    const float G = (float)S.N;
-    const F3 t0 = f3(__fsub_rn(0.0f, ro.x), __fsub_rn(0.0f, ro.y), __fsub_rn(0.0f, ro.z)) * invRd;
-    const F3 t1 = (f3(G, G, G) - ro) * invRd;
-    const F3 tmin3 = min3(t0, t1);
-    const F3 tmax3 = max3(t0, t1);
-    const float tEnter = fmax_(fmax_(tmin3.x, tmin3.y), fmax_(tmin3.z, 0.0f));
-    tExit = fmin_(fmin_(tmax3.x, tmax3.y), fmin_(tmax3.z, maxT));
-    iter = 0;
-    j = 0;
-    ax = 0;
-    if (tEnter > tExit) { state = kDone; return; }
-    if (tmin3.x >= tmin3.y && tmin3.x >= tmin3.z) ax = 0;
-    else if (tmin3.y >= tmin3.z) ax = 1;
-    else ax = 2;
-    t = tEnter;
-    const F3 sp = ro + rd * (t + 1e-4f);
-    // x / 8 as x * 0.125: the same real number, so the same rounding
-    cx = iclamp_(ifloor_(sp.x * 0.125f), 0, S.BG - 1);
-    cy = iclamp_(ifloor_(sp.y * 0.125f), 0, S.BG - 1);
-    cz = iclamp_(ifloor_(sp.z * 0.125f), 0, S.BG - 1);
-    tm = ((f3((float)cx, (float)cy, (float)cz) + stepGE) * 8.0f - ro) * invRd;
-    sc = 8.0f;
-    ext = S.BG;
-    state = 0;   // brick level, test first
-  }
-
-  // The voxel walk of the current brick ends: brick step next.
-  VRT_DI void leave_brick(const DScene& S, DCount& c) {
-    c.inner += (uint32_t)j;
-    cx = bx; cy = by; cz = bz;
-    tm = tmB;
-    sc = 8.0f;
-    ext = S.BG;
-    state = kPending;
-  }
-
-  // kSharedOcc: occ is the block's shared-memory copy of the occupancy bitmap;
-  // otherwise it is the scene's bitmap in global memory, read through the
-  // read-only path.
-  template <bool kSharedOcc>
-  VRT_DI void step(const DScene& S, const uint32_t* occ, F3 rd, DCount& c) {
-    const bool lv = (state & kLevelVoxel) != 0;
-    if (state & kPending) {
-      const bool px = tm.x <= tm.y && tm.x <= tm.z;
-      const bool py = !px && tm.y <= tm.z;
-      const float tn = px ? tm.x : (py ? tm.y : tm.z);
-      const float ia = fabsf(px ? invRd.x : (py ? invRd.y : invRd.z));
-      const float nv = __fmaf_rn(ia, sc, tn);
-      int cn;
-      if (px) { tm.x = nv; cx += sx; cn = cx; }
-      else if (py) { tm.y = nv; cy += sy; cn = cy; }
-      else { tm.z = nv; cz += sz; cn = cz; }
-      t = tn;
-      ax = px ? 0 : (py ? 1 : 2);
-      if ((unsigned)cn >= (unsigned)ext) {   // left the brick (voxel walk) or the grid (brick walk)
-        if (lv) leave_brick(S, c);
-        else state = kDone;
-        return;
-      }
-      state &= ~kPending;
-    }
-    if (lv) {
-      if (j >= 3 * kBrick) { leave_brick(S, c); return; }   // voxel loop exhausted
-      j++;
-    } else {
-      if (iter >= 3 * S.BG + 2 || t > tExit) { state = kDone; return; }
-      iter++;
-    }
-    // the cell's bit index: the brick index bx + BG (by + BG bz) at brick level,
-    // the mask bit lx + 8 (ly + 8 lz) in a brick
-    const uint32_t idx = (uint32_t)cx + (uint32_t)ext * ((uint32_t)cy + (uint32_t)ext * (uint32_t)cz);
-    // two typed loads (the bitmap may be in shared memory, the masks are in
-    // global memory) rather than one load through a selected pointer
-    const uint32_t word = lv ? __ldg(S.masks + (size_t)bi16 + (idx >> 5))
-                             : (kSharedOcc ? occ[idx >> 5] : __ldg(occ + (idx >> 5)));
-    if (!((word >> (idx & 31u)) & 1u)) {
-      state |= kPending;
-      return;
-    }
-    if (lv) {
-      state = kDone | kHitCell;   // finish() reads the voxel
-      return;
-    }
-    // descend into the occupied brick (voxel.wgsl:104-109); t and ax carry over as tCur and vax
-    bx = cx; by = cy; bz = cz;
-    bi16 = idx * 16u;
-    tmB = tm;
-    const int mnx = bx * kBrick, mny = by * kBrick, mnz = bz * kBrick;
-    const F3 p = ro + rd * (t + 1e-4f);
-    const int vx = iclamp_(ifloor_(p.x), mnx, mnx + 7);
-    const int vy = iclamp_(ifloor_(p.y), mny, mny + 7);
-    const int vz = iclamp_(ifloor_(p.z), mnz, mnz + 7);
-    const F3 stepGE = f3(rd.x >= 0.0f ? 1.0f : 0.0f, rd.y >= 0.0f ? 1.0f : 0.0f, rd.z >= 0.0f ? 1.0f : 0.0f);
-    tm = ((f3((float)vx, (float)vy, (float)vz) + stepGE) - ro) * invRd;
-    cx = vx - mnx; cy = vy - mny; cz = vz - mnz;
-    j = 0;
-    sc = 1.0f;
-    ext = kBrick;
-    state = kLevelVoxel;
-  }
-};
-
-// ---------------------------------------------------------------------------
 // Job policies.  A "job" is one view (session) rendered in a wave: uniforms,
 // scene, size and output buffers.  Path state is indexed by a global pixel id
 // g (jobs are laid out back to back); outputs by the job-local pixel id.
@@ -275,6 +100,7 @@ struct SingleJob {
   VRT_DI int width(int) const { return W; }
   VRT_DI int height(int) const { return H; }
   VRT_DI uint32_t first(int) const { return 0u; }
+  bool wide() const { return S.BG > kNarrowBG; }
 };
 
 // Device job table entry of a batch (one per session in the batch).
@@ -304,6 +130,8 @@ struct MultiJob {
   const uint32_t* firsts;  // n entries, ascending
   int n;
   int cache_jobs;          // jobs with the cache on
+  int max_bg;              // largest brick grid side of the jobs' scenes
+  bool wide() const { return max_bg > kNarrowBG; }
   __host__ __device__ bool any_cache() const { return cache_jobs != 0; }
   VRT_DI const CacheDev& cache(int j) const { return jobs[j].cache; }
   VRT_DI int job_of(uint32_t g) const {
@@ -652,21 +480,23 @@ __global__ void __launch_bounds__(256) k_wf_generate(J jobs, uint32_t P, WfDev b
   b.S0[g] = make_float4(0.0f, 0.0f, 0.0f, __uint_as_float(rng));
 }
 
-// Persistent queue tracer.  kSmem: stage the (single) scene's occupancy
-// bitmap in shared memory.  kSteps DDA iterations per pass of the warp
-// bookkeeping (idle-lane ballot, refill, drain check).  kVarMaxT: shadow rays
-// carry their own maxT in R2.w (otherwise every ray ends at 1e4 m, the plain
-// path's bound, and the tracer keeps its register budget).
-template <class J, bool kSmem, int kSteps, int kMinB, bool kVarMaxT, int kUnroll = kSteps>
-__global__ void __launch_bounds__(256, kMinB) k_wf_trace(J jobs, WfDev b, int wave, int implicit_n,
+constexpr int kTraceThreads = 128;
+// Persistent queue tracer.  A pass of the warp bookkeeping (idle-lane ballot,
+// refill, drain check) covers kPhases rounds of up to kRun DDA steps and the
+// transitions due after them (dda_walk.cuh).  Lanes whose walk ended keep it
+// until the next refill, which stores all their hits together.  kVarMaxT:
+// shadow rays carry their own maxT in R2.w (otherwise every ray ends at 1e4 m,
+// the plain path's bound).  kWide: scenes of more than 128^3 bricks.
+//
+// Bound by instruction issue: on the 1080p / 256^3 frame (2 bounces, 6.4 M
+// rays, 32 cells each) the wave of vertex 0's shadow and bounce rays issues
+// 297 M warp instructions at 78% of the issue slots, 41% of them on the ALU
+// pipe; before the walk kept its transitions out of the step it was 444 M at
+// 86%.  The four waves' trace: 1.319 -> 0.949 ms (deep paths, 6 bounces:
+// 1.684 -> 1.210; the ReSTIR initial pass 1.918 -> 1.375).
+template <class J, bool kWide, int kPhases, int kMinB, int kRun, bool kVarMaxT>
+__global__ void __launch_bounds__(kTraceThreads, kMinB) k_wf_trace(J jobs, WfDev b, int wave, int implicit_n,
                                                               int refill_min, unsigned long long* stats) {
-  extern __shared__ uint32_t s_occ[];
-  if (kSmem) {
-    const DScene S0 = jobs.scene(0);
-    const int nwords = (S0.BG * S0.BG * S0.BG + 31) >> 5;
-    for (int i = threadIdx.x; i < nwords; i += blockDim.x) s_occ[i] = __ldg(S0.bits + i);
-    __syncthreads();
-  }
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const int nf = implicit_n > 0 ? 0 : b.ctr[4 * wave];   // shadow rays at the queue's front
@@ -674,17 +504,32 @@ __global__ void __launch_bounds__(256, kMinB) k_wf_trace(J jobs, WfDev b, int wa
   int* head = b.ctr + 4 * wave + 1;
   const uint32_t* queue = queue_of(b, wave);
   DCount c{0u, 0u, 0u, 0u};
-  FlatDDA d;
+  Walk<kWide> d;
   DScene S = jobs.scene(0);
   F3 rd = f3(0.0f, 0.0f, 0.0f);
   uint32_t entry = 0u;
   int jc = 0;                     // the lane's last job and its pixel range [jlo, jhi) (empty: none yet)
   uint32_t jlo = 0u, jhi = 0u;
   uint32_t passes = 0u;   // passes of the step loop with a lane walking (warp-uniform)
-  bool active = false, drained = false;
+  bool active = false, held = false, drained = false;   // held: the lane's ray is not stored yet
   while (true) {
     const unsigned idle = __ballot_sync(full, !active);
     const int nidle = __popc(idle);
+    if (nidle >= refill_min || nidle == 32 || drained) {
+      // the lanes whose walk ended store their hits together
+      if (held && !active) {
+        d.finish(S, c);
+        const uint32_t g = entry & ~kShadowBit;
+        uint32_t* h = reinterpret_cast<uint32_t*>(b.hit + g);
+        if (entry & kShadowBit) {
+          h[3] = d.tHit >= 0.0f ? 1u : 0u;
+        } else {
+          *reinterpret_cast<uint2*>(h) = make_uint2(__float_as_uint(d.tHit), d.mat);
+          h[2] = (uint32_t)d.hit_axis(S);
+        }
+        held = false;
+      }
+    }
     if (!drained && (nidle >= refill_min || nidle == 32)) {
       int base = 0;
       if (lane == 0) base = atomicAdd(head, nidle);
@@ -724,6 +569,7 @@ __global__ void __launch_bounds__(256, kMinB) k_wf_trace(J jobs, WfDev b, int wa
           }
           c.rays++;
           active = true;
+          held = true;
         }
       }
     }
@@ -733,26 +579,17 @@ __global__ void __launch_bounds__(256, kMinB) k_wf_trace(J jobs, WfDev b, int wa
     }
     passes++;
     if (active) {
-#pragma unroll kUnroll
-      for (int k = 0; k < kSteps; k++)
-        if (!d.done()) d.step<kSmem>(S, kSmem ? s_occ : S.bits, rd, c);
-      if (d.done()) {
-        d.finish(S, c);
-        const uint32_t g = entry & ~kShadowBit;
-        uint32_t* h = reinterpret_cast<uint32_t*>(b.hit + g);
-        if (entry & kShadowBit) {
-          h[3] = d.tHit >= 0.0f ? 1u : 0u;
-        } else {
-          *reinterpret_cast<uint2*>(h) = make_uint2(__float_as_uint(d.tHit), d.mat);
-          h[2] = (uint32_t)d.hit_axis();
-        }
-        active = false;
+#pragma unroll 1
+      for (int k = 0; k < kPhases; k++) {
+        d.template walk_run<kRun>(S);
+        if (!d.walking() && !d.done()) d.transition(S, rd, c);
       }
+      active = !d.done();
     }
   }
   if (stats) {
     block_flush_stats(stats, c, 0u);   // kStatRays..kStatVReads
-    block_flush_one(stats + kStatTraceSlots, lane == 0 ? passes * (uint32_t)(32 * kSteps) : 0u);
+    block_flush_one(stats + kStatTraceSlots, lane == 0 ? passes * (uint32_t)(32 * kPhases * kRun) : 0u);
   }
 }
 
@@ -897,7 +734,7 @@ __global__ void __launch_bounds__(256, 5) k_wf_shade(J jobs, WfDev b, int wave) 
 // training paths after every other path ended at its first bounce: one
 // thread finishes each path of wave `wave`'s active list, tracing its pending
 // shadow and bounce rays with the same resumable DDA the queue tracer runs
-// (FlatDDA: same walk, hits and counters) and shading each vertex as
+// (dda_walk.cuh: same walk, hits and counters) and shading each vertex as
 // k_wf_shade does, until the path ends.  The per-wave form would launch a
 // trace and a shade kernel for every remaining bounce, each waiting for the
 // slowest of ~10^5 latency-bound walks; here each path runs its own
@@ -906,15 +743,8 @@ __global__ void __launch_bounds__(256, 5) k_wf_shade(J jobs, WfDev b, int wave) 
 // shading when its own ray ends and then taking the next path -- ran 447
 // against 305 us per 1080p cache frame: some lane shades in nearly every pass,
 // so the warp runs the shading code far more often than once per bounce.)
-template <class J, bool kSmem>
+template <class J, bool kWide>
 __global__ void __launch_bounds__(128, 6) k_wf_tail(J jobs, WfDev b, int wave, unsigned long long* stats) {
-  extern __shared__ uint32_t s_occ[];
-  if (kSmem) {
-    const DScene S0 = jobs.scene(0);
-    const int nwords = (S0.BG * S0.BG * S0.BG + 31) >> 5;
-    for (int i = threadIdx.x; i < nwords; i += blockDim.x) s_occ[i] = __ldg(S0.bits + i);
-    __syncthreads();
-  }
   const bool any_cache = jobs.any_cache();
   const int n = b.ctr[4 * wave + 2];
   const uint32_t* list = active_of(b, wave);
@@ -936,7 +766,6 @@ __global__ void __launch_bounds__(128, 6) k_wf_tail(J jobs, WfDev b, int wave, u
       const int role = cache_role(cc, lp, W);
       const Uni& u = jobs.uni(j);
       const DScene S = jobs.scene(j);
-      const uint32_t* occ = kSmem ? s_occ : S.bits;
       for (int w = wave;; w++) {
         const float4 s0 = b.S0[g];
         const float4 s1 = b.S1[g];
@@ -952,27 +781,33 @@ __global__ void __launch_bounds__(128, 6) k_wf_tail(J jobs, WfDev b, int wave, u
         if (flags & kFlagShadow) {   // the previous vertex's sun shadow ray
           const float4 r2 = b.R2[g];
           const F3 ld = xyz(r2);
-          FlatDDA d;
+          Walk<kWide> d;
           d.init(S, surf, ld, r2.w);
           c.rays++;
-          while (!d.done()) d.step<kSmem>(S, occ, ld, c);
+          while (!d.done()) {
+            d.template walk_run<3>(S);
+            if (!d.walking()) d.transition(S, ld, c);
+          }
           d.finish(S, c);
           if (!(d.tHit >= 0.0f)) radiance = radiance + xyz(s2);
         }
         bool done = (flags & kFlagTerminal) != 0u;
         if (!done) {
           const F3 rd = xyz(r1);
-          FlatDDA d;
+          Walk<kWide> d;
           d.init(S, surf, rd, 1e4f);
           c.rays++;
-          while (!d.done()) d.step<kSmem>(S, occ, rd, c);
+          while (!d.done()) {
+            d.template walk_run<3>(S);
+            if (!d.walking()) d.transition(S, rd, c);
+          }
           d.finish(S, c);
           if (d.tHit < 0.0f) {
             radiance = radiance + tp * sky_color(u, rd, false);
             done = true;
           } else {
             const F3 pos = surf + rd * d.tHit;
-            const F3 nrm = hit_normal(d.hit_axis(), rd);
+            const F3 nrm = hit_normal(d.hit_axis(S), rd);
             const Mat mat = unpack_material(d.mat);
             const uint32_t kmax = role == kRolePlain ? u.params0[1] : cc.train_bounces;
             bool shadow = false, bounce = false;
@@ -1144,67 +979,56 @@ cudaError_t launch_cache_post(const J& jobs, const WfDev& b, const CacheLaunch* 
   return cudaSuccess;
 }
 
-template <class J, bool kSmem, int kSteps, int kMinB, bool kVarMaxT, int kUnroll = kSteps>
-cudaError_t wf_launch_trace(const J& jobs, int smem, int blocks_per_sm, int sms, const WfDev& b, int w,
-                            int implicit_n, int refill, unsigned long long* stats, cudaStream_t st) {
-  auto* fn = k_wf_trace<J, kSmem, kSteps, kMinB, kVarMaxT, kUnroll>;
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-  }
+template <class J, bool kWide, int kPhases, int kMinB, int kRun, bool kVarMaxT>
+cudaError_t wf_launch_trace(const J& jobs, int blocks_per_sm, int sms, const WfDev& b, int w, int implicit_n,
+                            int refill, unsigned long long* stats, cudaStream_t st) {
+  auto* fn = k_wf_trace<J, kWide, kPhases, kMinB, kRun, kVarMaxT>;
   int per = blocks_per_sm;
   if (per <= 0) {
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, 256, smem);
+    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, kTraceThreads, 0);
     if (e != cudaSuccess || per < 1) per = 1;
   }
-  fn<<<sms * per, 256, smem, st>>>(jobs, b, w, implicit_n, refill, stats);
+  fn<<<sms * per, kTraceThreads, 0, st>>>(jobs, b, w, implicit_n, refill, stats);
   return cudaGetLastError();
 }
 
-// Tracer variants (the autotuner's trace_variant): DDA iterations per pass of
-// the warp bookkeeping x minimum resident blocks per SM (register cap).
-// Measured on the 1080p / 256^3 frame with FlatDDA's current-level register
-// layout: 8 x 5 (48 registers) 1.48 ms of trace, 6 x 5 1.49, 12 x 5 1.63,
-// 16 x 5 1.69 ms; with the typed test loads 8 x 5 1.436, 8 x 6 (40 registers,
-// spilling) 1.491, 8 x 4 (59 registers) 1.497 ms; with the earlier layout 8 x 5 1.60-1.66, 6 x 5 1.67,
-// 6 x 4 (57 registers) 1.71, 4 x 4 1.74, 2 x 1 (69) 1.98, 1 x 1 2.20 ms.
-// (Stepping until enough lanes are idle, with a ballot after every iteration,
-// ran 1.88 ms: the per-iteration ballot costs more than the idle lanes of a
-// fixed pass.)  Also measured with the earlier layout and dropped, each
-// bit-identical: a step with every outcome selected instead of branched (only
-// the descent branched) 2.02 ms; descents parked until the end of each pass,
-// so that a warp runs the descent block once per pass, 1.71 (4 x 5) - 1.80 ms
-// (8 x 5); an exact empty-space skip (brick distance field and 4^3 sub-block
-// masks, the skipped steps replayed in closed form per axis: 41% fewer step
-// calls on this frame) 2.2 - 3.3 ms, because a warp runs the ~100-instruction
-// replay in nearly every step in which one of its lanes needs it.
-template <class J, bool kSmem, bool kVarMaxT = false>
-cudaError_t wf_dispatch_trace(int variant, const J& jobs, int smem, int tb, int sms, const WfDev& b, int w, int impl,
+// Tracer variants (the autotuner's trace_variant).  A transition runs for
+// every lane that waits for one, in about as many instructions as four steps,
+// and nearly every step of a warp makes some lane due for one: more steps per
+// round share a transition's cost among more lanes, and leave more lanes
+// waiting.  Trace time of the 1080p / 256^3 frame by steps per round (9 blocks
+// of 128 threads and 56 registers per SM, refill at 12 idle lanes): 1 step
+// 1.251 ms, 3 0.987, 4 0.955, 5 0.949, 6 0.952.  8 blocks (64 registers, no
+// spills) 0.971 at 4 steps; 10 (48 registers, spilling) 1.05 at 3.  Refill at 8
+// / 10 / 12 / 14 idle lanes: 0.959 / 0.950 / 0.949 / 0.953.  Fetching the next
+// cell's word before the checks that may end a level's walk: 0.990 against
+// 0.971 (it costs a register that spills).
+template <class J, bool kVarMaxT = false>
+cudaError_t wf_dispatch_trace(int variant, const J& jobs, int tb, int sms, const WfDev& b, int w, int impl,
                               int refill, unsigned long long* stats, cudaStream_t st) {
-  if (kVarMaxT)   // the ReSTIR passes: the default shape only
-    return wf_launch_trace<J, kSmem, 8, 5, kVarMaxT>(jobs, smem, tb, sms, b, w, impl, refill, stats, st);
+  if (jobs.wide())   // scenes of more than 128^3 bricks: the default shape only
+    return wf_launch_trace<J, true, 3, 9, 5, kVarMaxT>(jobs, tb, sms, b, w, impl, refill, stats, st);
+  if (kVarMaxT)      // the ReSTIR passes: the default shape only
+    return wf_launch_trace<J, false, 3, 9, 5, kVarMaxT>(jobs, tb, sms, b, w, impl, refill, stats, st);
   switch (variant) {
-    case 1: return wf_launch_trace<J, kSmem, 6, 5, false>(jobs, smem, tb, sms, b, w, impl, refill, stats, st);
-    case 2: return wf_launch_trace<J, kSmem, 6, 4, false>(jobs, smem, tb, sms, b, w, impl, refill, stats, st);
-    case 3: return wf_launch_trace<J, kSmem, 4, 4, false>(jobs, smem, tb, sms, b, w, impl, refill, stats, st);
-    case 4: return wf_launch_trace<J, kSmem, 2, 1, false>(jobs, smem, tb, sms, b, w, impl, refill, stats, st);
-    case 5: return wf_launch_trace<J, kSmem, 1, 1, false>(jobs, smem, tb, sms, b, w, impl, refill, stats, st);
-    // the default shape with the step loop unrolled 1, 2 or 4 times instead of 8 (smaller code;
-    // measured 1.396 / 1.354 / 1.358 ms of trace per 1080p frame against 1.349 fully unrolled)
-    case 6: return wf_launch_trace<J, kSmem, 8, 5, false, 1>(jobs, smem, tb, sms, b, w, impl, refill, stats, st);
-    case 7: return wf_launch_trace<J, kSmem, 8, 5, false, 2>(jobs, smem, tb, sms, b, w, impl, refill, stats, st);
-    case 8: return wf_launch_trace<J, kSmem, 8, 5, false, 4>(jobs, smem, tb, sms, b, w, impl, refill, stats, st);
-    default: return wf_launch_trace<J, kSmem, 8, 5, false>(jobs, smem, tb, sms, b, w, impl, refill, stats, st);
+    case 1: return wf_launch_trace<J, false, 4, 9, 4, false>(jobs, tb, sms, b, w, impl, refill, stats, st);
+    case 2: return wf_launch_trace<J, false, 3, 8, 4, false>(jobs, tb, sms, b, w, impl, refill, stats, st);
+    case 3: return wf_launch_trace<J, false, 4, 9, 3, false>(jobs, tb, sms, b, w, impl, refill, stats, st);
+    case 4: return wf_launch_trace<J, false, 2, 9, 4, false>(jobs, tb, sms, b, w, impl, refill, stats, st);
+    case 5: return wf_launch_trace<J, false, 8, 9, 1, false>(jobs, tb, sms, b, w, impl, refill, stats, st);
+    case 6: return wf_launch_trace<J, false, 4, 10, 3, false>(jobs, tb, sms, b, w, impl, refill, stats, st);
+    case 7: return wf_launch_trace<J, false, 3, 9, 6, false>(jobs, tb, sms, b, w, impl, refill, stats, st);
+    case 8: return wf_launch_trace<J, false, 3, 8, 6, false>(jobs, tb, sms, b, w, impl, refill, stats, st);
+    default: return wf_launch_trace<J, false, 3, 9, 5, false>(jobs, tb, sms, b, w, impl, refill, stats, st);
   }
 }
 
 // Launches generate + (trace, shade) x waves; shade(b, w, blocks) launches
-// the shading kernel of wave w.  smem > 0 selects the shared-memory bitmap
-// tracer (single scene only).
+// the shading kernel of wave w.
 constexpr int kPrimaryRefill = 32;   // idle lanes that trigger a refill in the primary wave (at least)
 
 template <class J, class ShadeFn, bool kVarMaxT = false>
-cudaError_t wf_run_waves(const J& jobs, uint32_t P, int waves, int smem, const WavefrontBufs& wb,
+cudaError_t wf_run_waves(const J& jobs, uint32_t P, int waves, const WavefrontBufs& wb,
                          const WavefrontTuning& tune, unsigned long long* stats, cudaStream_t st, uint32_t* launches,
                          cudaEvent_t* trace_ev, int max_timed_waves, int* timed_waves, ShadeFn shade,
                          int tail_from = 0) {
@@ -1213,7 +1037,7 @@ cudaError_t wf_run_waves(const J& jobs, uint32_t P, int waves, int smem, const W
   cudaError_t e = cudaMemsetAsync(wb.ctr, 0, (size_t)wb.max_waves * 16, st);
   if (e != cudaSuccess) return e;
   const int sms = wf_sm_count();
-  const int refill = tune.refill_min > 0 ? tune.refill_min : 8;
+  const int refill = tune.refill_min > 0 ? tune.refill_min : 12;
   const int sblocks = sms * (tune.shade_blocks_per_sm > 0 ? tune.shade_blocks_per_sm : 32);
   uint32_t nl = 0;
   k_wf_generate<J><<<(P + 255) / 256, 256, 0, st>>>(jobs, P, b);
@@ -1225,13 +1049,9 @@ cudaError_t wf_run_waves(const J& jobs, uint32_t P, int waves, int smem, const W
       // blocks (a block's round waits for its slowest path) and 262 with 64; a grid of one block per 256
       // training paths, blocks without paths returning at once, ran 291
       const int tblocks = sms * 6;
-      if (smem > 0) {
-        e = cudaFuncSetAttribute(k_wf_tail<J, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e == cudaSuccess) k_wf_tail<J, true><<<tblocks, 128, smem, st>>>(jobs, b, w, stats);
-      } else {
-        k_wf_tail<J, false><<<tblocks, 128, 0, st>>>(jobs, b, w, stats);
-      }
-      if (e != cudaSuccess || (e = cudaGetLastError()) != cudaSuccess) return e;
+      if (jobs.wide()) k_wf_tail<J, true><<<tblocks, 128, 0, st>>>(jobs, b, w, stats);
+      else k_wf_tail<J, false><<<tblocks, 128, 0, st>>>(jobs, b, w, stats);
+      if ((e = cudaGetLastError()) != cudaSuccess) return e;
       nl++;
       break;
     }
@@ -1243,10 +1063,7 @@ cudaError_t wf_run_waves(const J& jobs, uint32_t P, int waves, int smem, const W
     // 8 / 12 / 16 / 24 / 32 idle lanes (32: only whole warps refill), while the later waves are fastest at 8
     // (490 / 426 / 143 us against 530 / 479 / 153 at 24)
     const int rf = w == 0 ? std::max(refill, kPrimaryRefill) : refill;
-    if (smem > 0)
-      e = wf_dispatch_trace<J, true, kVarMaxT>(tune.trace_variant, jobs, smem, tb, sms, b, w, impl, rf, stats, st);
-    else
-      e = wf_dispatch_trace<J, false, kVarMaxT>(tune.trace_variant, jobs, 0, tb, sms, b, w, impl, rf, stats, st);
+    e = wf_dispatch_trace<J, kVarMaxT>(tune.trace_variant, jobs, tb, sms, b, w, impl, rf, stats, st);
     if (e != cudaSuccess) return e;
     if (tm && (e = cudaEventRecord(trace_ev[2 * w + 1], st)) != cudaSuccess) return e;
     if (tm) timed++;
@@ -1262,7 +1079,7 @@ cudaError_t wf_run_waves(const J& jobs, uint32_t P, int waves, int smem, const W
 // The plain path's wave sequence (with the radiance cache's counter reset
 // when any job has the cache on).
 template <class J>
-cudaError_t wf_launch_frame(const J& jobs, uint32_t P, int waves, int smem, const WavefrontBufs& wb,
+cudaError_t wf_launch_frame(const J& jobs, uint32_t P, int waves, const WavefrontBufs& wb,
                             const WavefrontTuning& tune, unsigned long long* stats, cudaStream_t st,
                             uint32_t* launches, cudaEvent_t* trace_ev, int max_timed_waves, int* timed_waves,
                             int njobs = 1, int tail_from = 0) {
@@ -1271,7 +1088,7 @@ cudaError_t wf_launch_frame(const J& jobs, uint32_t P, int waves, int smem, cons
     k_cache_reset<J><<<(njobs + 127) / 128, 128, 0, st>>>(jobs, njobs);
     if (launches) (*launches)++;
   }
-  return wf_run_waves(jobs, P, waves, smem, wb, tune, stats, st, launches, trace_ev, max_timed_waves, timed_waves,
+  return wf_run_waves(jobs, P, waves, wb, tune, stats, st, launches, trace_ev, max_timed_waves, timed_waves,
                       [&](const WfDev& b, int w, int sblocks) {
                         if (w == 0) k_wf_shade_primary<J><<<sblocks, 256, 0, st>>>(jobs, P, b, stats);
                         else k_wf_shade<J><<<sblocks, 256, 0, st>>>(jobs, b, w);
