@@ -1,4 +1,5 @@
-"""The queue tracer's brick -> voxel walk (csrc/dda_walk.cuh) against the
+"""The queue tracer's brick -> voxel walk (csrc/dda_walk.cuh).  Ray
+batches run it directly and are held to the CPU oracle; frames are held to the
 per-thread nested loops (the path-trace megakernel, itself held to the CPU
 oracle by the parity tests): the same frame through both, at the grid sizes
 where the walk's packed words change shape -- one brick, grids whose side is no
@@ -55,3 +56,53 @@ def test_walk_matches_nested_loops(vrt, ctx, n):
         assert np.array_equal(wave.gbuffer().view(np.uint32), mega.gbuffer().view(np.uint32))
     for o in (wave, mega, sc):
         o.close()
+
+
+def _odd_rays(n, ext, seed):
+    """Random rays, and the forms a walk can trip over: zero, tiny, huge, infinite and NaN components,
+    origins on voxel and brick edges, far away or not finite, bounds of every size."""
+    r = np.random.default_rng(seed)
+    o = (r.random((n, 3)) * ext).astype(np.float32)
+    d = r.normal(size=(n, 3))
+    d = (d / np.linalg.norm(d, axis=1, keepdims=True)).astype(np.float32)
+    t = np.where(r.random(n) < 0.6, 1e4, r.random(n) * ext).astype(np.float32)
+    form, ax = r.integers(0, 16, n), r.integers(0, 3, n)
+    rows = np.arange(n)
+
+    def put(a, k, v):
+        m = form == k
+        a[rows[m], ax[m]] = v
+    put(d, 0, 0.0)
+    put(d, 1, -0.0)
+    put(d, 2, 1e-9)
+    put(d, 3, 1e30)
+    put(d, 4, np.inf)
+    put(d, 5, np.nan)
+    put(o, 6, np.nan)
+    put(o, 7, np.inf)
+    o[form == 8] = np.floor(o[form == 8] * 16) / 16
+    o[form == 9] = np.floor(o[form == 9] * 2) / 2
+    d[form == 10] = np.sign(d[form == 10]) / np.float32(math.sqrt(3))
+    o[form == 11] = o[form == 11] * 3 - ext
+    o[form == 12] += np.float32(3e5)
+    d[form == 13] = np.eye(3, dtype=np.float32)[ax[form == 13]]
+    t[form == 14] = np.float32(np.nan)
+    t[form == 15] = np.float32(-1.0)
+    return o, d, t
+
+
+@pytest.mark.parametrize("grid", [8, 104, 256])
+@pytest.mark.parametrize("n", [1, 31, 33, 4097, 600_001, 1_100_003])
+def test_ray_batch_matches_oracle(vrt, orc, ctx, grid, n):
+    vox, _ = vrt.generate_scene(vrt.VRT_SCENE_RANDOM, grid, 3)
+    b, m = orc.build_bricks(vox, grid)
+    sc = vrt.Scene(ctx, vox, grid)
+    o, d, t = _odd_rays(n, grid / 16.0, grid + n)
+    got, want = sc.trace_rays(o, d, t), orc.trace(vox, b, m, grid, o, d, t)
+    for f in ("t", "n"):            # as bits, any NaN equal to any other
+        x, y = got[f], want[f]
+        assert np.array_equal(np.isnan(x), np.isnan(y))
+        assert np.array_equal(x.view(np.uint32)[~np.isnan(x)], y.view(np.uint32)[~np.isnan(y)])
+    for f in ("mat", "voxel", "face", "steps", "bytes"):
+        assert np.array_equal(got[f], want[f]), f
+    sc.close()

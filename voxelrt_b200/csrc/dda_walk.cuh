@@ -37,6 +37,16 @@
 
 namespace vrt {
 
+// Normal of a hit on entry axis `vax` for direction rd (same value the DDA
+// returns: -vmask * sign(rd)).
+VRT_DI F3 hit_normal(int vax, F3 rd) {
+  const int sx = rd.x > 0.0f ? 1 : (rd.x < 0.0f ? -1 : 0);
+  const int sy = rd.y > 0.0f ? 1 : (rd.y < 0.0f ? -1 : 0);
+  const int sz = rd.z > 0.0f ? 1 : (rd.z < 0.0f ? -1 : 0);
+  return f3(face_normal_component(vax == 0, sx), face_normal_component(vax == 1, sy),
+            face_normal_component(vax == 2, sz));
+}
+
 // Walk states.  kWalkOdd: a direction component of 0 or NaN, or values so
 // large that a point on the ray may lie far from its cell.
 enum : int { kWalkVoxel = 1, kWalkOdd = 2, kWalkOcc = 4, kWalkOut = 8, kWalkDone = 16, kWalkWaits = 4 };

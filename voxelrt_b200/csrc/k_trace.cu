@@ -1,4 +1,4 @@
-// k_trace.cu -- path-trace pass and the DDA parity entry (sm_100a).
+// k_trace.cu -- path-trace pass and the ray-batch entry (sm_100a).
 //
 // k_pathtrace is the plain branch of pathtrace.wgsl (lines 248-330): one
 // thread per pixel, 16x16-pixel blocks whose warps cover 8x4 pixel tiles so
@@ -6,6 +6,8 @@
 // per 8^3 brick, 4 KB at 256^3, 32 KB at 512^3) is staged once per block in
 // shared memory; brick masks and voxels are read through the read-only path
 // (L1/L2 resident: 2 MB + 64 MB at 256^3 fit the 126 MB L2).
+#include <algorithm>
+#include "dda_walk.cuh"
 #include "trace_kernel.cuh"
 
 namespace vrt {
@@ -95,25 +97,72 @@ __global__ void __launch_bounds__(256) k_pathtrace(DScene S, Uni u, float fclamp
   if (out.stats) block_flush_stats(out.stats, cnt, pix);
 }
 
-template <bool kSmem>
-__global__ void __launch_bounds__(256) k_trace_rays(DScene S, const float* __restrict__ o, const float* __restrict__ d,
-                                                    const float* __restrict__ tmax, int n, VrtHit* __restrict__ out) {
-  extern __shared__ uint32_t s_occ[];
-  const uint32_t* occ = stage_occupancy<kSmem>(S, s_occ);
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  DCount cnt{0u, 0u, 0u, 0u};
-  const F3 ro = f3(o[3 * i], o[3 * i + 1], o[3 * i + 2]);
-  const F3 rd = f3(d[3 * i], d[3 * i + 1], d[3 * i + 2]);
-  const DHit h = trace<true>(S, occ, ro, rd, tmax[i], cnt);
-  VrtHit r;
-  r.t = h.t; r.n[0] = h.n.x; r.n[1] = h.n.y; r.n[2] = h.n.z; r.mat = h.mat;
-  r.voxel[0] = h.vx; r.voxel[1] = h.vy; r.voxel[2] = h.vz;
-  r.face = h.t >= 0.0f ? face_of(h.n) : -1;
-  r.steps = cnt.outer + cnt.inner;
-  r.bytes = 4u * (cnt.outer + cnt.inner + cnt.vreads);
-  r.pad = 0u;
-  out[i] = r;
+// A batch of rays on the resumable walk (dda_walk.cuh).  A warp owns a run of
+// `run` consecutive rays and refills its idle lanes from it, so no counter in
+// memory is needed; blocks are many and short, and the block scheduler evens
+// the runs out.  Bound by instruction issue, like the queue tracer; against one
+// thread per ray on the nested loops, 2 M incoherent rays at 256^3 took 470 ->
+// 256 us (call with its wait), 1.2 M at 128^3 256 -> 166, 64 rays 27 -> 13, 1000
+// 27 -> 19; 20 K - 100 K rays, where the longest walk decides, 34 - 41 -> 35 - 43.
+constexpr int kRayThreads = 128, kRayRefill = 12, kRayMaxRun = 256;
+
+template <bool kWide>
+__global__ void __launch_bounds__(kRayThreads, 9) k_trace_rays(DScene S, const float* __restrict__ o,
+                                                               const float* __restrict__ d,
+                                                               const float* __restrict__ tmax, int n, int run,
+                                                               VrtHit* __restrict__ out) {
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const long long first = ((long long)blockIdx.x * (kRayThreads / 32) + (threadIdx.x >> 5)) * run;
+  if (first >= n) return;                                   // warp-uniform
+  uint32_t next = (uint32_t)first;
+  const uint32_t end = (uint32_t)min((long long)n, first + run);
+  DCount c{0u, 0u, 0u, 0u};
+  Walk<kWide> w;
+  F3 rd = f3(0.0f, 0.0f, 0.0f);
+  uint32_t i = 0u;
+  bool active = false, held = false;
+  while (true) {
+    const unsigned idle = __ballot_sync(full, !active);
+    const int nidle = __popc(idle);
+    if (nidle >= kRayRefill || next >= end) {
+      if (held && !active) {
+        VrtHit r;
+        int vx = -1, vy = -1, vz = -1;
+        const bool hit = w.finish(S, c, vx, vy, vz);
+        const F3 nrm = hit ? hit_normal(w.hit_axis(S), rd) : f3(-rd.x, -rd.y, -rd.z);
+        r.t = w.tHit; r.n[0] = nrm.x; r.n[1] = nrm.y; r.n[2] = nrm.z; r.mat = w.mat;
+        r.voxel[0] = hit ? vx : -1; r.voxel[1] = hit ? vy : -1; r.voxel[2] = hit ? vz : -1;
+        r.face = r.t >= 0.0f ? face_of(nrm) : -1;
+        r.steps = c.outer + c.inner;
+        r.bytes = 4u * (c.outer + c.inner + c.vreads);
+        r.pad = 0u;
+        out[i] = r;
+        held = false;
+      }
+      if (next < end) {
+        const uint32_t mine = next + __popc(idle & ((1u << lane) - 1u));
+        next += (uint32_t)nidle;
+        if (!active && mine < end) {
+          i = mine;
+          rd = f3(d[3 * (size_t)i], d[3 * (size_t)i + 1], d[3 * (size_t)i + 2]);
+          w.init(S, f3(o[3 * (size_t)i], o[3 * (size_t)i + 1], o[3 * (size_t)i + 2]), rd, tmax[i]);
+          c = DCount{0u, 0u, 0u, 0u};
+          active = held = true;
+        }
+      } else if (nidle == 32) {
+        return;
+      }
+    }
+    if (active) {
+#pragma unroll 1
+      for (int k = 0; k < 3; k++) {
+        w.template walk_run<5>(S);
+        if (!w.walking() && !w.done()) w.transition(S, rd, c);
+      }
+      active = !w.done();
+    }
+  }
 }
 
 cudaError_t launch_pathtrace(const SceneDev& s, const VrtUniforms& u, float fclamp, int W, int H,
@@ -135,17 +184,16 @@ cudaError_t launch_pathtrace(const SceneDev& s, const VrtUniforms& u, float fcla
 cudaError_t launch_trace_rays(const SceneDev& s, const float* o, const float* d, const float* tmax, int n,
                               VrtHit* out, cudaStream_t st) {
   if (n <= 0) return cudaSuccess;
-  const size_t smem = occ_words(s.BG) * sizeof(uint32_t);
-  const int blocks = (n + 255) / 256;
-  if (smem <= kMaxSmemOccBytes) {
-    if (smem > 48 * 1024) {
-      cudaError_t e = cudaFuncSetAttribute(k_trace_rays<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e != cudaSuccess) return e;
-    }
-    k_trace_rays<true><<<blocks, 256, smem, st>>>(to_dscene(s), o, d, tmax, n, out);
-  } else {
-    k_trace_rays<false><<<blocks, 256, 0, st>>>(to_dscene(s), o, d, tmax, n, out);
-  }
+  // Rays per warp.  Few rays are spread over all warps the GPU holds (9 blocks
+  // on each of 148 SMs), down to one per warp, since lanes on different paths
+  // take turns; from 32 per warp on, one per lane until the rays fill the GPU
+  // three times over, then longer runs with refills.
+  const int warps = kRayThreads / 32, resident = 148 * 9 * warps;
+  const int run = n <= 32 * resident ? (n + resident - 1) / resident
+                                     : std::min(kRayMaxRun, std::max(32, n / (3 * resident) / 32 * 32));
+  const unsigned blocks = (unsigned)(((long long)n + (long long)run * warps - 1) / ((long long)run * warps));
+  if (s.BG > kNarrowBG) k_trace_rays<true><<<blocks, kRayThreads, 0, st>>>(to_dscene(s), o, d, tmax, n, run, out);
+  else k_trace_rays<false><<<blocks, kRayThreads, 0, st>>>(to_dscene(s), o, d, tmax, n, run, out);
   return cudaGetLastError();
 }
 

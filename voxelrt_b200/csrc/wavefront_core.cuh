@@ -58,16 +58,6 @@ VRT_DI uint32_t warp_append(int* counter, bool pred) {
 
 VRT_DI F3 xyz(float4 v) { return f3(v.x, v.y, v.z); }
 
-// Normal of a hit on entry axis `vax` for direction rd (same value the DDA
-// returns: -vmask * sign(rd)).
-VRT_DI F3 hit_normal(int vax, F3 rd) {
-  const int sx = rd.x > 0.0f ? 1 : (rd.x < 0.0f ? -1 : 0);
-  const int sy = rd.y > 0.0f ? 1 : (rd.y < 0.0f ? -1 : 0);
-  const int sz = rd.z > 0.0f ? 1 : (rd.z < 0.0f ? -1 : 0);
-  return f3(face_normal_component(vax == 0, sx), face_normal_component(vax == 1, sy),
-            face_normal_component(vax == 2, sz));
-}
-
 // ---------------------------------------------------------------------------
 // Job policies.  A "job" is one view (session) rendered in a wave: uniforms,
 // scene, size and output buffers.  Path state is indexed by a global pixel id
