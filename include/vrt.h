@@ -119,8 +119,9 @@ typedef struct VrtTuning {
                                  one thread (their rays traced in turn, not in
                                  per-wave launches); 0 = never, -1 = automatic
                                  (wave 2 for a cache-assisted session, or for a
-                                 batch whose every job is cache-assisted; else
-                                 never); the image is the same either way      */
+                                 batch whose every job is cache-assisted; else by
+                                 pixels and bounces); the image is the same either
+                                 way                                           */
 } VrtTuning;
 
 /* One traced ray (vrt_trace_rays).  face: 0..5 = +x,-x,+y,-y,+z,-z normal,

@@ -106,3 +106,25 @@ def test_ray_batch_matches_oracle(vrt, orc, ctx, grid, n):
     for f in ("mat", "voxel", "face", "steps", "bytes"):
         assert np.array_equal(got[f], want[f]), f
     sc.close()
+
+
+# pixel counts on both sides of the lines at which the remaining paths of a
+# frame move to one thread each, by default and at every wave
+@pytest.mark.parametrize("W,H,bounces", [(401, 297, 2), (401, 303, 3), (611, 331, 2), (611, 331, 3), (811, 501, 4),
+                                         (1201, 801, 5)])
+def test_tail_waves_leave_the_image(vrt, ctx, W, H, bounces):
+    vox, spawn = vrt.generate_scene(vrt.VRT_SCENE_VOXELRT, 128, 7)
+    sc = vrt.Scene(ctx, vox, 128)
+    u = vrt.make_uniforms(vrt.camera_spline(spawn, 3), None, vrt.Lighting(), 9, bounces, 0, W, H)
+    want = None
+    for tail in (0, -1, 1, bounces + 1):
+        s = vrt.Session(ctx, sc, W, H, keep_radiance_f32=True)
+        s.set_tuning(tail_wave=tail)
+        s.set_timing(True)
+        s.frame(u)
+        st = s.stats()
+        got = (s.radiance_f32().tobytes(), s.ldr().tobytes(), st.rays, st.dda_outer, st.dda_inner, st.voxel_reads)
+        want = want or got
+        assert got == want, f"tail wave {tail}"
+        s.close()
+    sc.close()

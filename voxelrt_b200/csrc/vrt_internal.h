@@ -99,8 +99,7 @@ struct WavefrontTuning {
                                 // warp-bookkeeping pass, steps per round, min blocks/SM)
   int atrous_rows = 0;          // a-trous output tile rows: 0 or 8 = 8 at all steps, 16 = 16 at steps 1-2 and 8 at step 4
   int tail_wave = -1;           // first wave whose paths finish one thread each (k_wf_tail); 0 = never;
-                                // -1 = automatic: wave 2 for cache-assisted frames (a session's, or a
-                                // batch's whose every job has the cache on), else never
+                                // -1 = automatic (auto_tail in wavefront_core.cuh)
 };
 
 // Host mirror of the device job table entry (JobDev in wavefront_core.cuh):

@@ -501,11 +501,17 @@ __global__ void __launch_bounds__(kTraceThreads, kMinB) k_wf_trace(J jobs, WfDev
   int jc = 0;                     // the lane's last job and its pixel range [jlo, jhi) (empty: none yet)
   uint32_t jlo = 0u, jhi = 0u;
   uint32_t passes = 0u;   // passes of the step loop with a lane walking (warp-uniform)
+  // Lanes of a warp on different walks take turns, so the rays of a small wave are spread over all
+  // resident warps: each warp uses as many lanes as it has rays to take.
+  const int nwarps = (int)(gridDim.x * (kTraceThreads / 32));
+  const int lanes = min(32, max(1, (n + nwarps - 1) / nwarps));
+  const int refill = min(refill_min, lanes);
+  const unsigned in_use = lanes == 32 ? full : (1u << lanes) - 1u;
   bool active = false, held = false, drained = false;   // held: the lane's ray is not stored yet
   while (true) {
-    const unsigned idle = __ballot_sync(full, !active);
+    const unsigned idle = __ballot_sync(full, !active) & in_use;
     const int nidle = __popc(idle);
-    if (nidle >= refill_min || nidle == 32 || drained) {
+    if (nidle >= refill || drained) {
       // the lanes whose walk ended store their hits together
       if (held && !active) {
         d.finish(S, c);
@@ -520,12 +526,12 @@ __global__ void __launch_bounds__(kTraceThreads, kMinB) k_wf_trace(J jobs, WfDev
         held = false;
       }
     }
-    if (!drained && (nidle >= refill_min || nidle == 32)) {
+    if (!drained && nidle >= refill) {
       int base = 0;
       if (lane == 0) base = atomicAdd(head, nidle);
       base = __shfl_sync(full, base, 0);
       if (base + nidle >= n) drained = true;
-      if (!active) {
+      if ((idle >> lane) & 1u) {
         const int slot = base + __popc(idle & ((1u << lane) - 1u));
         if (slot < n) {
           entry = implicit_n > 0 ? (uint32_t)slot
@@ -729,19 +735,23 @@ __global__ void __launch_bounds__(256, 5) k_wf_shade(J jobs, WfDev b, int wave) 
 // trace and a shade kernel for every remaining bounce, each waiting for the
 // slowest of ~10^5 latency-bound walks; here each path runs its own
 // sequence.  Same per-path arithmetic and RNG draws, so the same image.
+// Few paths are spread over all warps, a few lanes each: lanes on different
+// walks take turns.
 // (A per-lane state machine -- lanes stepping their walks together, each
 // shading when its own ray ends and then taking the next path -- ran 447
 // against 305 us per 1080p cache frame: some lane shades in nearly every pass,
 // so the warp runs the shading code far more often than once per bounce.)
 template <class J, bool kWide>
-__global__ void __launch_bounds__(128, 6) k_wf_tail(J jobs, WfDev b, int wave, unsigned long long* stats) {
+__global__ void __launch_bounds__(128, 5) k_wf_tail(J jobs, WfDev b, int wave, unsigned long long* stats) {
   const bool any_cache = jobs.any_cache();
   const int n = b.ctr[4 * wave + 2];
   const uint32_t* list = active_of(b, wave);
-  const int stride = gridDim.x * blockDim.x;
+  // few paths are spread over all warps (as in k_wf_trace); every block runs every round
+  const int nwarps = (int)(gridDim.x * (blockDim.x >> 5)), warp = (int)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5));
+  const int lanes = min(32, max(1, (n + nwarps - 1) / nwarps)), lane = threadIdx.x & 31;
   DCount c{0u, 0u, 0u, 0u};
-  for (int base = blockIdx.x * blockDim.x; base < n; base += stride) {
-    const int i = base + threadIdx.x;
+  for (int base = 0; base < n; base += nwarps * lanes) {
+    const int i = lane < lanes ? base + warp * lanes + lane : n;
     bool fin_train = false;
     uint32_t ti = 0u;
     F3 rfin = f3(0.0f, 0.0f, 0.0f);
@@ -775,7 +785,7 @@ __global__ void __launch_bounds__(128, 6) k_wf_tail(J jobs, WfDev b, int wave, u
           d.init(S, surf, ld, r2.w);
           c.rays++;
           while (!d.done()) {
-            d.template walk_run<3>(S);
+            d.template walk_run<5>(S);
             if (!d.walking()) d.transition(S, ld, c);
           }
           d.finish(S, c);
@@ -788,7 +798,7 @@ __global__ void __launch_bounds__(128, 6) k_wf_tail(J jobs, WfDev b, int wave, u
           d.init(S, surf, rd, 1e4f);
           c.rays++;
           while (!d.done()) {
-            d.template walk_run<3>(S);
+            d.template walk_run<5>(S);
             if (!d.walking()) d.transition(S, rd, c);
           }
           d.finish(S, c);
@@ -1035,10 +1045,10 @@ cudaError_t wf_run_waves(const J& jobs, uint32_t P, int waves, const WavefrontBu
   int timed = 0;
   for (int w = 0; w < waves; w++) {
     if (tail_from > 0 && w == tail_from) {   // the remaining paths, one thread each
-      // a resident grid of 128-thread blocks: 260 us per 1080p cache frame against 282 with 256-thread
-      // blocks (a block's round waits for its slowest path) and 262 with 64; a grid of one block per 256
-      // training paths, blocks without paths returning at once, ran 291
-      const int tblocks = sms * 6;
+      // a resident grid of 128-thread blocks (a block's round waits for its slowest path); 5 per SM (96
+      // registers): 0.125 ms of path trace at 58 K pixels and 1.050 of a 1080p cache frame, against 0.133
+      // and 1.060 at 6, 0.146 and 1.082 at 8
+      const int tblocks = sms * 5;
       if (jobs.wide()) k_wf_tail<J, true><<<tblocks, 128, 0, st>>>(jobs, b, w, stats);
       else k_wf_tail<J, false><<<tblocks, 128, 0, st>>>(jobs, b, w, stats);
       if ((e = cudaGetLastError()) != cudaSuccess) return e;
@@ -1064,6 +1074,34 @@ cudaError_t wf_run_waves(const J& jobs, uint32_t P, int waves, const WavefrontBu
   if (launches) *launches += nl;
   if (timed_waves) *timed_waves = timed;
   return cudaGetLastError();
+}
+
+// The wave whose remaining paths finish one thread each when the tuning leaves
+// it open (0: none).  A wave has a floor of 25-35 us of trace and 5-8 of
+// shading -- its longest walk, whatever its size -- which k_wf_tail pays once for all the
+// waves it replaces, at a lower rate per ray; so the line lies at a number of
+// paths, later the more pixels there are.  Path-trace pass in ms by tail wave
+// (pixels, bounces: none / 1 / 2 / 3 / 4 / 5):
+//   58 K, 2: .183 / .125 / .149 / .167      58 K, 6: .400 / .208 / .246 / .282 / .301
+//  130 K, 2: .299 / .285 / .260 / .283     130 K, 6: .454 / .250 / .292 / .327 / .354
+//  230 K, 2: .333 / .341 / .347 / .316     230 K, 4: .372 / .328 / .287 / .316 / .330
+//  518 K, 2: .472 / .623 / .534 / .469     518 K, 6: .702 / .784 / .698 / .640 / .602 / .633
+//  925 K, 6: .830 / 1.10 / .908 / .765 / .734 / .762
+//  2.1 M, 2: 1.212 / 2.00 / 1.62 / 1.252   2.1 M, 6: 1.539 / 2.65 / 2.24 / 1.78 / 1.517 / 1.471
+// (The tail's grid holds 95 K paths at once; a few more cost it a second round.)
+// Cache-assisted frames (every path but the training paths ends at wave 1)
+// always take wave 2, and no job with the cache can take wave 1.
+inline int auto_tail(uint32_t P, int waves, bool any_cache, bool all_cache) {
+  if (all_cache) return 2;
+  const bool deep = waves > 4;   // 3 bounces or more
+  int w;
+  if (P <= 120000u) w = any_cache ? 2 : 1;
+  else if (P <= 200000u) w = 2;
+  else if (P <= 300000u) w = deep ? 2 : 3;
+  else if (P <= 700000u) w = deep ? 4 : 3;
+  else if (P <= 1500000u) w = 4;
+  else w = 5;
+  return w < waves ? w : 0;
 }
 
 // The plain path's wave sequence (with the radiance cache's counter reset
