@@ -112,9 +112,8 @@ typedef struct VrtTuning {
                                  min blocks per SM) = 0: (3,5,9) default,
                                  1: (4,4,9), 2: (3,4,8), 3: (4,3,9), 4: (2,4,9),
                                  5: (8,1,9), 6: (4,3,10), 7: (3,6,9), 8: (3,6,8) */
-  int atrous_tile_rows;       /* a-trous output tile rows: 0 (default) or 8 = 8
-                                 at every step, 16 = 16 at steps 1-2 and 8 at
-                                 step 4                                          */
+  int atrous_tile_rows;       /* 0, 8 or 16: accepted and returned; the a-trous
+                                 pass has one tile shape (32 x 32 pixels)      */
   int tail_wave;              /* first wave whose remaining paths each finish on
                                  one thread (their rays traced in turn, not in
                                  per-wave launches); 0 = never, -1 = automatic

@@ -93,3 +93,41 @@ def test_noalloc_rejects_images_above_its_limit(vrt):
     code = lib.vrt_denoise_atrous_noalloc(C.c_void_p(16), 0, C.c_void_p(16), C.c_void_p(16), 1920, 1081, None)
     assert code == 1
     assert "1920x1080" in lib.vrt_last_error_string().decode()
+
+
+# Tiles of both heights and their remainders; `form` picks what the tile code
+# decides on: axis-aligned normals (and none), normals off the axes, and values
+# that only the per-pixel form may see (negative, infinite and NaN colours,
+# long normals, NaN distances).  The oracle evaluates the same expressions, so
+# the bits are equal (any NaN equal to any other).
+@pytest.mark.parametrize("form", ["axes", "free", "odd"])
+@pytest.mark.parametrize("W,H,acc_f32", [(1, 1, False), (33, 17, True), (65, 47, False), (970, 965, False)])
+def test_noalloc_tiles(vrt, orc, W, H, acc_f32, form):
+    import torch
+    from voxelrt_b200._lib import lib
+
+    r = np.random.default_rng(W * H + len(form))
+    gb = np.zeros((H, W, 4), np.float32)
+    ax = r.integers(0, 4, (H, W))                      # 3: no normal at all
+    for k in range(3):
+        gb[..., k] = np.where(ax == k, r.choice([-1.0, 1.0], (H, W)), 0.0)
+    gb[..., 3] = np.where(r.random((H, W)) < 0.1, -1.0, 2.0 + 5.0 * r.random((H, W)))
+    acc = np.zeros((H, W, 4), np.float32)
+    acc[..., :3] = np.exp(r.normal(size=(H, W, 3)))
+    acc[..., :3][r.random((H, W)) < 0.05] = 0.0
+    acc[..., 3] = r.integers(0, 65, (H, W))
+    if form == "free":
+        m = r.random((H, W)) < 0.5
+        n = r.normal(size=(H, W, 3)).astype(np.float32)
+        gb[m, :3] = (n / np.linalg.norm(n, axis=-1, keepdims=True))[m]
+    if form == "odd":
+        for k, v in enumerate([-2.0, -0.0, np.inf, np.nan]):
+            acc[r.random((H, W)) < 0.002, k % 3] = v
+        gb[r.random((H, W)) < 0.002, 0] = 1.5
+        gb[r.random((H, W)) < 0.001, 3] = np.nan
+    src = acc if acc_f32 else acc.astype(np.float16).view(np.uint16)
+    got, _, _ = _run_noalloc(lib, torch, torch.device("cuda:0"), src, acc_f32, gb, W, H)
+    want = _oracle_chain(orc, src, acc_f32, gb, W, H)
+    nan = np.isnan(want.view(np.float16))
+    assert np.array_equal(nan, np.isnan(got.view(np.float16)))
+    assert np.array_equal(got[~nan], want[~nan])

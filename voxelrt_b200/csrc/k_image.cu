@@ -1,4 +1,4 @@
-// k_image.cu -- image-space passes (temporal, a-trous, present) and the
+// k_image.cu -- image-space passes (temporal, present) and the
 // brick/mask builders of the voxel world, for sm_100a.
 //
 // The image passes are HBM/L2-bound gathers: one thread per pixel in 32x8
@@ -25,17 +25,6 @@ __global__ void __launch_bounds__(256) k_temporal(Uni u, int W, int H, const uin
   if (gx >= W || gy >= H) return;
   const float4 res = temporal_pixel(u, W, H, gx, gy, rad, gcur, accPrev, kAccF32, gprev);
   store_px(accOut, kAccF32, (size_t)gy * W + gx, res);
-}
-
-// atrous.wgsl:26-83, one iteration at `step` (body in image_core.cuh).
-template <bool kSrcF32>
-__global__ void __launch_bounds__(256) k_atrous(int W, int H, const void* __restrict__ src,
-                                                const float4* __restrict__ gbuf, uint2* __restrict__ dst, int step) {
-  const int px = blockIdx.x * 32 + (threadIdx.x & 31);
-  const int py = blockIdx.y * 8 + (threadIdx.x >> 5);
-  if (px >= W || py >= H) return;
-  const float4 v = atrous_pixel(W, H, px, py, src, kSrcF32, gbuf, step);
-  dst[(size_t)py * W + px] = pack_h4(v.x, v.y, v.z, v.w);
 }
 
 // present.wgsl:40-55 as a compute pass writing a headless rgba8 buffer.  The
@@ -236,14 +225,6 @@ cudaError_t launch_temporal(const VrtUniforms& u, int W, int H, const void* rad1
   else
     k_temporal<false><<<grid, 256, 0, st>>>(to_uni(u), W, H, (const uint2*)rad16, (const float4*)gcur, acc_prev,
                                            (const float4*)gprev, acc_out);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_atrous(int W, int H, const void* src, bool src_f32, const void* gbuf, void* dst, int step,
-                          cudaStream_t st) {
-  dim3 grid((W + 31) / 32, (H + 7) / 8);
-  if (src_f32) k_atrous<true><<<grid, 256, 0, st>>>(W, H, src, (const float4*)gbuf, (uint2*)dst, step);
-  else k_atrous<false><<<grid, 256, 0, st>>>(W, H, src, (const float4*)gbuf, (uint2*)dst, step);
   return cudaGetLastError();
 }
 

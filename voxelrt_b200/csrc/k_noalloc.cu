@@ -22,10 +22,8 @@
 //   * the array needs no clearing: every pixel of it is written before it is
 //     read within one call.
 //
-// The iterations run the TMA-staged a-trous kernel (k_atrous_tma.cu), which
-// needs no memory beyond its tensor maps (kernel parameters); buffers that do
-// not meet its copy constraints (16-byte alignment; an even width for an
-// rgba16f source) take the unstaged kernel, which allocates nothing either.
+// The iterations run the frame loop's a-trous kernel (k_atrous.cu), which needs
+// no memory beyond its shared tiles.
 #include <cuda_runtime.h>
 #include <cstdint>
 #include "vrt_internal.h"
@@ -78,11 +76,9 @@ extern "C" int vrt_denoise_atrous_noalloc(const void* accum, int accum_f32, cons
   cudaStream_t st = (cudaStream_t)stream;
   // history -> out (step 1) -> scratch (step 2) -> out (step 4), the chain
   // accum -> dA -> dB -> dA of the frame loop with dA = out, dB = scratch.
-  // No error word is passed to the staged kernel: a tile whose bounded copy
-  // wait ran out is left unwritten and the call still returns.
-  e = launch_atrous_staged(width, height, accum, accum_f32 != 0, gbuf, out, 1, nullptr, st);
-  if (e == cudaSuccess) e = launch_atrous_staged(width, height, out, false, gbuf, scratch, 2, nullptr, st);
-  if (e == cudaSuccess) e = launch_atrous_staged(width, height, scratch, false, gbuf, out, 4, nullptr, st);
+  e = launch_atrous(width, height, accum, accum_f32 != 0, gbuf, out, 1, st);
+  if (e == cudaSuccess) e = launch_atrous(width, height, out, false, gbuf, scratch, 2, st);
+  if (e == cudaSuccess) e = launch_atrous(width, height, scratch, false, gbuf, out, 4, st);
   if (e != cudaSuccess) return vrt_noalloc_fail(VRT_ERR_CUDA, cudaGetErrorString(e));
   return VRT_OK;
 }

@@ -629,29 +629,6 @@ int vrt_session_autotune(VrtSession* s, const VrtUniforms* u, int frames, VrtTun
     win = s->tune;
     win_ms = best_tail;
   }
-  // the a-trous tile shape: the three iterations of a frame timed per shape
-  if (u->params0[2] & 2u) {
-    if (int r = vrt_pass_temporal(s, u)) { s->tune = keep; return r; }
-    float best_atrous = 1e30f;
-    int best_rows = win.atrous_rows;
-    for (int rows : {0, 16}) {
-      s->tune.atrous_rows = rows;
-      for (int it = 0; it < 3; it++)
-        if (int r = vrt_pass_atrous(s, u, it)) { s->tune = keep; return r; }   // warm-up
-      for (int f = 0; f < frames; f++) {
-        CUDA_TRY(cudaEventRecord(s->ev[0], st));
-        for (int it = 0; it < 3; it++)
-          if (int r = vrt_pass_atrous(s, u, it)) { s->tune = keep; return r; }
-        CUDA_TRY(cudaEventRecord(s->ev[1], st));
-        CUDA_TRY(cudaEventSynchronize(s->ev[1]));
-        CUDA_TRY(cudaEventElapsedTime(&ms[(size_t)f], s->ev[0], s->ev[1]));
-      }
-      std::sort(ms.begin(), ms.end());
-      if (ms[(size_t)frames / 2] < best_atrous) { best_atrous = ms[(size_t)frames / 2]; best_rows = rows; }
-    }
-    s->tune.atrous_rows = best_rows;
-    win = s->tune;
-  }
   if (best) {
     best->refill_min = win.refill_min;
     best->trace_blocks_per_sm = win.trace_blocks_per_sm;
@@ -857,8 +834,7 @@ int vrt_pass_atrous(VrtSession* s, const VrtUniforms* u, int it) {
   const void* src = it == 0 ? s->accum[p] : (it == 1 ? s->den[0] : s->den[1]);
   const bool src_f32 = it == 0 && s->acc_f32;
   void* dst = it == 1 ? s->den[1] : s->den[0];
-  CUDA_TRY(launch_atrous_staged(s->W, s->H, src, src_f32, s->gbuf[p], dst, 1 << it, s->stats + kStatError,
-                                s->ctx->stream, s->tune.atrous_rows));
+  CUDA_TRY(launch_atrous(s->W, s->H, src, src_f32, s->gbuf[p], dst, 1 << it, s->ctx->stream));
   s->launches++;
   return VRT_OK;
 }
@@ -937,7 +913,6 @@ int vrt_session_last_stats(VrtSession* s, VrtFrameStats* out) {
   out->pixels = h[kStatPixels];
   out->trace_step_slots = h[kStatTraceSlots];
   out->launches = s->launches;
-  if (h[kStatError]) return fail(VRT_ERR_TIMEOUT, "a bounded wait for staged image tiles ran out");
   out->cache_on = s->cache_on ? 1u : 0u;
   out->cache_queries = h[kStatCacheQueries];
   out->cache_samples = h[kStatCacheSamples];
@@ -1109,7 +1084,7 @@ int vrt_batch_destroy(VrtBatch* b) {
   cudaStreamSynchronize(c->stream);
   batch_drop_graph(b);
   dev_free(c, b->d_jobs, b->sessions.size() * sizeof(JobHost), &b->bytes);
-  dev_free(c, b->d_firsts, (3 * b->sessions.size() + 2) * 4, &b->bytes);
+  dev_free(c, b->d_firsts, (2 * b->sessions.size() + 1) * 4, &b->bytes);
   dev_free(c, b->wf_mem, b->wf_bytes, &b->bytes);
   dev_free(c, b->stats, kStatCount * 8, &b->bytes);
   if (b->h_jobs) cudaFreeHost(b->h_jobs);
@@ -1141,10 +1116,10 @@ static int batch_create_capacity(VrtCtx* ctx, VrtSession* const* sessions, int n
   b->wf_bytes = wavefront_bytes((int)b->P, 1, max_waves);
   int r = dev_alloc(ctx, &b->wf_mem, b->wf_bytes, &b->bytes);
   if (!r) r = dev_alloc(ctx, &b->d_jobs, (size_t)n * sizeof(JobHost), &b->bytes);
-  if (!r) r = dev_alloc(ctx, (void**)&b->d_firsts, (size_t)(3 * n + 2) * 4, &b->bytes);   // firsts, tile tables
+  if (!r) r = dev_alloc(ctx, (void**)&b->d_firsts, (size_t)(2 * n + 1) * 4, &b->bytes);   // firsts, tile table
   if (!r) r = dev_alloc(ctx, (void**)&b->stats, kStatCount * 8, &b->bytes);
   if (!r && (cudaMallocHost((void**)&b->h_jobs, (size_t)n * sizeof(JobHost)) != cudaSuccess ||
-             cudaMallocHost((void**)&b->h_firsts, (size_t)(3 * n + 2) * 4) != cudaSuccess))
+             cudaMallocHost((void**)&b->h_firsts, (size_t)(2 * n + 1) * 4) != cudaSuccess))
     r = fail(VRT_ERR_OOM, "pinned job table");
   if (!r && (cudaEventCreate(&b->ev_start) != cudaSuccess || cudaEventCreate(&b->ev_end) != cudaSuccess ||
              cudaEventCreateWithFlags(&b->ev_upload, cudaEventDisableTiming) != cudaSuccess))
@@ -1268,19 +1243,16 @@ static int batch_frame_impl(VrtBatch* b, const int* idx, int m, const VrtUniform
   }
   const uint32_t P = first;
   if (P > b->P) return fail(VRT_ERR_INVALID, "batch frame of %u pixels exceeds the pool's %u", P, b->P);
-  // a-trous tile tables: prefix counts of each job's 32 x 16 and 32 x 8 tiles
-  uint32_t* t16 = b->h_firsts + n;
-  uint32_t* t8 = t16 + n + 1;
-  t16[0] = t8[0] = 0u;
+  // a-trous tile table: prefix counts of each job's 32 x 32 tiles
+  uint32_t* tiles = b->h_firsts + n;
+  tiles[0] = 0u;
   for (int i = 0; i < m; i++) {
     const VrtSession* s = ss[(size_t)i];
-    const uint32_t tw = (uint32_t)(s->W + 31) / 32u;
-    t16[i + 1] = t16[i] + tw * (uint32_t)((s->H + 15) / 16);
-    t8[i + 1] = t8[i] + tw * (uint32_t)((s->H + 7) / 8);
+    tiles[i + 1] = tiles[i] + (uint32_t)((s->W + 31) / 32) * (uint32_t)((s->H + 31) / 32);
   }
-  const AtrousTiles at{b->d_firsts + n, b->d_firsts + 2 * n + 1, t16[m], t8[m]};
+  const AtrousTiles at{b->d_firsts + n, tiles[m]};
   CUDA_TRY(cudaMemcpyAsync(b->d_jobs, b->h_jobs, (size_t)m * sizeof(JobHost), cudaMemcpyHostToDevice, st));
-  CUDA_TRY(cudaMemcpyAsync(b->d_firsts, b->h_firsts, (size_t)(3 * n + 2) * 4, cudaMemcpyHostToDevice, st));
+  CUDA_TRY(cudaMemcpyAsync(b->d_firsts, b->h_firsts, (size_t)(2 * n + 1) * 4, cudaMemcpyHostToDevice, st));
   CUDA_TRY(cudaEventRecord(b->ev_upload, st));
   b->uploaded = true;
   CUDA_TRY(cudaMemsetAsync(b->stats, 0, kStatCount * 8, st));
@@ -1294,7 +1266,7 @@ static int batch_frame_impl(VrtBatch* b, const int* idx, int m, const VrtUniform
       CUDA_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed));
       uint32_t nl = 0;
       cudaError_t e = launch_batch_frame(b->d_jobs, b->d_firsts, m, max_bg, P, waves, b->wf, b->tune, b->stats, st, &nl,
-                                         b->ctx->present_lut, cls.data(), (int)cls.size(), &at);
+                                         b->ctx->present_lut, at, cls.data(), (int)cls.size());
       cudaError_t e2 = cudaStreamEndCapture(st, &graph);
       if (e != cudaSuccess || e2 != cudaSuccess) {
         if (graph) cudaGraphDestroy(graph);
@@ -1316,7 +1288,7 @@ static int batch_frame_impl(VrtBatch* b, const int* idx, int m, const VrtUniform
     CUDA_TRY(cudaGraphLaunch(b->gexec, st));
   } else {
     CUDA_TRY(launch_batch_frame(b->d_jobs, b->d_firsts, m, max_bg, P, waves, b->wf, b->tune, b->stats, st, &b->launches,
-                                b->ctx->present_lut, cls.data(), (int)cls.size(), &at));
+                                b->ctx->present_lut, at, cls.data(), (int)cls.size()));
   }
   CUDA_TRY(cudaEventRecord(b->ev_end, st));
   for (int i = 0; i < m; i++) {
@@ -1403,21 +1375,6 @@ int vrt_batch_autotune(VrtBatch* b, const VrtUniforms* u, int frames, VrtTuning*
   for (int tw : {2, 3, 4}) {
     b->tune = win;
     b->tune.tail_wave = tw;
-    int r = vrt_batch_frame(b, u);
-    for (int f = 0; f < frames && !r; f++) {
-      r = vrt_batch_frame(b, u);
-      VrtFrameStats st;
-      if (!r) r = vrt_batch_last_stats(b, &st);
-      ms[(size_t)f] = st.ms_total;
-    }
-    if (r) { b->tune = keep; b->use_graph = keep_graph; return r; }
-    std::sort(ms.begin(), ms.end());
-    if (ms[(size_t)frames / 2] < win_ms) { win_ms = ms[(size_t)frames / 2]; win = b->tune; }
-  }
-  // the a-trous tile rows (8 at every step, or 16 at steps 1-2)
-  {
-    b->tune = win;
-    b->tune.atrous_rows = win.atrous_rows == 16 ? 0 : 16;
     int r = vrt_batch_frame(b, u);
     for (int f = 0; f < frames && !r; f++) {
       r = vrt_batch_frame(b, u);

@@ -36,9 +36,8 @@ inline uint32_t recip_pad2(int BG) { return recip_up((uint32_t)(BG + 2) * (uint3
 // Per-frame counters written by the path kernel (u64 each).
 enum StatSlot {
   kStatRays = 0, kStatOuter, kStatInner, kStatVReads, kStatPixels, kStatCacheQueries, kStatCacheSamples,
-  kStatError,   // nonzero: a bounded wait on staged copies ran out
   kStatTraceSlots,   // lane step slots of the queue tracer: 32 x steps per pass x passes, per warp
-  kStatCount = 9
+  kStatCount = 8
 };
 static_assert(kStatRays == 0 && kStatOuter == 1 && kStatInner == 2 && kStatVReads == 3 && kStatPixels == 4,
               "block_flush_stats adds to the first five counters in this order");
@@ -97,7 +96,7 @@ struct WavefrontTuning {
   int shade_blocks_per_sm = 32;
   int trace_variant = 0;        // shape of the tracer (wf_dispatch_trace): (transition rounds per
                                 // warp-bookkeeping pass, steps per round, min blocks/SM)
-  int atrous_rows = 0;          // a-trous output tile rows: 0 or 8 = 8 at all steps, 16 = 16 at steps 1-2 and 8 at step 4
+  int atrous_rows = 0;          // kept from the caller's tuning; the a-trous tiles have one shape
   int tail_wave = -1;           // first wave whose paths finish one thread each (k_wf_tail); 0 = never;
                                 // -1 = automatic (auto_tail in wavefront_core.cuh)
 };
@@ -130,12 +129,11 @@ struct JobHost {
   CacheDev cache;
 };
 
-// The batch a-trous tile tables: per job, the prefix counts of its 32 x 16 and
-// 32 x 8 output tiles (m + 1 entries each, in device memory) and their totals.
+// The batch a-trous tile table: the prefix counts of the jobs' 32 x 32 output tiles (m + 1 entries in
+// device memory) and their total.
 struct AtrousTiles {
-  const uint32_t* d16;
-  const uint32_t* d8;
-  uint32_t n16, n8;
+  const uint32_t* first;
+  uint32_t n;
 };
 
 
@@ -164,8 +162,8 @@ struct CacheLaunch {
 // max_bg: the largest brick grid side of the jobs' scenes.
 cudaError_t launch_batch_frame(const void* d_jobs, const uint32_t* d_firsts, int n, int max_bg, uint32_t P, int waves,
                                const WavefrontBufs& wb, const WavefrontTuning& tune, unsigned long long* stats,
-                               cudaStream_t st, uint32_t* launches, const float* present_lut,
-                               const CacheLaunch* cls = nullptr, int ncl = 0, const AtrousTiles* at = nullptr);
+                               cudaStream_t st, uint32_t* launches, const float* present_lut, const AtrousTiles& at,
+                               const CacheLaunch* cls = nullptr, int ncl = 0);
 
 // Radiance-cache MLP kernels (k_mlp.cu).  q9: n x 9 floats (position in
 // metres, normal, albedo); y3: n x 3 target radiance; weights bf16 row-major.
@@ -262,11 +260,7 @@ cudaError_t launch_trace_rays(const SceneDev& s, const float* o, const float* d,
 cudaError_t launch_temporal(const VrtUniforms& u, int W, int H, const void* rad16, const void* gcur,
                             const void* acc_prev, const void* gprev, void* acc_out, bool acc_f32,
                             cudaStream_t st);
-// The a-trous iteration with its input tile staged by TMA (falls back to
-// launch_atrous when the buffers do not meet the copy constraints); err
-// (may be null) is set when a bounded wait for the copies ran out.
-cudaError_t launch_atrous_staged(int W, int H, const void* src, bool src_f32, const void* gbuf, void* dst, int step,
-                                 unsigned long long* err, cudaStream_t st, int rows = 0);
+// One a-trous iteration at step 1, 2 or 4.
 cudaError_t launch_atrous(int W, int H, const void* src, bool src_f32, const void* gbuf, void* dst, int step,
                           cudaStream_t st);
 // Present with the context's lookup table (kPresentLut 4-byte words: albedo
