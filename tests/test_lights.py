@@ -86,3 +86,23 @@ def test_light_build_matches_oracle(vrt, orc, kind, n, seed):
     np.testing.assert_array_equal(w2, ow2)
     np.testing.assert_array_equal(a2, orc.light_alias(ow2w))
     np.testing.assert_array_equal(g2, orc.light_grid(n, ow2, ow2w))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,fill", [(8, 0.3), (24, 0.02), (72, 0.0), (72, 0.004), (72, 0.08)])
+def test_light_build_sizes(vrt, orc, n, fill):
+    """One cell and cell counts that are no multiple of a block's, no light at all, few and many lights per
+    group; equal weights (ties), black lights (weight 0) and solid voxels between them."""
+    r = np.random.default_rng(n + int(1000 * fill))
+    vox = np.where(r.random(n ** 3) < 0.05, 0x00808080, 0).astype(np.uint32)
+    lit = r.random(n ** 3) < fill
+    colours = np.array([0xFFFFFFFF, 0x40FFFFFF, 0x40FFFFFF, 0x01000000, 0x80102030], np.uint32)
+    vox[lit] = colours[r.integers(0, len(colours), int(lit.sum()))]
+    ctx = vrt.Context(0)
+    sc = vrt.Scene(ctx, vox, n)
+    sc.build_lights()
+    words, alias, grid = sc.lights()
+    ow, oweights = orc.light_list(vox, n)
+    np.testing.assert_array_equal(words, ow)
+    np.testing.assert_array_equal(alias, orc.light_alias(oweights))
+    np.testing.assert_array_equal(grid, orc.light_grid(n, ow, oweights))
