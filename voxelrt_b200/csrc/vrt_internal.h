@@ -185,14 +185,14 @@ struct MlpTask {
   float extent;             // world size in metres
   int* step;                // Adam step counter (advanced by the reduction)
   float* partial;           // per-CTA gradient partials [mlp_max_ctas()][params]
-  float* loss;              // per-CTA loss sums
+  float* loss;              // per-CTA loss sums (host memory, mapped: read after a wait, without a copy)
   float* grad;              // reduced gradient
   float* wm;                // fp32 masters
   float* m;
   float* v;
   uint16_t* wbw;            // bf16 copy written by Adam (= wb)
   float lr;
-  int* err;                 // a bounded tensor-core wait ran out
+  int* err;                 // a bounded tensor-core wait ran out (host memory, mapped)
   int cta0, ctas;           // CTA range of the task (set by the launcher)
 };
 constexpr int kMaxMlpTasks = 48;
