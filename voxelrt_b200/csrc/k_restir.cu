@@ -1326,15 +1326,16 @@ VRT_DI void x1_of(const RestirDev& R, uint32_t g, F3& x1, F3& n1, F3& surf1) {
 
 struct URays {
   bool shadow = false, shadow2 = false, bounce = false;
+  bool lo = false;   // resolved into a vertex of estimateLo (or a bounce at x1): the active list's back part
 };
 
 // The path's candidate is final: reservoir A.
 VRT_DI void unified_finish(const RestirDev& R, uint32_t g, const Ris& ris) { store_ris(R.resA, g, R.u, R.W, R.H, ris); }
 
 // Runs x1's stages from the start of stage `st` (earlier stages resolved)
-// until a ray is pending (returned in rays, state saved) or the candidate
-// path ends.
-VRT_DI void x1_run(const RestirDev& R, const RestirWf& r, const WfDev& b, uint32_t g, uint32_t st, Ris& ris,
+// until a ray is pending (returned in rays, state saved); true when the
+// candidate path ends instead.
+VRT_DI bool x1_run(const RestirDev& R, const RestirWf& r, const WfDev& b, uint32_t g, uint32_t st, Ris& ris,
                    uint32_t& bits, uint32_t& rng, F3 x1, F3 n1, F3 surf1, URays& rays) {
   const Uni& u = R.u;
   if (st == kStLight) {   // light-list NEE at x1: RIS over emissive faces
@@ -1377,14 +1378,15 @@ VRT_DI void x1_run(const RestirDev& R, const RestirWf& r, const WfDev& b, uint32
       b.R1[g] = make_float4(brd.x, brd.y, brd.z, 1e4f);
       bits = bits_set(bits, 14, 2, kStBounce);
       rays.bounce = true;
+      rays.lo = true;
     } else {
-      unified_finish(R, g, ris);
-      return;
+      return true;
     }
   }
   ris_save(r, g, ris, bits);
   b.S0[g] = make_float4(0.0f, 0.0f, 0.0f, __uint_as_float(rng));
   r.x2[g] = make_float4(0.0f, 0.0f, 0.0f, __uint_as_float(bits));
+  return false;
 }
 
 // estimateLo's vertex v with unification (pathtrace.wgsl:213-244): sun shadow,
@@ -1470,20 +1472,20 @@ VRT_DI bool lo_vertex(const RestirDev& R, const WfDev& b, const RestirWf& r, uin
 }
 
 // The end of estimateLo: the bounce candidate at x2, then the final RIS.
-VRT_DI void lo_finish(const RestirDev& R, const RestirWf& r, uint32_t g, F3 Lo, uint32_t bits, uint32_t& rng) {
+VRT_DI void lo_finish(const RestirDev& R, const RestirWf& r, uint32_t g, F3 Lo, uint32_t bits, uint32_t& rng,
+                      Ris& ris) {
   F3 x1, n1, surf1;
   x1_of(R, g, x1, n1, surf1);
   const float4 x2c = r.x2[g];
   RSample s;
   float Wc;
   cand_point(x1, n1, xyz(x2c), normal_decode(bits_get(bits, 0, 6)), fclamp3(R, fclamp3(R, Lo)), s, Wc);
-  Ris ris = ris_load(r, g, bits);
+  ris = ris_load(r, g, bits);
   const float pt = eval_target(s, x1, n1);
   ris.add(s, pt, pt * Wc, rng);
-  unified_finish(R, g, ris);
 }
 
-__global__ void __launch_bounds__(256, 5) k_wf_unified_primary(const __grid_constant__ RestirDev R, RestirWf r,
+__global__ void __launch_bounds__(128, 10) k_wf_unified_primary(const __grid_constant__ RestirDev R, RestirWf r,
                                                             uint32_t P, WfDev b) {
   const uint32_t stride = gridDim.x * blockDim.x;
   if (R.stats && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(R.stats + kStatPixels, (unsigned long long)P);
@@ -1528,22 +1530,30 @@ __global__ void __launch_bounds__(256, 5) k_wf_unified_primary(const __grid_cons
           b.S0[g] = make_float4(0.0f, 0.0f, 0.0f, __uint_as_float(rng));
           r.x2[g] = make_float4(0.0f, 0.0f, 0.0f, __uint_as_float(bits_set(bits, 14, 2, kStSun)));
           rays.shadow = true;
-        } else {
-          x1_run(R, r, b, g, kStLight, ris, bits, rng, x1, n1, surf1, rays);
+        } else if (x1_run(R, r, b, g, kStLight, ris, bits, rng, x1, n1, surf1, rays)) {
+          unified_finish(R, g, ris);
         }
       }
     }
     const bool keep = rays.shadow || rays.shadow2 || rays.bounce;
-    emit2_block(b, 1, g, P, rays.shadow, rays.shadow2, rays.bounce, keep);
+    emit2_block(b, 1, g, P, rays.shadow, rays.shadow2, rays.bounce, keep, rays.lo);
   }
 }
 
-// Four blocks per SM (64 registers): the wave gathers scattered path state and
-// waits on it; ours 5.11 -> 5.05 ms per frame against three blocks at 80
-// registers (five at 48 registers spill ~1 KB and run slower).
-__global__ void __launch_bounds__(256, 4) k_wf_unified_wave(const __grid_constant__ RestirDev R, RestirWf r, WfDev b,
-                                                         int wave) {
-  const int n = b.ctr[4 * wave + 2];
+// Bound by instruction supply and divergence before it was laid out like this:
+// paths of all stages shared warps, a block's warps waited for the one with the
+// longest mix of stages, and the stages' code was expanded once per use
+// (no-instruction stalls up to 8 per issue).  So every stage's work appears
+// once -- the stages only say what to do next -- the active list keeps paths
+// whose x1 stages are open in front and those that bounce or walk estimateLo
+// at the back, and blocks are of 128 threads, 7 per SM (72 registers).  The five
+// waves of the 1080p `ours` frame: 788 -> 549 us (8 per SM, 64 registers: 577; 6:
+// 568; 5: 594).
+constexpr int kUnifiedThreads = 128;
+__global__ void __launch_bounds__(kUnifiedThreads, 7) k_wf_unified_wave(const __grid_constant__ RestirDev R, RestirWf r,
+                                                                       WfDev b, int wave) {
+  const int nfront = b.ctr[4 * wave + 2];
+  const int n = nfront + b.act2[wave];
   const uint32_t* list = active_of(b, wave);
   const Uni& u = R.u;
   const int stride = gridDim.x * blockDim.x;
@@ -1552,91 +1562,108 @@ __global__ void __launch_bounds__(256, 4) k_wf_unified_wave(const __grid_constan
     URays rays;
     uint32_t g = 0u;
     if (i < n) {
-      g = list[i];
+      g = i < nfront ? list[i] : list[b.acap - 1u - (uint32_t)(i - nfront)];
       const float4 s0 = b.S0[g];
       uint32_t rng = __float_as_uint(s0.w);
-      uint32_t bits = __float_as_uint(r.x2[g].w);
+      const float4 x2c = r.x2[g];
+      uint32_t bits = __float_as_uint(x2c.w);
       const uint32_t st = bits_get(bits, 14, 2);
       const uint4 h = b.hit[g];
+      const float t = __uint_as_float(h.x);
+      Ris ris;
+      bool finish = false;       // the candidate is final
+      bool vertex = false;       // a vertex of estimateLo at (pos, nrm) of material h.y is next
+      bool lo_ends = false;      // estimateLo ends with Lo
+      uint32_t v = 1u;
+      F3 pos, nrm, Lo = f3(0.0f, 0.0f, 0.0f), tp = f3(1.0f, 1.0f, 1.0f);
       if (st != kStLo) {
         F3 x1, n1, surf1;
         x1_of(R, g, x1, n1, surf1);
-        Ris ris = ris_load(r, g, bits);
-        if (st == kStSun) {   // the sun-cone shadow ray resolved
-          if (h.w == 0u) {
+        ris = ris_load(r, g, bits);
+        // the candidate that the resolved ray decides on, if it is one
+        RSample s = null_sample(0.0f);
+        float pt = 0.0f, Wc = 0.0f;
+        bool add = false;
+        if (st == kStSun) {          // the sun-cone shadow ray
+          add = h.w == 0u;
+          if (add) {
             const float4 l = b.R2[g];
             const float coneSA = kTwoPi * (1.0f - u.sunDir[3]);
-            RSample s = null_sample(0.0f);
             s.kind = kSkDir;
             s.pos = f3(l.x, l.y, l.z);
             const float den = fmax_(coneSA, 1e-5f);
             s.rad = f3(u.sunRadiance[0] / den, u.sunRadiance[1] / den, u.sunRadiance[2] / den);
-            const float pt = eval_target(s, x1, n1);
-            ris.add(s, pt, pt * coneSA, rng);
+            Wc = coneSA;
           }
-          x1_run(R, r, b, g, kStLight, ris, bits, rng, x1, n1, surf1, rays);
-        } else if (st == kStLight) {   // the light-list candidate's shadow ray resolved
-          if (h.w == 0u) {
+        } else if (st == kStLight) { // the light-list candidate's shadow ray
+          add = h.w == 0u;
+          if (add) {
             const float4 a = r.aux[g], a2 = r.aux2[g];
-            RSample eSel = null_sample(0.0f);
-            eSel.kind = kSkPoint;
-            eSel.pos = f3(a.x, a.y, a.z);
-            eSel.n = normal_decode(bits_get(bits, 16, 6));
-            eSel.rad = f3(a2.x, a2.y, a2.z);
-            const float We = a.w / a2.w;
-            ris.add(eSel, a2.w, a2.w * We, rng);
+            s.kind = kSkPoint;
+            s.pos = f3(a.x, a.y, a.z);
+            s.n = normal_decode(bits_get(bits, 16, 6));
+            s.rad = f3(a2.x, a2.y, a2.z);
+            pt = a2.w;
+            Wc = a.w / a2.w;
           }
-          x1_run(R, r, b, g, kStBounce, ris, bits, rng, x1, n1, surf1, rays);
-        } else {   // the bounce ray resolved: x2, or a sky direction candidate
+        } else {                     // the bounce ray: x2, or a sky direction candidate
           const F3 brd = xyz(b.R1[g]);
-          const float t = __uint_as_float(h.x);
           if (t < 0.0f) {
-            RSample s;
-            float Wc;
             cand_dir(u, n1, brd, s, Wc);
-            const float pt = eval_target(s, x1, n1);
-            ris.add(s, pt, pt * Wc, rng);
-            unified_finish(R, g, ris);
+            add = finish = true;
           } else {
-            const F3 x2 = surf1 + brd * t;
-            const F3 n2 = hit_normal((int)h.z, brd);
-            bits = bits_set(bits, 0, 6, normal_code(n2));
+            pos = surf1 + brd * t;
+            nrm = hit_normal((int)h.z, brd);
+            bits = bits_set(bits, 0, 6, normal_code(nrm));
             bits = bits_set(bits, 14, 2, kStLo);
             bits = bits_set(bits, 22, 8, 1u);
             ris_save(r, g, ris, bits);
-            r.x2[g] = make_float4(x2.x, x2.y, x2.z, __uint_as_float(bits));
-            if (!lo_vertex(R, b, r, g, 1u, x2, n2, unpack_material(h.y), f3(0.0f, 0.0f, 0.0f),
-                           f3(1.0f, 1.0f, 1.0f), rng, rays))
-              lo_finish(R, r, g, f3(0.0f, 0.0f, 0.0f), bits, rng);
+            r.x2[g] = make_float4(pos.x, pos.y, pos.z, __uint_as_float(bits));
+            vertex = true;
           }
         }
-      } else {   // estimateLo vertex (wave - 3) resolved: shadows, then the bounce hit
+        if (add) {
+          if (st != kStLight) pt = eval_target(s, x1, n1);
+          ris.add(s, pt, pt * Wc, rng);
+        }
+        if (st == kStSun || st == kStLight)
+          finish = x1_run(R, r, b, g, st == kStSun ? (uint32_t)kStLight : (uint32_t)kStBounce, ris, bits, rng, x1, n1,
+                          surf1, rays);
+      } else {   // estimateLo's vertex resolved: its shadows, then the bounce hit
         const float4 s1 = b.S1[g], s2 = b.S2[g];
         const uint32_t flags = __float_as_uint(s2.w);
-        F3 Lo = xyz(s0), tp = xyz(s1);
+        Lo = xyz(s0);
+        tp = xyz(s1);
         if ((flags & kFlagShadow) && h.w == 0u) Lo = Lo + xyz(s2);
         if ((flags & kFlagShadow2) && b.hit[g + (uint32_t)r.W * (uint32_t)r.H].w == 0u) Lo = Lo + xyz(r.aux[g]);
-        bool done = (flags & kFlagTerminal) != 0u;
-        if (!done) {
+        lo_ends = (flags & kFlagTerminal) != 0u;
+        if (!lo_ends) {
           const F3 rd = xyz(b.R1[g]);
-          const float t = __uint_as_float(h.x);
           if (t < 0.0f) {
             Lo = Lo + tp * sky_color(u, rd, false);
-            done = true;
+            lo_ends = true;
           } else {
-            const uint32_t v = bits_get(bits, 22, 8) + 1u;
+            v = bits_get(bits, 22, 8) + 1u;
             bits = bits_set(bits, 22, 8, v);
-            const float4 x2c = r.x2[g];
             r.x2[g] = make_float4(x2c.x, x2c.y, x2c.z, __uint_as_float(bits));
-            const F3 pos = xyz(b.R0[g]) + rd * t;
-            done = !lo_vertex(R, b, r, g, v, pos, hit_normal((int)h.z, rd), unpack_material(h.y), Lo, tp, rng, rays);
+            pos = xyz(b.R0[g]) + rd * t;
+            nrm = hit_normal((int)h.z, rd);
+            vertex = true;
           }
         }
-        if (done) lo_finish(R, r, g, Lo, bits, rng);
       }
+      if (vertex) {
+        lo_ends = !lo_vertex(R, b, r, g, v, pos, nrm, unpack_material(h.y), Lo, tp, rng, rays);
+        rays.lo = true;
+      }
+      if (lo_ends) {
+        lo_finish(R, r, g, Lo, bits, rng, ris);
+        finish = true;
+      }
+      if (finish) unified_finish(R, g, ris);
     }
     const bool keep = rays.shadow || rays.shadow2 || rays.bounce;
-    emit2_block(b, wave + 1, g, (uint32_t)r.W * (uint32_t)r.H, rays.shadow, rays.shadow2, rays.bounce, keep);
+    emit2_block(b, wave + 1, g, (uint32_t)r.W * (uint32_t)r.H, rays.shadow, rays.shadow2, rays.bounce, keep, rays.lo);
   }
 }
 
@@ -1734,8 +1761,8 @@ cudaError_t launch_restir_unified_wavefront(const SceneDev& s, const VrtUniforms
                    sc + 4 * (size_t)P};
   // x1's three sequential rays, then one wave per estimateLo vertex
   auto shade = [&](const WfDev& b, int w, int sblocks) {
-    if (w == 0) k_wf_unified_primary<<<sblocks, 256, 0, st>>>(R, r, P, b);
-    else k_wf_unified_wave<<<sblocks, 256, 0, st>>>(R, r, b, w);
+    if (w == 0) k_wf_unified_primary<<<sblocks * 2, 128, 0, st>>>(R, r, P, b);
+    else k_wf_unified_wave<<<sblocks * 2, kUnifiedThreads, 0, st>>>(R, r, b, w);
     return cudaGetLastError();
   };
   return wf_run_waves<SingleJob, decltype(shade), true>(job, P, (int)job.u.params0[1] + 4, wb, tune, out.stats,

@@ -36,7 +36,7 @@ static size_t queue_entries(size_t P, int slots) { return (slots > 1 ? 4 : 2) * 
 
 size_t wavefront_bytes(int W, int H, int max_waves, int slots) {
   const size_t P = (size_t)W * H;
-  return P * 16 * (4 + 3 * (size_t)slots) + queue_entries(P, slots) * 4 * 2 + P * 4 * 2 + (size_t)max_waves * 16;
+  return P * 16 * (4 + 3 * (size_t)slots) + queue_entries(P, slots) * 4 * 2 + P * 4 * 2 + (size_t)max_waves * 20;
 }
 
 void carve_wavefront(void* mem, size_t P, int max_waves, WavefrontBufs& wb, int slots) {
@@ -51,6 +51,7 @@ void carve_wavefront(void* mem, size_t P, int max_waves, WavefrontBufs& wb, int 
   for (int i = 0; i < 2; i++) { wb.q[i] = (uint32_t*)m; m += queue_entries(P, slots) * 4; }
   wb.qcap = queue_entries(P, slots);
   for (int i = 0; i < 2; i++) { wb.act[i] = (uint32_t*)m; m += P * 4; }
+  wb.acap = P;
   wb.ctr = (int*)m;
   wb.max_waves = max_waves;
   wb.slots = slots;

@@ -32,7 +32,10 @@ struct WfDev {
   uint32_t* a1;
   int* ctr;        // per wave k: [4k] shadow rays (queue front), [4k+1] queue head, [4k+2] active count,
                    // [4k+3] bounce rays (queue back)
+  int* act2;       // per wave k: paths at the back of the active list (a list in two parts: path i of the
+                   // back part sits at acap - 1 - i)
   uint32_t qcap;   // queue capacity in entries: bounce ray i of a wave sits at qcap - 1 - i
+  uint32_t acap;   // active-list capacity
 };
 
 // Ray queues: a wave's shadow rays are appended from the front, its bounce
@@ -388,9 +391,10 @@ VRT_DI bool shade_vertex(const Uni& u, const WfDev& b, uint32_t g, uint32_t k, F
 // block call it (block-uniform control flow).  Entries of a block are in
 // thread order; a path's results do not depend on the order of the queues.
 VRT_DI void block_append(int* c_front, int* c_back, int* c_act, int nf, int nb, bool act, uint32_t& fslot,
-                         uint32_t& bslot, uint32_t& aslot) {
-  __shared__ int s_cnt[3][8];
-  __shared__ int s_base[3];
+                         uint32_t& bslot, uint32_t& aslot, int* c_act2 = nullptr, bool act2 = false,
+                         uint32_t* a2slot = nullptr) {
+  __shared__ int s_cnt[4][8];
+  __shared__ int s_base[4];
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   int incf = nf, incb = nb;
@@ -401,24 +405,28 @@ VRT_DI void block_append(int* c_front, int* c_back, int* c_act, int nf, int nb, 
     if (lane >= o) { incf += vf; incb += vb; }
   }
   const unsigned ma = __ballot_sync(full, act);
+  const unsigned m2 = c_act2 ? __ballot_sync(full, act2) : 0u;
   if (lane == 31) { s_cnt[0][w] = incf; s_cnt[1][w] = incb; }
-  if (lane == 0) s_cnt[2][w] = __popc(ma);
+  if (lane == 0) { s_cnt[2][w] = __popc(ma); s_cnt[3][w] = __popc(m2); }
   __syncthreads();
-  if (threadIdx.x < 3) {   // thread 0: front, 1: back, 2: list
+  if (threadIdx.x < (c_act2 ? 4 : 3)) {   // thread 0: front, 1: back, 2: list, 3: the list's back part
     int tot = 0;
+    const int nw = (int)(blockDim.x >> 5);   // blocks of up to 256 threads
 #pragma unroll
     for (int k = 0; k < 8; k++) {
+      if (k >= nw) break;
       const int v = s_cnt[threadIdx.x][k];
       s_cnt[threadIdx.x][k] = tot;
       tot += v;
     }
-    int* c = threadIdx.x == 0 ? c_front : (threadIdx.x == 1 ? c_back : c_act);
+    int* c = threadIdx.x == 0 ? c_front : (threadIdx.x == 1 ? c_back : (threadIdx.x == 2 ? c_act : c_act2));
     s_base[threadIdx.x] = tot ? atomicAdd(c, tot) : 0;
   }
   __syncthreads();
   fslot = (uint32_t)(s_base[0] + s_cnt[0][w] + incf - nf);
   bslot = (uint32_t)(s_base[1] + s_cnt[1][w] + incb - nb);
   aslot = (uint32_t)(s_base[2] + s_cnt[2][w]) + (uint32_t)__popc(ma & ((1u << lane) - 1u));
+  if (c_act2) *a2slot = (uint32_t)(s_base[3] + s_cnt[3][w]) + (uint32_t)__popc(m2 & ((1u << lane) - 1u));
   __syncthreads();   // s_cnt / s_base are rewritten by the block's next call
 }
 
@@ -434,17 +442,19 @@ VRT_DI void emit_block(const WfDev& b, int next, uint32_t g, bool shadow, bool b
   if (keep) active_of(b, next)[as] = g;
 }
 
-// emit_block() with a second shadow ray of the path, traced as path g + P.
+// emit_block() with a second shadow ray of the path, traced as path g + P, and
+// the active list in two parts: paths with `back` set go to its back.
 VRT_DI void emit2_block(const WfDev& b, int next, uint32_t g, uint32_t P, bool shadow, bool shadow2, bool bounce,
-                        bool keep) {
-  uint32_t fs, bs, as;
+                        bool keep, bool back) {
+  uint32_t fs, bs, as, as2;
   int* c = b.ctr + 4 * next;
-  block_append(c, c + 3, c + 2, (int)shadow2 + (int)shadow, (int)bounce, keep, fs, bs, as);
+  block_append(c, c + 3, c + 2, (int)shadow2 + (int)shadow, (int)bounce, keep && !back, fs, bs, as, b.act2 + next,
+               keep && back, &as2);
   uint32_t* q = queue_of(b, next);
   if (shadow2) q[fs++] = (g + P) | kShadowBit;
   if (shadow) q[fs] = g | kShadowBit;
   if (bounce) q[b.qcap - 1u - bs] = g;
-  if (keep) active_of(b, next)[as] = g;
+  if (keep) active_of(b, next)[back ? b.acap - 1u - as2 : as] = g;
 }
 
 // ---------------------------------------------------------------------------
@@ -888,7 +898,9 @@ inline WfDev wf_view(const WavefrontBufs& w) {
   d.hit = (uint4*)w.hit;
   d.q0 = w.q[0]; d.q1 = w.q[1]; d.a0 = w.act[0]; d.a1 = w.act[1];
   d.ctr = w.ctr;
+  d.act2 = w.ctr + 4 * (size_t)w.max_waves;
   d.qcap = (uint32_t)w.qcap;
+  d.acap = (uint32_t)w.acap;
   return d;
 }
 
@@ -1034,7 +1046,7 @@ cudaError_t wf_run_waves(const J& jobs, uint32_t P, int waves, const WavefrontBu
                          int tail_from = 0) {
   if (waves + 1 > wb.max_waves) return cudaErrorInvalidValue;
   const WfDev b = wf_view(wb);
-  cudaError_t e = cudaMemsetAsync(wb.ctr, 0, (size_t)wb.max_waves * 16, st);
+  cudaError_t e = cudaMemsetAsync(wb.ctr, 0, (size_t)wb.max_waves * 20, st);
   if (e != cudaSuccess) return e;
   const int sms = wf_sm_count();
   const int refill = tune.refill_min > 0 ? tune.refill_min : 12;
