@@ -128,3 +128,11 @@ def test_tail_waves_leave_the_image(vrt, ctx, W, H, bounces):
         assert got == want, f"tail wave {tail}"
         s.close()
     sc.close()
+
+
+def test_stored_albedo_is_the_material_byte():
+    """rgba8unorm of sqrt(albedo) gives back each colour byte, in binary32 as the shader forms it."""
+    s = np.float32(1.0) / np.float32(255.0)
+    a = np.arange(256, dtype=np.float32) * s
+    q = np.clip(np.sqrt(a * a), np.float32(0.0), np.float32(1.0))
+    np.testing.assert_array_equal(np.floor(q * np.float32(255.0) + np.float32(0.5)).astype(np.int64), np.arange(256))

@@ -6,6 +6,7 @@
 // 512 B of rgba32f per request).
 #include "vrt_device.cuh"
 #include "image_core.cuh"
+#include "trace_kernel.cuh"
 #include "vrt_internal.h"
 #include <cstring>
 
@@ -186,12 +187,6 @@ __global__ void k_fill_box(uint32_t* __restrict__ vox, int N, int x0, int y0, in
 // ---------------------------------------------------------------------------
 // launch wrappers
 // ---------------------------------------------------------------------------
-static Uni to_uni(const VrtUniforms& u) {
-  Uni r;
-  std::memcpy(&r, &u, sizeof(Uni));
-  return r;
-}
-
 cudaError_t launch_build_bricks(const SceneDev& s, int bx0, int by0, int bz0, int bx1, int by1, int bz1,
                                 cudaStream_t st) {
   const int nbx = bx1 - bx0 + 1, nby = by1 - by0 + 1, nbz = bz1 - bz0 + 1;

@@ -460,8 +460,7 @@ VRT_DI void initial_pixel(const RestirDev& R, const uint32_t* occ, int gx, int g
   const F3 x1 = ro + rd * h0.t;
   const F3 n1 = h0.n;
   const F3 surf1 = x1 + n1 * fmax_(1e-3f, h0.t * 1e-4f);
-  R.alb8[p] = unorm8_(__fsqrt_rn(mat1.albedo.x)) | (unorm8_(__fsqrt_rn(mat1.albedo.y)) << 8) |
-              (unorm8_(__fsqrt_rn(mat1.albedo.z)) << 16) | (255u << 24);
+  R.alb8[p] = sqrt_albedo8(h0.mat);
   R.gbuf[p] = make_float4(n1.x, n1.y, n1.z, h0.t);
 
   const bool unified = rflag(u, kRfUnified);
@@ -1155,8 +1154,7 @@ __global__ void __launch_bounds__(256) k_wf_restir_primary(const __grid_constant
         const Mat mat1 = unpack_material(h.y);
         const F3 x1 = f3(u.camPos[0], u.camPos[1], u.camPos[2]) + rd * t;
         const F3 n1 = hit_normal((int)h.z, rd);
-        job.out.alb8[g] = unorm8_(__fsqrt_rn(mat1.albedo.x)) | (unorm8_(__fsqrt_rn(mat1.albedo.y)) << 8) |
-                          (unorm8_(__fsqrt_rn(mat1.albedo.z)) << 16) | (255u << 24);
+        job.out.alb8[g] = sqrt_albedo8(h.y);
         job.out.gbuf[g] = make_float4(n1.x, n1.y, n1.z, t);
         uint32_t rng = __float_as_uint(b.S0[g].w);
         const F3 surf1 = x1 + n1 * fmax_(1e-3f, t * 1e-4f);
@@ -1511,8 +1509,7 @@ __global__ void __launch_bounds__(128, 10) k_wf_unified_primary(const __grid_con
         const Mat mat1 = unpack_material(h.y);
         const F3 x1 = f3(u.camPos[0], u.camPos[1], u.camPos[2]) + rd * t;
         const F3 n1 = hit_normal((int)h.z, rd);
-        R.alb8[g] = unorm8_(__fsqrt_rn(mat1.albedo.x)) | (unorm8_(__fsqrt_rn(mat1.albedo.y)) << 8) |
-                    (unorm8_(__fsqrt_rn(mat1.albedo.z)) << 16) | (255u << 24);
+        R.alb8[g] = sqrt_albedo8(h.y);
         R.gbuf[g] = make_float4(n1.x, n1.y, n1.z, t);
         const float em = mat1.emissive * kEmissiveScale;   // unified: the sun goes through the reservoir
         R.direct[g] = pack_h4(em, em, em, 1.0f);
@@ -1743,8 +1740,8 @@ cudaError_t launch_restir_initial_wavefront(const SceneDev& s, const VrtUniforms
   unsigned long long* stats = out.stats;
   return wf_run_waves(job, P, (int)job.u.params0[1] + 2, wb, tune, stats, st, launches, trace_ev,
                       max_timed_waves, timed_waves, [&](const WfDev& b, int w, int sblocks) {
-                        if (w == 0) k_wf_restir_primary<<<sblocks, 256, 0, st>>>(job, r, P, b, stats);
-                        else k_wf_restir_wave<<<sblocks, 256, 0, st>>>(job, r, b, w);
+                        if (w == 0) k_wf_restir_primary<<<(sblocks + 1) / 2, 256, 0, st>>>(job, r, P, b, stats);
+                        else k_wf_restir_wave<<<(sblocks + 1) / 2, 256, 0, st>>>(job, r, b, w);
                         return cudaGetLastError();
                       });
 }
@@ -1761,8 +1758,8 @@ cudaError_t launch_restir_unified_wavefront(const SceneDev& s, const VrtUniforms
                    sc + 4 * (size_t)P};
   // x1's three sequential rays, then one wave per estimateLo vertex
   auto shade = [&](const WfDev& b, int w, int sblocks) {
-    if (w == 0) k_wf_unified_primary<<<sblocks * 2, 128, 0, st>>>(R, r, P, b);
-    else k_wf_unified_wave<<<sblocks * 2, kUnifiedThreads, 0, st>>>(R, r, b, w);
+    if (w == 0) k_wf_unified_primary<<<sblocks, 128, 0, st>>>(R, r, P, b);
+    else k_wf_unified_wave<<<sblocks, kUnifiedThreads, 0, st>>>(R, r, b, w);
     return cudaGetLastError();
   };
   return wf_run_waves<SingleJob, decltype(shade), true>(job, P, (int)job.u.params0[1] + 4, wb, tune, out.stats,

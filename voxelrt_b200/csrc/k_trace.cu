@@ -34,8 +34,7 @@ VRT_DI void path_pixel(const DScene& S, const uint32_t* occ, const Uni& u, float
   const Mat mat1 = unpack_material(h0.mat);
   const F3 x1 = ro + rd * h0.t;
   const F3 n1 = h0.n;
-  alb = unorm8_(__fsqrt_rn(mat1.albedo.x)) | (unorm8_(__fsqrt_rn(mat1.albedo.y)) << 8) |
-        (unorm8_(__fsqrt_rn(mat1.albedo.z)) << 16) | (255u << 24);
+  alb = sqrt_albedo8(h0.mat);
   gb = make_float4(n1.x, n1.y, n1.z, h0.t);
 
   F3 radiance = f3(0.0f, 0.0f, 0.0f);

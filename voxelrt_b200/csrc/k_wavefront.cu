@@ -59,7 +59,7 @@ void carve_wavefront(void* mem, size_t P, int max_waves, WavefrontBufs& wb, int 
 
 static SingleJob make_job(const SceneDev& s, const VrtUniforms& uu, float fclamp, int W, int H, const PathOut& out) {
   SingleJob job;
-  std::memcpy(&job.u, &uu, sizeof(Uni));
+  job.u = to_uni(uu);
   job.S = to_dscene(s);
   job.out.rad16 = (uint2*)out.rad16;
   job.out.rad32 = (float4*)out.rad32;

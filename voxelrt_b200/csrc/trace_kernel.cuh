@@ -32,8 +32,9 @@ inline DScene to_dscene(const SceneDev& s) {
 
 inline Uni to_uni(const VrtUniforms& u) {
   Uni r;
-  static_assert(sizeof(Uni) == sizeof(VrtUniforms), "uniform layouts differ");
-  std::memcpy(&r, &u, sizeof(Uni));
+  static_assert(offsetof(Uni, sunT) == sizeof(VrtUniforms), "uniform layouts differ");
+  std::memcpy(&r, &u, sizeof(VrtUniforms));
+  sun_frame(u.sunDir, r.sunT, r.sunB);
   return r;
 }
 

@@ -38,6 +38,17 @@ static int fail(int code, const char* fmt, ...) {
 
 int vrt::set_error(int code, const char* msg) { return fail(code, "%s", msg); }
 
+void vrt::sun_frame(const float w[4], float tang[4], float bitan[4]) {
+  const float a[3] = {std::fabs(w[0]) > 0.9f ? 0.0f : 1.0f, std::fabs(w[0]) > 0.9f ? 1.0f : 0.0f, 0.0f};
+  const float c[3] = {a[1] * w[2] - a[2] * w[1], a[2] * w[0] - a[0] * w[2], a[0] * w[1] - a[1] * w[0]};
+  const float l = std::sqrt((c[0] * c[0] + c[1] * c[1]) + c[2] * c[2]);
+  for (int k = 0; k < 3; k++) tang[k] = c[k] / l;
+  bitan[0] = w[1] * tang[2] - w[2] * tang[1];
+  bitan[1] = w[2] * tang[0] - w[0] * tang[2];
+  bitan[2] = w[0] * tang[1] - w[1] * tang[0];
+  tang[3] = bitan[3] = 0.0f;
+}
+
 #define CUDA_TRY(expr)                                                                           \
   do {                                                                                           \
     cudaError_t e_ = (expr);                                                                     \
@@ -1250,6 +1261,7 @@ static int batch_frame_impl(VrtBatch* b, const int* idx, int m, const VrtUniform
     std::memset(&j, 0, sizeof j);
     const int p = parity_of(s);
     j.u = u[i];
+    sun_frame(j.u.sunDir, j.sunT, j.sunB);
     j.vox = s->scene->dev.vox; j.cells = s->scene->dev.cells; j.bits = s->scene->dev.bits;
     j.N = s->scene->dev.N; j.BG = s->scene->dev.BG;
     j.rP = recip_pad(j.BG); j.rP2 = recip_pad2(j.BG);

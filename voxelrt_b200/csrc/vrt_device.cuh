@@ -7,6 +7,7 @@
 // which makes the results bit-identical to a scalar IEEE evaluation of the
 // same expressions on the host.
 #pragma once
+#include <cstddef>
 #include <cstdint>
 #include <cuda_fp16.h>
 
@@ -33,8 +34,11 @@ struct Uni {
   float params1[4];
   uint32_t params2[4];
   float params3[4], params4[4], params5[4], params6[4];
+  // Derived on the host, once per frame instead of once per sample: the
+  // tangent and bitangent of sampleSunDir's cone around sunDir.
+  float sunT[4], sunB[4];
 };
-static_assert(sizeof(Uni) == 304, "uniform block is 304 bytes");
+static_assert(offsetof(Uni, sunT) == 304 && sizeof(Uni) == 336, "the uniform block is 304 bytes");
 
 // ---------------------------------------------------------------------------
 // Scalar helpers.  min/max are written as selects so that signed zeros and
@@ -282,9 +286,8 @@ VRT_DI F3 sample_sun_dir(const Uni& u, uint32_t& rng) {
   float sinT = __fsqrt_rn(fmax_(0.0f, 1.0f - cosT * cosT));
   float phi = kTwoPi * ry;
   F3 w = f3(u.sunDir[0], u.sunDir[1], u.sunDir[2]);
-  F3 a = fabsf(w.x) > 0.9f ? f3(0.0f, 1.0f, 0.0f) : f3(1.0f, 0.0f, 0.0f);
-  F3 tang = normalize3(cross3(a, w));
-  F3 bitan = cross3(w, tang);
+  F3 tang = f3(u.sunT[0], u.sunT[1], u.sunT[2]);
+  F3 bitan = f3(u.sunB[0], u.sunB[1], u.sunB[2]);
   float sp, cp;
   sincos_(phi, sp, cp);
   return normalize3((tang * (cp * sinT) + bitan * (sp * sinT)) + w * cosT);
@@ -296,7 +299,10 @@ VRT_DI F3 cosine_hemisphere(F3 n, uint32_t& rng) {
   float phi = kTwoPi * rx;
   float sr = __fsqrt_rn(ry);
   F3 a = fabsf(n.x) > 0.9f ? f3(0.0f, 1.0f, 0.0f) : f3(1.0f, 0.0f, 0.0f);
-  F3 tang = normalize3(cross3(a, n));
+  // normals lie along an axis, where the cross product has length 1 and
+  // dividing by it changes nothing
+  F3 tang = cross3(a, n);
+  if (dot3(tang, tang) != 1.0f) tang = normalize3(tang);
   F3 bitan = cross3(n, tang);
   float sp, cp;
   sincos_(phi, sp, cp);
@@ -305,6 +311,10 @@ VRT_DI F3 cosine_hemisphere(F3 n, uint32_t& rng) {
 
 // Material unpack (voxel.wgsl:41-51)
 struct Mat { F3 albedo; float emissive; };
+// The stored albedo (rgba8unorm of sqrt(albedo)) of material m: albedo is the
+// square of byte / 255, whose square root is byte / 255 again and rounds to the
+// byte.
+VRT_DI uint32_t sqrt_albedo8(uint32_t m) { return (m & 0xffffffu) | 0xff000000u; }
 VRT_DI Mat unpack_material(uint32_t m) {
   const float s = 1.0f / 255.0f;
   F3 a = f3((float)(m & 0xffu), (float)((m >> 8) & 0xffu), (float)((m >> 16) & 0xffu)) * s;

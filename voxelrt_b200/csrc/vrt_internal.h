@@ -6,6 +6,11 @@
 
 namespace vrt {
 
+// The orthonormal frame of sampleSunDir (common.wgsl:112-124) around the sun's direction w: tangent
+// normalize(cross(a, w)) and bitangent cross(w, tangent) -- single binary32 operations in the shader's order,
+// so the values are those the kernels formed per sample.
+void sun_frame(const float w[4], float tang[4], float bitan[4]);
+
 // Device-resident scene: packed voxels, per-brick words and masks, plus the
 // 1-bit-per-brick occupancy bitmap the per-thread traversal stages in shared
 // memory and the padded one the queue tracer walks (dda_walk.cuh).
@@ -106,6 +111,7 @@ struct WavefrontTuning {
 // one session rendered inside a batch frame.  Same field order and layout.
 struct JobHost {
   VrtUniforms u;
+  float sunT[4], sunB[4];   // sun_frame(u.sunDir)
   const uint32_t* vox;
   const uint32_t* cells;
   const uint32_t* bits;

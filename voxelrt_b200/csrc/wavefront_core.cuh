@@ -601,6 +601,8 @@ __global__ void __launch_bounds__(kTraceThreads, kMinB) k_wf_trace(J jobs, WfDev
   }
 }
 
+constexpr int kShadeThreads = 128;
+
 // shade(0): primary hits over all pixels.  The shading kernels are bound by
 // instruction issue (77% of the issue slots on a 1080p frame) and run 1280
 // threads per SM (48 registers; 6 x 256 threads spill and gain nothing), in
@@ -608,7 +610,7 @@ __global__ void __launch_bounds__(kTraceThreads, kMinB) k_wf_trace(J jobs, WfDev
 // instead of eight (cache frames 1.040 -> 1.024 ms of path tracing against
 // blocks of 256; plain frames equal).
 template <class J>
-__global__ void __launch_bounds__(128, 10) k_wf_shade_primary(J jobs, uint32_t P, WfDev b, unsigned long long* stats) {
+__global__ void __launch_bounds__(kShadeThreads, 1280 / kShadeThreads) k_wf_shade_primary(J jobs, uint32_t P, WfDev b, unsigned long long* stats) {
   const bool any_cache = jobs.any_cache();
   const CacheDev* ccp = nullptr;
   const uint32_t stride = gridDim.x * blockDim.x;
@@ -639,8 +641,7 @@ __global__ void __launch_bounds__(128, 10) k_wf_shade_primary(J jobs, uint32_t P
         const F3 ro = f3(u.camPos[0], u.camPos[1], u.camPos[2]);
         const F3 x1 = ro + rd * t;
         const F3 n1 = hit_normal((int)h.z, rd);
-        out.alb8[lp] = unorm8_(__fsqrt_rn(mat1.albedo.x)) | (unorm8_(__fsqrt_rn(mat1.albedo.y)) << 8) |
-                       (unorm8_(__fsqrt_rn(mat1.albedo.z)) << 16) | (255u << 24);
+        out.alb8[lp] = sqrt_albedo8(h.y);
         out.gbuf[lp] = make_float4(n1.x, n1.y, n1.z, t);
         uint32_t rng = __float_as_uint(s0w);
         F3 radiance = f3(0.0f, 0.0f, 0.0f), tp = f3(1.0f, 1.0f, 1.0f);
@@ -664,7 +665,7 @@ __global__ void __launch_bounds__(128, 10) k_wf_shade_primary(J jobs, uint32_t P
 
 // shade(k), k >= 1: resolve vertex k-1's shadow ray, then the bounce hit.
 template <class J>
-__global__ void __launch_bounds__(128, 10) k_wf_shade(J jobs, WfDev b, int wave) {
+__global__ void __launch_bounds__(kShadeThreads, 1280 / kShadeThreads) k_wf_shade(J jobs, WfDev b, int wave) {
   const bool any_cache = jobs.any_cache();
   const int n = b.ctr[4 * wave + 2];
   const uint32_t* list = active_of(b, wave);
@@ -1054,7 +1055,10 @@ cudaError_t wf_run_waves(const J& jobs, uint32_t P, int waves, const WavefrontBu
   if (e != cudaSuccess) return e;
   const int sms = wf_sm_count();
   const int refill = tune.refill_min > 0 ? tune.refill_min : 12;
-  const int sblocks = sms * (tune.shade_blocks_per_sm > 0 ? tune.shade_blocks_per_sm : 32);
+  // shading blocks (the tuning counts them as blocks of 256 threads), no more than the pixels need: the full
+  // grid's idle blocks cost 2 us of a 320x180 frame's 175
+  const int sblocks = std::min(sms * (tune.shade_blocks_per_sm > 0 ? tune.shade_blocks_per_sm : 32) * (256 / kShadeThreads),
+                               (int)((P + kShadeThreads - 1) / kShadeThreads));
   uint32_t nl = 0;
   k_wf_generate<J><<<(P + 255) / 256, 256, 0, st>>>(jobs, P, b);
   nl++;
@@ -1134,8 +1138,8 @@ cudaError_t wf_launch_frame(const J& jobs, uint32_t P, int waves, const Wavefron
   }
   return wf_run_waves(jobs, P, waves, wb, tune, stats, st, launches, trace_ev, max_timed_waves, timed_waves,
                       [&](const WfDev& b, int w, int sblocks) {
-                        if (w == 0) k_wf_shade_primary<J><<<sblocks * 2, 128, 0, st>>>(jobs, P, b, stats);
-                        else k_wf_shade<J><<<sblocks * 2, 128, 0, st>>>(jobs, b, w);
+                        if (w == 0) k_wf_shade_primary<J><<<sblocks, kShadeThreads, 0, st>>>(jobs, P, b, stats);
+                        else k_wf_shade<J><<<sblocks, kShadeThreads, 0, st>>>(jobs, b, w);
                         return cudaGetLastError();
                       }, tail_from);
 }
