@@ -130,6 +130,30 @@ def test_tail_waves_leave_the_image(vrt, ctx, W, H, bounces):
     sc.close()
 
 
+# The kernels of a frame overlap the launch of the next one; a session with
+# timing on has an event between its passes, which orders them fully.
+@pytest.mark.parametrize("preset", ["base", "ours"])
+@pytest.mark.parametrize("W,H", [(33, 17), (401, 297), (1283, 721)])
+def test_overlapped_frames_match_ordered_frames(vrt, ctx, W, H, preset):
+    vox, spawn = vrt.generate_scene(vrt.VRT_SCENE_FULL, 64, 7)
+    sc = vrt.Scene(ctx, vox, 64)
+    lights = int(sc.build_lights().count) if preset != "base" else 0
+    us = [vrt.make_uniforms(vrt.camera_spline(spawn, f), vrt.camera_spline(spawn, max(f - 1, 0)), vrt.Lighting(), f,
+                            2, 3, W, H, preset=preset, light_count=lights) for f in range(12)]
+    got = []
+    for ordered in (True, False):
+        s = vrt.Session(ctx, sc, W, H, keep_radiance_f32=True)
+        s.set_timing(ordered)
+        for u in us:
+            s.frame(u)
+            if ordered:
+                ctx.synchronize()
+        got.append((s.radiance_f32().tobytes(), s.ldr().tobytes()))
+        s.close()
+    assert got[0] == got[1]
+    sc.close()
+
+
 def test_stored_albedo_is_the_material_byte():
     """rgba8unorm of sqrt(albedo) gives back each colour byte, in binary32 as the shader forms it."""
     s = np.float32(1.0) / np.float32(255.0)

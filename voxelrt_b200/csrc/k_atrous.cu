@@ -18,6 +18,7 @@ namespace vrt {
 template <int S, int R, bool kSrcF32>
 __global__ void __launch_bounds__(8 * R, 96 / R) k_atrous(int W, int H, const void* __restrict__ src,
                                                           const float4* __restrict__ gbuf, uint2* __restrict__ dst) {
+  frame_begin();
   extern __shared__ float4 sm[];
   atrous_tile<S, R>(sm, AtrousImage{W, H, src, kSrcF32, gbuf, dst}, blockIdx.x * kAtrousTile, blockIdx.y * R);
 }
@@ -29,7 +30,7 @@ static cudaError_t run_tiles(int W, int H, const void* src, const void* gbuf, vo
   const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, G::smem);
   if (e != cudaSuccess) return e;
   const dim3 grid((W + kAtrousTile - 1) / kAtrousTile, (H + R - 1) / R);
-  fn<<<grid, G::threads, G::smem, st>>>(W, H, src, (const float4*)gbuf, (uint2*)dst);
+  launch_after(fn, grid, G::threads, G::smem, st, W, H, src, (const float4*)gbuf, (uint2*)dst);
   return cudaGetLastError();
 }
 

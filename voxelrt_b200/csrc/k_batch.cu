@@ -26,6 +26,7 @@ static_assert(offsetof(JobDev, cache) == offsetof(JobHost, cache), "job table la
 
 // temporal.wgsl:17-77 over all jobs.
 __global__ void __launch_bounds__(256) k_b_temporal(MultiJob J, uint32_t P) {
+  frame_begin();
   const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= P) return;
   const int j = J.job_of(g);
@@ -46,6 +47,7 @@ constexpr int kBatchRows = 32;   // tile rows
 template <int S>
 __global__ void __launch_bounds__(8 * kBatchRows, 96 / kBatchRows) k_b_atrous(MultiJob J,
                                                                              const uint32_t* __restrict__ tiles) {
+  frame_begin();
   extern __shared__ float4 sm[];
   const uint32_t b = blockIdx.x;
   int lo = 0, hi = J.n - 1;
@@ -68,12 +70,13 @@ static cudaError_t launch_b_atrous(const MultiJob& J, const AtrousTiles& at, cud
   const cudaError_t e =
       cudaFuncSetAttribute(k_b_atrous<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, G::smem);
   if (e != cudaSuccess) return e;
-  k_b_atrous<S><<<at.n, G::threads, G::smem, st>>>(J, at.first);
+  launch_after(k_b_atrous<S>, at.n, G::threads, G::smem, st, J, at.first);
   return cudaGetLastError();
 }
 
 // present.wgsl:40-55 over all jobs.
 __global__ void __launch_bounds__(256) k_b_present(MultiJob J, uint32_t P, const float* __restrict__ lut) {
+  frame_begin();
   const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= P) return;
   const int j = J.job_of(g);
@@ -100,11 +103,11 @@ cudaError_t launch_batch_frame(const void* d_jobs, const uint32_t* d_firsts, int
   // the cache jobs' inference, resolve and training, all jobs per launch
   if (ncl > 0 && (e = launch_cache_post(J, wf_view(wb), cls, ncl, stats, st, launches)) != cudaSuccess) return e;
   const unsigned blocks = (P + 255) / 256;
-  k_b_temporal<<<blocks, 256, 0, st>>>(J, P);
+  launch_after(k_b_temporal, blocks, 256, 0, st, J, P);
   if ((e = launch_b_atrous<1>(J, at, st)) != cudaSuccess || (e = launch_b_atrous<2>(J, at, st)) != cudaSuccess ||
       (e = launch_b_atrous<4>(J, at, st)) != cudaSuccess)
     return e;
-  k_b_present<<<blocks, 256, 0, st>>>(J, P, present_lut);
+  launch_after(k_b_present, blocks, 256, 0, st, J, P, present_lut);
   if (launches) *launches += 5;
   return cudaGetLastError();
 }

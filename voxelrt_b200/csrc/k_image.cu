@@ -21,6 +21,7 @@ template <bool kAccF32>
 __global__ void __launch_bounds__(256) k_temporal(Uni u, int W, int H, const uint2* __restrict__ rad,
                                                   const float4* __restrict__ gcur, const void* __restrict__ accPrev,
                                                   const float4* __restrict__ gprev, void* __restrict__ accOut) {
+  frame_begin();
   const int gx = blockIdx.x * 32 + (threadIdx.x & 31);
   const int gy = blockIdx.y * 8 + (threadIdx.x >> 5);
   if (gx >= W || gy >= H) return;
@@ -37,6 +38,7 @@ template <bool kFinF32>
 __global__ void __launch_bounds__(256) k_present(float exposure, uint32_t P, uint32_t n4,
                                                  const void* __restrict__ fin, const uint32_t* __restrict__ alb8,
                                                  uint32_t* __restrict__ ldr, const float* __restrict__ lut) {
+  frame_begin();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n4) {
     float4 il[4];
@@ -215,10 +217,10 @@ cudaError_t launch_temporal(const VrtUniforms& u, int W, int H, const void* rad1
                             const void* acc_prev, const void* gprev, void* acc_out, bool acc_f32, cudaStream_t st) {
   dim3 grid((W + 31) / 32, (H + 7) / 8);
   if (acc_f32)
-    k_temporal<true><<<grid, 256, 0, st>>>(to_uni(u), W, H, (const uint2*)rad16, (const float4*)gcur, acc_prev,
+    launch_after(k_temporal<true>, grid, 256, 0, st, to_uni(u), W, H, (const uint2*)rad16, (const float4*)gcur, acc_prev,
                                           (const float4*)gprev, acc_out);
   else
-    k_temporal<false><<<grid, 256, 0, st>>>(to_uni(u), W, H, (const uint2*)rad16, (const float4*)gcur, acc_prev,
+    launch_after(k_temporal<false>, grid, 256, 0, st, to_uni(u), W, H, (const uint2*)rad16, (const float4*)gcur, acc_prev,
                                            (const float4*)gprev, acc_out);
   return cudaGetLastError();
 }
@@ -231,8 +233,8 @@ cudaError_t launch_present(const VrtUniforms& u, int W, int H, const void* fin, 
   const uint32_t n4 = aligned ? P >> 2 : 0u;
   const uint32_t threads = n4 + (P - 4u * n4);
   const unsigned blocks = (threads + 255u) / 256u;
-  if (fin_f32) k_present<true><<<blocks, 256, 0, st>>>(u.params1[2], P, n4, fin, alb8, ldr, lut);
-  else k_present<false><<<blocks, 256, 0, st>>>(u.params1[2], P, n4, fin, alb8, ldr, lut);
+  if (fin_f32) launch_after(k_present<true>, blocks, 256, 0, st, u.params1[2], P, n4, fin, alb8, ldr, lut);
+  else launch_after(k_present<false>, blocks, 256, 0, st, u.params1[2], P, n4, fin, alb8, ldr, lut);
   return cudaGetLastError();
 }
 

@@ -566,6 +566,7 @@ VRT_DI bool valid_prev(const RestirDev& R, int px, int py, F3 wp, F3 n1) {
 // Five blocks per SM (48 registers) for the per-pixel reuse and wave kernels below:
 // they wait on scattered reservoir, G-buffer and path-state reads (gi 2.87 -> 2.77 ms).
 __global__ void __launch_bounds__(256, 5) k_restir_temporal(const __grid_constant__ RestirDev R) {
+  frame_begin();
   int gx, gy;
   block_pixel_16x16(gx, gy);
   if (gx >= R.W || gy >= R.H) return;
@@ -965,6 +966,7 @@ __global__ void __launch_bounds__(256) k_restir_spatial(const __grid_constant__ 
 template <bool kVector>
 __global__ void __launch_bounds__(256, 3) k_restir_spatial_select(const __grid_constant__ RestirDev R, WfDev b,
                                                                int wave) {
+  frame_begin();
   int gx, gy;
   block_pixel_16x16(gx, gy);
   const uint32_t P = (uint32_t)R.W * (uint32_t)R.H;
@@ -990,6 +992,7 @@ __global__ void __launch_bounds__(256, 3) k_restir_spatial_select(const __grid_c
 
 __global__ void __launch_bounds__(256) k_restir_spatial_resolve(const __grid_constant__ RestirDev R, WfDev b,
                                                                 int wave) {
+  frame_begin();
   const int n = b.ctr[4 * wave + 2];
   const uint32_t* list = active_of(b, wave);
   const uint32_t P = (uint32_t)R.W * (uint32_t)R.H;
@@ -1014,6 +1017,7 @@ __global__ void __launch_bounds__(256) k_restir_spatial_resolve(const __grid_con
 // 16 x 16 tile and its 4-pixel halo are staged in shared memory as (seed,
 // non-null) pairs; the count is an integer, so the window order is free.
 __global__ void __launch_bounds__(256) k_restir_dupmap(const __grid_constant__ RestirDev R) {
+  frame_begin();
   constexpr int kHalo = 4, kT = 16 + 2 * kHalo;
   __shared__ uint32_t s_seed[kT * kT];
   __shared__ uint8_t s_live[kT * kT];
@@ -1130,6 +1134,7 @@ VRT_DI void finish_point(const SingleJob& job, const RestirWf& r, uint32_t g, F3
 
 __global__ void __launch_bounds__(256) k_wf_restir_primary(const __grid_constant__ SingleJob job, RestirWf r,
                                                            uint32_t P, WfDev b, unsigned long long* stats) {
+  frame_begin();
   const uint32_t stride = gridDim.x * blockDim.x;
   if (stats && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(stats + kStatPixels, (unsigned long long)P);
   const Uni& u = job.u;
@@ -1194,6 +1199,7 @@ __global__ void __launch_bounds__(256) k_wf_restir_primary(const __grid_constant
 
 __global__ void __launch_bounds__(256, 5) k_wf_restir_wave(const __grid_constant__ SingleJob job, RestirWf r, WfDev b,
                                                         int wave) {
+  frame_begin();
   const int n = b.ctr[4 * wave + 2];
   const uint32_t* list = active_of(b, wave);
   const Uni& u = job.u;
@@ -1485,6 +1491,7 @@ VRT_DI void lo_finish(const RestirDev& R, const RestirWf& r, uint32_t g, F3 Lo, 
 
 __global__ void __launch_bounds__(128, 10) k_wf_unified_primary(const __grid_constant__ RestirDev R, RestirWf r,
                                                             uint32_t P, WfDev b) {
+  frame_begin();
   const uint32_t stride = gridDim.x * blockDim.x;
   if (R.stats && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(R.stats + kStatPixels, (unsigned long long)P);
   const Uni& u = R.u;
@@ -1549,6 +1556,7 @@ __global__ void __launch_bounds__(128, 10) k_wf_unified_primary(const __grid_con
 constexpr int kUnifiedThreads = 128;
 __global__ void __launch_bounds__(kUnifiedThreads, 7) k_wf_unified_wave(const __grid_constant__ RestirDev R, RestirWf r,
                                                                        WfDev b, int wave) {
+  frame_begin();
   const int nfront = b.ctr[4 * wave + 2];
   const int n = nfront + b.act2[wave];
   const uint32_t* list = active_of(b, wave);
@@ -1740,8 +1748,8 @@ cudaError_t launch_restir_initial_wavefront(const SceneDev& s, const VrtUniforms
   unsigned long long* stats = out.stats;
   return wf_run_waves(job, P, (int)job.u.params0[1] + 2, wb, tune, stats, st, launches, trace_ev,
                       max_timed_waves, timed_waves, [&](const WfDev& b, int w, int sblocks) {
-                        if (w == 0) k_wf_restir_primary<<<(sblocks + 1) / 2, 256, 0, st>>>(job, r, P, b, stats);
-                        else k_wf_restir_wave<<<(sblocks + 1) / 2, 256, 0, st>>>(job, r, b, w);
+                        if (w == 0) launch_after(k_wf_restir_primary, (sblocks + 1) / 2, 256, 0, st, job, r, P, b, stats);
+                        else launch_after(k_wf_restir_wave, (sblocks + 1) / 2, 256, 0, st, job, r, b, w);
                         return cudaGetLastError();
                       });
 }
@@ -1758,8 +1766,8 @@ cudaError_t launch_restir_unified_wavefront(const SceneDev& s, const VrtUniforms
                    sc + 4 * (size_t)P};
   // x1's three sequential rays, then one wave per estimateLo vertex
   auto shade = [&](const WfDev& b, int w, int sblocks) {
-    if (w == 0) k_wf_unified_primary<<<sblocks, 128, 0, st>>>(R, r, P, b);
-    else k_wf_unified_wave<<<sblocks, kUnifiedThreads, 0, st>>>(R, r, b, w);
+    if (w == 0) launch_after(k_wf_unified_primary, sblocks, 128, 0, st, R, r, P, b);
+    else launch_after(k_wf_unified_wave, sblocks, kUnifiedThreads, 0, st, R, r, b, w);
     return cudaGetLastError();
   };
   return wf_run_waves<SingleJob, decltype(shade), true>(job, P, (int)job.u.params0[1] + 4, wb, tune, out.stats,
@@ -1769,7 +1777,7 @@ cudaError_t launch_restir_unified_wavefront(const SceneDev& s, const VrtUniforms
 cudaError_t launch_restir_temporal(const SceneDev& s, const VrtUniforms& u, int W, int H, const PathOut& out,
                                    const RestirBufs& rb, cudaStream_t st) {
   const RestirDev R = restir_dev(s, u, 0.0f, W, H, out, rb);
-  k_restir_temporal<<<dim3((W + 15) / 16, (H + 15) / 16), 256, 0, st>>>(R);
+  launch_after(k_restir_temporal, dim3((W + 15) / 16, (H + 15) / 16), 256, 0, st, R);
   return cudaGetLastError();
 }
 
@@ -1783,7 +1791,7 @@ cudaError_t launch_restir_dupmap(const VrtUniforms& u, int W, int H, const Resti
   SceneDev none;
   PathOut out;
   const RestirDev R = restir_dev(none, u, 0.0f, W, H, out, rb);
-  k_restir_dupmap<<<dim3((W + 15) / 16, (H + 15) / 16), 256, 0, st>>>(R);
+  launch_after(k_restir_dupmap, dim3((W + 15) / 16, (H + 15) / 16), 256, 0, st, R);
   return cudaGetLastError();
 }
 
@@ -1797,15 +1805,15 @@ cudaError_t launch_restir_spatial_wavefront(const SceneDev& s, const VrtUniforms
   cudaError_t e = cudaMemsetAsync(wb.ctr, 0, 16, st);
   if (e != cudaSuccess) return e;
   const dim3 grid((W + 15) / 16, (H + 15) / 16);
-  if (u.params2[0] & kRfVector) k_restir_spatial_select<true><<<grid, 256, 0, st>>>(R, b, wave);
-  else k_restir_spatial_select<false><<<grid, 256, 0, st>>>(R, b, wave);
+  if (u.params2[0] & kRfVector) launch_after(k_restir_spatial_select<true>, grid, 256, 0, st, R, b, wave);
+  else launch_after(k_restir_spatial_select<false>, grid, 256, 0, st, R, b, wave);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   const int sms = wf_sm_count();
   const int refill = tune.refill_min > 0 ? tune.refill_min : 12;
   e = wf_dispatch_trace<SingleJob, true>(tune.trace_variant, job, tune.trace_blocks_per_sm, sms, b, wave, 0, refill,
                                          out.stats, st);
   if (e != cudaSuccess) return e;
-  k_restir_spatial_resolve<<<sms * 8, 256, 0, st>>>(R, b, wave);
+  launch_after(k_restir_spatial_resolve, sms * 8, 256, 0, st, R, b, wave);
   if (launches) *launches += 3;
   return cudaGetLastError();
 }

@@ -309,6 +309,36 @@ VRT_DI F3 cosine_hemisphere(F3 n, uint32_t& rng) {
   return normalize3((tang * (cp * sr) + bitan * (sp * sr)) + n * __fsqrt_rn(fmax_(0.0f, 1.0f - ry)));
 }
 
+// The kernels of a frame are launched with launch_after: their blocks may be
+// resident before the kernel ahead in the stream is complete.  Each begins with
+// frame_begin, before it reads or writes memory: all threads wait until the
+// kernels ahead are complete and their writes visible, then allow the next kernel's
+// blocks onto the SMs.  A kernel so launched is complete only after its own
+// wait, so the order of the whole stream holds.
+VRT_DI void frame_begin() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// Launch a kernel that begins with frame_begin: its launch overlaps the end of
+// the kernel ahead of it in the stream (frames, launch after launch against
+// this: 96x54 128 -> 115 us, 320x180 172 -> 163, 1283x721 with 6 bounces
+// 796 -> 769, 1080p 1375 -> 1349).
+template <class... P, class... A>
+inline cudaError_t launch_after(void (*kern)(P...), dim3 grid, int block, size_t smem, cudaStream_t st, const A&... args) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c = {};
+  c.gridDim = grid;
+  c.blockDim = dim3(block);
+  c.dynamicSmemBytes = smem;
+  c.stream = st;
+  c.attrs = &attr;
+  c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, kern, static_cast<P>(args)...);
+}
+
 // Material unpack (voxel.wgsl:41-51)
 struct Mat { F3 albedo; float emissive; };
 // The stored albedo (rgba8unorm of sqrt(albedo)) of material m: albedo is the

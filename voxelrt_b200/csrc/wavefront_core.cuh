@@ -463,6 +463,7 @@ VRT_DI void emit2_block(const WfDev& b, int next, uint32_t g, uint32_t P, bool s
 // generate: RNG stream, jitter, camera ray (pathtrace.wgsl:249-263)
 template <class J>
 __global__ void __launch_bounds__(256) k_wf_generate(J jobs, uint32_t P, WfDev b) {
+  frame_begin();
   const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= P) return;
   const int j = jobs.job_of(g);
@@ -497,6 +498,7 @@ constexpr int kTraceThreads = 128;
 template <class J, bool kWide, int kPhases, int kMinB, int kRun, bool kVarMaxT>
 __global__ void __launch_bounds__(kTraceThreads, kMinB) k_wf_trace(J jobs, WfDev b, int wave, int implicit_n,
                                                               int refill_min, unsigned long long* stats) {
+  frame_begin();
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   // The bounce rays (the queue's back) first: their walks are the longer ones, and a wave ends with its
@@ -611,6 +613,7 @@ constexpr int kShadeThreads = 128;
 // blocks of 256; plain frames equal).
 template <class J>
 __global__ void __launch_bounds__(kShadeThreads, 1280 / kShadeThreads) k_wf_shade_primary(J jobs, uint32_t P, WfDev b, unsigned long long* stats) {
+  frame_begin();
   const bool any_cache = jobs.any_cache();
   const CacheDev* ccp = nullptr;
   const uint32_t stride = gridDim.x * blockDim.x;
@@ -666,6 +669,7 @@ __global__ void __launch_bounds__(kShadeThreads, 1280 / kShadeThreads) k_wf_shad
 // shade(k), k >= 1: resolve vertex k-1's shadow ray, then the bounce hit.
 template <class J>
 __global__ void __launch_bounds__(kShadeThreads, 1280 / kShadeThreads) k_wf_shade(J jobs, WfDev b, int wave) {
+  frame_begin();
   const bool any_cache = jobs.any_cache();
   const int n = b.ctr[4 * wave + 2];
   const uint32_t* list = active_of(b, wave);
@@ -758,6 +762,7 @@ __global__ void __launch_bounds__(kShadeThreads, 1280 / kShadeThreads) k_wf_shad
 // so the warp runs the shading code far more often than once per bounce.)
 template <class J, bool kWide>
 __global__ void __launch_bounds__(128, 5) k_wf_tail(J jobs, WfDev b, int wave, unsigned long long* stats) {
+  frame_begin();
   const bool any_cache = jobs.any_cache();
   const int n = b.ctr[4 * wave + 2];
   const uint32_t* list = active_of(b, wave);
@@ -1005,7 +1010,7 @@ cudaError_t wf_launch_trace(const J& jobs, int blocks_per_sm, int sms, const WfD
     cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, kTraceThreads, 0);
     if (e != cudaSuccess || per < 1) per = 1;
   }
-  fn<<<sms * per, kTraceThreads, 0, st>>>(jobs, b, w, implicit_n, refill, stats);
+  launch_after(fn, sms * per, kTraceThreads, 0, st, jobs, b, w, implicit_n, refill, stats);
   return cudaGetLastError();
 }
 
@@ -1060,7 +1065,7 @@ cudaError_t wf_run_waves(const J& jobs, uint32_t P, int waves, const WavefrontBu
   const int sblocks = std::min(sms * (tune.shade_blocks_per_sm > 0 ? tune.shade_blocks_per_sm : 32) * (256 / kShadeThreads),
                                (int)((P + kShadeThreads - 1) / kShadeThreads));
   uint32_t nl = 0;
-  k_wf_generate<J><<<(P + 255) / 256, 256, 0, st>>>(jobs, P, b);
+  launch_after(k_wf_generate<J>, (P + 255) / 256, 256, 0, st, jobs, P, b);
   nl++;
   int timed = 0;
   for (int w = 0; w < waves; w++) {
@@ -1069,8 +1074,8 @@ cudaError_t wf_run_waves(const J& jobs, uint32_t P, int waves, const WavefrontBu
       // registers): 0.125 ms of path trace at 58 K pixels and 1.050 of a 1080p cache frame, against 0.133
       // and 1.060 at 6, 0.146 and 1.082 at 8
       const int tblocks = sms * 5;
-      if (jobs.wide()) k_wf_tail<J, true><<<tblocks, 128, 0, st>>>(jobs, b, w, stats);
-      else k_wf_tail<J, false><<<tblocks, 128, 0, st>>>(jobs, b, w, stats);
+      if (jobs.wide()) launch_after(k_wf_tail<J, true>, tblocks, 128, 0, st, jobs, b, w, stats);
+      else launch_after(k_wf_tail<J, false>, tblocks, 128, 0, st, jobs, b, w, stats);
       if ((e = cudaGetLastError()) != cudaSuccess) return e;
       nl++;
       break;
@@ -1138,8 +1143,8 @@ cudaError_t wf_launch_frame(const J& jobs, uint32_t P, int waves, const Wavefron
   }
   return wf_run_waves(jobs, P, waves, wb, tune, stats, st, launches, trace_ev, max_timed_waves, timed_waves,
                       [&](const WfDev& b, int w, int sblocks) {
-                        if (w == 0) k_wf_shade_primary<J><<<sblocks, kShadeThreads, 0, st>>>(jobs, P, b, stats);
-                        else k_wf_shade<J><<<sblocks, kShadeThreads, 0, st>>>(jobs, b, w);
+                        if (w == 0) launch_after(k_wf_shade_primary<J>, sblocks, kShadeThreads, 0, st, jobs, P, b, stats);
+                        else launch_after(k_wf_shade<J>, sblocks, kShadeThreads, 0, st, jobs, b, w);
                         return cudaGetLastError();
                       }, tail_from);
 }
