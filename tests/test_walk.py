@@ -58,6 +58,27 @@ def test_walk_matches_nested_loops(vrt, ctx, n):
         o.close()
 
 
+# The primary rays start in 8 x 4 tiles: sizes below, at and past a tile's side, alone and as the views of a batch.
+@pytest.mark.parametrize("W,H", [(1, 1), (7, 3), (8, 4), (9, 5), (33, 2), (3, 33), (131, 67)])
+def test_primary_order_covers_the_image(vrt, ctx, W, H):
+    vox, spawn = vrt.generate_scene(vrt.VRT_SCENE_FULL, 64, 3)
+    sc = vrt.Scene(ctx, vox, 64)
+    mega = vrt.Session(ctx, sc, W, H, keep_radiance_f32=True, path_kernel="megakernel")
+    wave = vrt.Session(ctx, sc, W, H, keep_radiance_f32=True)
+    views = [vrt.Session(ctx, sc, W + k, H, keep_radiance_f32=True, path_kernel="batch_only") for k in (0, 1, 0)]
+    batch = vrt.Batch(ctx, views)
+    u = [vrt.make_uniforms(vrt.camera_spline(spawn, 2), None, vrt.Lighting(), 5, 2, 0, W + k, H) for k in (0, 1, 0)]
+    mega.frame(u[0])
+    wave.frame(u[0])
+    batch.frame(u)
+    want = (mega.radiance_f32().tobytes(), mega.gbuffer().tobytes())
+    for s in (wave, views[0], views[2]):
+        assert (s.radiance_f32().tobytes(), s.gbuffer().tobytes()) == want
+    batch.close()
+    for o in (mega, wave, *views, sc):
+        o.close()
+
+
 def _odd_rays(n, ext, seed):
     """Random rays, and the forms a walk can trip over: zero, tiny, huge, infinite and NaN components,
     origins on voxel and brick edges, far away or not finite, bounds of every size."""

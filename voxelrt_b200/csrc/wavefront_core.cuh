@@ -481,6 +481,20 @@ __global__ void __launch_bounds__(256) k_wf_generate(J jobs, uint32_t P, WfDev b
   b.S0[g] = make_float4(0.0f, 0.0f, 0.0f, __uint_as_float(rng));
 }
 
+// The q-th pixel of a W x H image in tiles of kTileX x kTileY (row by row in
+// the tile and over the tiles; what is left at the right and at the bottom keeps
+// the same order in narrower and lower tiles).  A warp's primary rays so start
+// through a compact part of the image and walk together: the primary wave of the
+// 1080p frame 192 -> 177 us against rows of 32.
+constexpr uint32_t kTileX = 8, kTileY = 4;
+VRT_DI uint32_t tile_order(uint32_t q, uint32_t W, uint32_t H) {
+  const uint32_t y0 = q / (kTileY * W) * kTileY, r = q - y0 * W;   // strip of rows, pixel in it
+  const uint32_t h = min(kTileY, H - y0);
+  const uint32_t x0 = r / (kTileX * h) * kTileX, t = r - x0 * h;   // tile of the strip, pixel in it
+  const uint32_t w = min(kTileX, W - x0);
+  return (y0 + t / w) * W + x0 + t % w;
+}
+
 constexpr int kTraceThreads = 128;
 // Persistent queue tracer.  A pass of the warp bookkeeping (idle-lane ballot,
 // refill, drain check) covers kPhases rounds of up to kRun DDA steps and the
@@ -550,9 +564,13 @@ __global__ void __launch_bounds__(kTraceThreads, kMinB) k_wf_trace(J jobs, WfDev
         if (slot < n) {
           entry = implicit_n > 0 ? (uint32_t)slot
                                  : (slot < nb ? queue[b.qcap - 1u - (uint32_t)slot] : queue[slot - nb]);
-          const uint32_t g = entry & ~kShadowBit;
+          uint32_t g = entry & ~kShadowBit;
           const int j = jobs.job_of_cached(g, jc, jlo, jhi);   // consecutive rays mostly share a job
           S = jobs.scene(j);
+          if (implicit_n > 0) {
+            const uint32_t p0 = jobs.first(j);
+            g = entry = p0 + tile_order(g - p0, (uint32_t)jobs.width(j), (uint32_t)jobs.height(j));
+          }
           // primary rays start at the camera: its position comes from the job's
           // uniforms (k_wf_generate writes no R0, so no wave-0 shading kernel
           // may read R0 either); later waves read the origin their shading stored
