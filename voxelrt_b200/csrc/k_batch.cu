@@ -28,8 +28,8 @@ static_assert(offsetof(JobDev, cache) == offsetof(JobHost, cache), "job table la
 __global__ void __launch_bounds__(256) k_b_temporal(MultiJob J, uint32_t P) {
   frame_begin();
   const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
+  const int j = J.job_of_warp(g);
   if (g >= P) return;
-  const int j = J.job_of(g);
   const JobDev& jd = J.jobs[j];
   const int W = jd.W, H = jd.H;
   const uint32_t lp = g - jd.first;
@@ -42,7 +42,7 @@ __global__ void __launch_bounds__(256) k_b_temporal(MultiJob J, uint32_t P) {
 // atrous.wgsl:26-83 iteration `it` (step 1 << it) of every job whose denoise
 // flag is set; chain accum -> dA -> dB -> dA (main.js:503-507).  A CTA computes
 // one 32 x 32 tile of one job (atrous_tile.cuh).  tiles: m + 1 prefix counts of
-// the jobs' tiles; CTA b finds its job by binary search.
+// the jobs' tiles, in which CTA b finds its job.
 constexpr int kBatchRows = 32;   // tile rows
 template <int S>
 __global__ void __launch_bounds__(8 * kBatchRows, 96 / kBatchRows) k_b_atrous(MultiJob J,
@@ -50,18 +50,18 @@ __global__ void __launch_bounds__(8 * kBatchRows, 96 / kBatchRows) k_b_atrous(Mu
   frame_begin();
   extern __shared__ float4 sm[];
   const uint32_t b = blockIdx.x;
-  int lo = 0, hi = J.n - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (__ldg(tiles + mid) <= b) lo = mid;
-    else hi = mid - 1;
-  }
+  const int lo = last_at_or_before(tiles, J.n, b);
   const JobDev& jd = J.jobs[lo];
   if ((jd.u.params0[2] & 2u) == 0u) return;
   const int tb = (int)(b - __ldg(tiles + lo)), tw = (jd.W + kAtrousTile - 1) / kAtrousTile;
   const void* src = S == 1 ? jd.acc_cur : (S == 2 ? (const void*)jd.den0 : (const void*)jd.den1);
-  const AtrousImage I{jd.W, jd.H, src, S == 1 && jd.acc_f32 != 0, jd.out.gbuf, S == 2 ? jd.den1 : jd.den0};
-  atrous_tile<S, kBatchRows>(sm, I, (tb % tw) * kAtrousTile, (tb / tw) * kBatchRows);
+  uint2* dst = S == 2 ? jd.den1 : jd.den0;
+  const int x0 = (tb % tw) * kAtrousTile, y0 = (tb / tw) * kBatchRows;
+  // one copy of the filter for each type of history, as for a single view
+  if (S == 1 && jd.acc_f32 != 0)
+    atrous_tile<S, kBatchRows>(sm, AtrousImage{jd.W, jd.H, src, true, jd.out.gbuf, dst}, x0, y0);
+  else
+    atrous_tile<S, kBatchRows>(sm, AtrousImage{jd.W, jd.H, src, false, jd.out.gbuf, dst}, x0, y0);
 }
 
 template <int S>
@@ -78,8 +78,8 @@ static cudaError_t launch_b_atrous(const MultiJob& J, const AtrousTiles& at, cud
 __global__ void __launch_bounds__(256) k_b_present(MultiJob J, uint32_t P, const float* __restrict__ lut) {
   frame_begin();
   const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
+  const int j = J.job_of_warp(g);
   if (g >= P) return;
-  const int j = J.job_of(g);
   const JobDev& jd = J.jobs[j];
   const uint32_t lp = g - jd.first;
   const bool denoise = (jd.u.params0[2] & 2u) != 0u;

@@ -85,6 +85,7 @@ struct SingleJob {
   __host__ __device__ bool any_cache() const { return cc.on != 0; }
   VRT_DI const CacheDev& cache(int) const { return cc; }
   VRT_DI int job_of(uint32_t) const { return 0; }
+  VRT_DI int job_of_warp(uint32_t) const { return 0; }
   VRT_DI int job_of_cached(uint32_t, int&, uint32_t&, uint32_t&) const { return 0; }
   VRT_DI const Uni& uni(int) const { return u; }
   VRT_DI DScene scene(int) const { return S; }
@@ -116,8 +117,21 @@ struct JobDev {
   CacheDev cache;          // radiance cache of the job's session (cache.on == 0: plain path)
 };
 
-// Many sessions: job table in device memory, job found by binary search on
-// the sorted first-pixel array.
+// The last of n ascending values (the first is 0) that is not above v, which all lanes of the warp hold; all
+// lanes call it.
+VRT_DI int last_at_or_before(const uint32_t* __restrict__ a, int n, uint32_t v) {
+  const int lane = threadIdx.x & 31;
+  int c = 0;
+  for (int base = 0; base < n; base += 32) {
+    const unsigned m = __ballot_sync(0xffffffffu, base + lane < n && __ldg(a + base + lane) <= v);
+    c += __popc(m);
+    if (m != 0xffffffffu) break;
+  }
+  return c - 1;
+}
+
+// Many sessions: job table in device memory, job found by search on the sorted
+// first-pixel array.
 struct MultiJob {
   const JobDev* jobs;
   const uint32_t* firsts;  // n entries, ascending
@@ -135,6 +149,13 @@ struct MultiJob {
       else hi = mid - 1;
     }
     return lo;
+  }
+  // job_of for a whole warp whose lanes hold consecutive pixels (all lanes call it; a pixel past the last
+  // one gives some job): one load per 32 jobs instead of a dependent load per halving
+  VRT_DI int job_of_warp(uint32_t g) const {
+    const uint32_t g0 = __shfl_sync(0xffffffffu, g, 0);
+    const int lo = last_at_or_before(firsts, n, g0);
+    return __any_sync(0xffffffffu, lo + 1 < n && __ldg(firsts + lo + 1) <= g) ? job_of(g) : lo;
   }
   // job_of with the caller's last answer (job jc for pixels [lo, hi), lo <= hi; lo == hi: none)
   // tried first
@@ -465,8 +486,8 @@ template <class J>
 __global__ void __launch_bounds__(256) k_wf_generate(J jobs, uint32_t P, WfDev b) {
   frame_begin();
   const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
+  const int j = jobs.job_of_warp(g);
   if (g >= P) return;
-  const int j = jobs.job_of(g);
   const Uni& u = jobs.uni(j);
   const int W = jobs.width(j), H = jobs.height(j);
   const uint32_t lp = g - jobs.first(j);
@@ -642,8 +663,8 @@ __global__ void __launch_bounds__(kShadeThreads, 1280 / kShadeThreads) k_wf_shad
     bool fin_train = false;
     uint32_t ti = 0u;
     F3 rfin = f3(0.0f, 0.0f, 0.0f);
+    const int j = jobs.job_of_warp(g);
     if (g < P) {
-      const int j = jobs.job_of(g);
       const Uni& u = jobs.uni(j);
       const JobOut out = jobs.outs(j);
       const uint32_t lp = g - jobs.first(j);
