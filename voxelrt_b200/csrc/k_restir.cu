@@ -1143,7 +1143,8 @@ __global__ void __launch_bounds__(256) k_wf_restir_primary(const __grid_constant
     bool shadow = false, bounce = false, keep = false;
     if (g < P) {
       const uint4 h = b.hit[g];
-      const F3 rd = xyz(b.R1[g]);
+      const float4 r1 = b.R1[g];
+      const F3 rd = xyz(r1);
       const float t = __uint_as_float(h.x);
       if (t < 0.0f) {
         const F3 sky = sky_color(u, rd, true);
@@ -1161,7 +1162,7 @@ __global__ void __launch_bounds__(256) k_wf_restir_primary(const __grid_constant
         const F3 n1 = hit_normal((int)h.z, rd);
         job.out.alb8[g] = sqrt_albedo8(h.y);
         job.out.gbuf[g] = make_float4(n1.x, n1.y, n1.z, t);
-        uint32_t rng = __float_as_uint(b.S0[g].w);
+        uint32_t rng = __float_as_uint(r1.w);
         const F3 surf1 = x1 + n1 * fmax_(1e-3f, t * 1e-4f);
         const F3 l = sample_sun_dir(u, rng);
         const float ndl = dot3(n1, l);
@@ -1500,7 +1501,8 @@ __global__ void __launch_bounds__(128, 10) k_wf_unified_primary(const __grid_con
     URays rays;
     if (g < P) {
       const uint4 h = b.hit[g];
-      const F3 rd = xyz(b.R1[g]);
+      const float4 r1 = b.R1[g];
+      const F3 rd = xyz(r1);
       const float t = __uint_as_float(h.x);
       if (t < 0.0f) {
         const F3 sky = sky_color(u, rd, true);
@@ -1520,7 +1522,7 @@ __global__ void __launch_bounds__(128, 10) k_wf_unified_primary(const __grid_con
         R.gbuf[g] = make_float4(n1.x, n1.y, n1.z, t);
         const float em = mat1.emissive * kEmissiveScale;   // unified: the sun goes through the reservoir
         R.direct[g] = pack_h4(em, em, em, 1.0f);
-        uint32_t rng = __float_as_uint(b.S0[g].w);
+        uint32_t rng = __float_as_uint(r1.w);
         const F3 surf1 = x1 + n1 * fmax_(1e-3f, t * 1e-4f);
         Ris ris;
         ris.sel = null_sample(0.0f);

@@ -19,9 +19,9 @@ constexpr uint32_t kFlagShadow2 = 4u;           // a second shadow ray of the pr
 
 struct WfDev {
   float4* R0;      // ray origin of waves 1..: surf = pos + n*1e-3 (primary rays start at the camera)
-  float4* R1;      // primary / bounce direction
+  float4* R1;      // primary / bounce direction; w = RNG state bits in wave 0
   float4* R2;      // direction (xyz) and maxT (w) of the pending shadow ray
-  float4* S0;      // radiance xyz, w = RNG state bits
+  float4* S0;      // radiance xyz, w = RNG state bits (waves 1..)
   float4* S1;      // throughput xyz, w = primary material bits
   float4* S2;      // pending sun contribution xyz, w = flags
   uint4* hit;      // x = t bits, y = material, z = entry axis, w = shadow occluded
@@ -498,8 +498,8 @@ __global__ void __launch_bounds__(256) k_wf_generate(J jobs, uint32_t P, WfDev b
   const float uvx = (((float)gx + 0.5f) + jx) / (float)W;
   const float uvy = (((float)gy + 0.5f) + jy) / (float)H;
   const F3 rd = camera_ray(u, uvx, uvy);
-  b.R1[g] = make_float4(rd.x, rd.y, rd.z, 0.0f);
-  b.S0[g] = make_float4(0.0f, 0.0f, 0.0f, __uint_as_float(rng));
+  // the path state of wave 0 is this one word: no radiance yet, and the RNG state in the direction's free lane
+  b.R1[g] = make_float4(rd.x, rd.y, rd.z, __uint_as_float(rng));
 }
 
 // The q-th pixel of a W x H image in tiles of kTileX x kTileY (row by row in
@@ -669,8 +669,8 @@ __global__ void __launch_bounds__(kShadeThreads, 1280 / kShadeThreads) k_wf_shad
       const JobOut out = jobs.outs(j);
       const uint32_t lp = g - jobs.first(j);
       const uint4 h = b.hit[g];
-      const F3 rd = xyz(b.R1[g]);
-      const float s0w = b.S0[g].w;   // RNG state, loaded with the hit rather than after the sky test
+      const float4 r1 = b.R1[g];
+      const F3 rd = xyz(r1);
       const float t = __uint_as_float(h.x);
       if (t < 0.0f) {
         const F3 sky = sky_color(u, rd, true);
@@ -685,7 +685,7 @@ __global__ void __launch_bounds__(kShadeThreads, 1280 / kShadeThreads) k_wf_shad
         const F3 n1 = hit_normal((int)h.z, rd);
         out.alb8[lp] = sqrt_albedo8(h.y);
         out.gbuf[lp] = make_float4(n1.x, n1.y, n1.z, t);
-        uint32_t rng = __float_as_uint(s0w);
+        uint32_t rng = __float_as_uint(r1.w);
         F3 radiance = f3(0.0f, 0.0f, 0.0f), tp = f3(1.0f, 1.0f, 1.0f);
         const int W = jobs.width(j);
         const CacheDev& cc = jobs.cache(j);
