@@ -13,12 +13,12 @@
 //   trace(k)  : queue k;  shade(k): resolve vertex k-1's shadow ray, shade
 //               vertex k, append queue k+1 ... until every path terminated.
 //
-// Queues and active-path lists are compacted with warp ballots (one atomic
-// per warp).  The trace kernel is persistent: each warp owns 32 lanes that
-// walk the DDA as a flat state machine shared by brick-level and voxel-level
-// lanes; lanes whose ray ended are refilled from the queue once enough of
-// them are idle, so warps stay full until the queue drains.  The kernels are
-// defined in wavefront_core.cuh and shared with the batched form (k_batch.cu).
+// Queues and active-path lists are compacted with one atomic per block.  The
+// trace kernel is persistent: each warp owns 32 lanes that step through bricks
+// or voxels in one loop (dda_walk.cuh) and change between the levels together;
+// lanes whose ray ended are refilled from the queue once enough of them are
+// idle, so warps stay full until the queue drains.  The kernels are defined in
+// wavefront_core.cuh and shared with the batched form (k_batch.cu).
 //
 // The per-path arithmetic (RNG draws, shading, order of radiance sums) is
 // exactly the megakernel's, so results are bit-identical to it and to the

@@ -1,7 +1,7 @@
-// wavefront.cuh -- building blocks of the wavefront path tracer shared by the
-// single-session kernels (k_wavefront.cu) and the batched kernels
-// (k_batch.cu): path-state layout, block-aggregated queue appends, the flat
-// two-level DDA, and per-vertex shading.
+// wavefront_core.cuh -- building blocks of the wavefront path tracer shared by
+// the single-session kernels (k_wavefront.cu) and the batched kernels
+// (k_batch.cu): path-state layout, block-aggregated queue appends, the queue
+// tracer, and per-vertex shading.
 #pragma once
 #include "dda_walk.cuh"
 #include "vrt_device.cuh"
@@ -73,8 +73,7 @@ struct JobOut {
   float4* gbuf;     // rgba32f normal + distance of this frame
 };
 
-// One session: everything in kernel parameters, occupancy bitmap staged in
-// shared memory by the tracer.
+// One session: everything in kernel parameters.
 struct SingleJob {
   Uni u;
   DScene S;
