@@ -457,6 +457,7 @@ __device__ __forceinline__ bool group_publish_and(int g, bool ok) {
 // issuing thread waiting -- ran 70.7 against 65.8 us for 983 K queries: the
 // issuer's polling and the warps it holds back cost more than the barrier.)
 __global__ void __launch_bounds__(256, 2) k_mlp_infer(const __grid_constant__ MlpTaskSet ts) {
+  frame_begin();
   using namespace mlp;
   const MlpTask& tk = ts.t[task_of(ts, blockIdx.x)];
   int n = tk.n_max;
@@ -578,6 +579,7 @@ __global__ void __launch_bounds__(256, 2) k_mlp_infer(const __grid_constant__ Ml
 // of building 192 mask bits per sample cut the instructions 5.3 -> 3.8 M and
 // the time 28.7 -> 25.7 us for 65,536 samples (983 K: a call 312 -> 271 us).
 __global__ void __launch_bounds__(256, 1) k_mlp_grad(const __grid_constant__ MlpTaskSet ts) {
+  frame_begin();
   using namespace mlp;
   const MlpTask& tk = ts.t[task_of(ts, blockIdx.x)];
   const int cb = blockIdx.x - tk.cta0;
@@ -731,6 +733,7 @@ __global__ void __launch_bounds__(256, 1) k_mlp_grad(const __grid_constant__ Mlp
 constexpr int kReduceRows = 16, kReduceCols = 32, kReduceRuns = 16;   // up to 256 partial rows per pass
 
 __global__ void __launch_bounds__(kReduceCols * kReduceRuns) k_mlp_reduce(const __grid_constant__ MlpTaskSet ts) {
+  frame_begin();
   __shared__ float s_run[kReduceRuns][kReduceCols];
   const MlpTask& tk = ts.t[blockIdx.y];
   const int i = blockIdx.x * kReduceCols + threadIdx.x;   // kParams is a multiple of kReduceCols
@@ -758,6 +761,7 @@ static_assert(mlp::kParams % kReduceCols == 0, "a reduction block covers whole p
 // the bf16 copy.  Output columns >= 3 stay 0.  Skipped when the step had no
 // samples.  blockIdx.y = task.
 __global__ void k_mlp_adam(const __grid_constant__ MlpTaskSet ts, float b1, float b2, float eps) {
+  frame_begin();
   const MlpTask& tk = ts.t[blockIdx.y];
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= mlp::kParams) return;
@@ -839,7 +843,7 @@ cudaError_t mlp_infer_tasks(MlpTaskSet& ts, cudaStream_t st) {
     attr = true;
   }
   const int grid = assign_ctas(ts, sm_count_mlp() * 2, 512);   // 2 x 108 KB of shared memory per SM
-  k_mlp_infer<<<grid, 256, mlp::kInferSmem, st>>>(ts);
+  launch_after(k_mlp_infer, grid, 256, mlp::kInferSmem, st, ts);
   return cudaGetLastError();
 }
 
@@ -853,16 +857,16 @@ cudaError_t mlp_gradient_tasks(MlpTaskSet& ts, cudaStream_t st) {
   }
   // partial buffers hold mlp_max_ctas() rows per network
   const int grid = assign_ctas(ts, sm_count_mlp(), 256);
-  k_mlp_grad<<<grid, 256, mlp::kTrainSmem, st>>>(ts);
+  launch_after(k_mlp_grad, grid, 256, mlp::kTrainSmem, st, ts);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  k_mlp_reduce<<<dim3(mlp::kParams / kReduceCols, ts.n), dim3(kReduceCols, kReduceRuns), 0, st>>>(ts);
+  launch_after(k_mlp_reduce, dim3(mlp::kParams / kReduceCols, ts.n), dim3(kReduceCols, kReduceRuns), 0, st, ts);
   return cudaGetLastError();
 }
 
 cudaError_t mlp_adam_tasks(const MlpTaskSet& ts, cudaStream_t st) {
   if (ts.n <= 0) return cudaSuccess;
-  k_mlp_adam<<<dim3((mlp::kParams + 255) / 256, ts.n), 256, 0, st>>>(ts, 0.9f, 0.99f, 1e-8f);
+  launch_after(k_mlp_adam, dim3((mlp::kParams + 255) / 256, ts.n), 256, 0, st, ts, 0.9f, 0.99f, 1e-8f);
   return cudaGetLastError();
 }
 

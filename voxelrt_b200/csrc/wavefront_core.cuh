@@ -888,6 +888,7 @@ __global__ void __launch_bounds__(128, 5) k_wf_tail(J jobs, WfDev b, int wave, u
 // Zeroes the per-frame query and sample counters of every cache job.
 template <class J>
 __global__ void k_cache_reset(J jobs, int njobs) {
+  frame_begin();
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= njobs) return;
   const CacheDev& c = jobs.cache(j);
@@ -917,6 +918,7 @@ struct ResolveSet {
 template <class J>
 __global__ void __launch_bounds__(256) k_cache_resolve(J jobs, WfDev b, const __grid_constant__ ResolveSet rs,
                                                        unsigned long long* stats) {
+  frame_begin();
   const ResolveEntry& r = rs.e[blockIdx.y];
   const int n = *r.qcount;
   if (stats && blockIdx.x == 0 && threadIdx.x == 0) {
@@ -1022,7 +1024,7 @@ cudaError_t launch_cache_post(const J& jobs, const WfDev& b, const CacheLaunch* 
     cudaError_t e = mlp_infer_tasks(ts, st);
     if (e != cudaSuccess) return e;
     const int bx = std::max(1, std::min((maxP + 255) / 256, wf_sm_count() * 8 / cn));
-    k_cache_resolve<J><<<dim3(bx, rs.n), 256, 0, st>>>(jobs, b, rs, stats);
+    launch_after(k_cache_resolve<J>, dim3(bx, rs.n), 256, 0, st, jobs, b, rs, stats);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     nl += 2;
     for (int k = 0; k < steps; k++) {
@@ -1176,7 +1178,7 @@ cudaError_t wf_launch_frame(const J& jobs, uint32_t P, int waves, const Wavefron
                             int njobs = 1, int tail_from = 0) {
   if (waves + 1 > wb.max_waves) return cudaErrorInvalidValue;
   if (jobs.any_cache()) {
-    k_cache_reset<J><<<(njobs + 127) / 128, 128, 0, st>>>(jobs, njobs);
+    launch_after(k_cache_reset<J>, (njobs + 127) / 128, 128, 0, st, jobs, njobs);
     if (launches) (*launches)++;
   }
   return wf_run_waves(jobs, P, waves, wb, tune, stats, st, launches, trace_ev, max_timed_waves, timed_waves,
