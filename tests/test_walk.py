@@ -130,8 +130,9 @@ def test_ray_batch_matches_oracle(vrt, orc, ctx, grid, n):
 
 
 # pixel counts on both sides of the lines at which the remaining paths of a
-# frame move to one thread each, by default and at every wave
-@pytest.mark.parametrize("W,H,bounces", [(401, 297, 2), (401, 303, 3), (611, 331, 2), (611, 331, 3), (811, 501, 4),
+# frame move to one thread each, by default and at every wave, and below the
+# line at which a path has two lanes there
+@pytest.mark.parametrize("W,H,bounces", [(1, 1, 2), (64, 41, 3), (223, 213, 4), (401, 297, 2), (401, 303, 3), (611, 331, 2), (611, 331, 3), (811, 501, 4),
                                          (1201, 801, 5)])
 def test_tail_waves_leave_the_image(vrt, ctx, W, H, bounces):
     vox, spawn = vrt.generate_scene(vrt.VRT_SCENE_VOXELRT, 128, 7)

@@ -783,9 +783,10 @@ __global__ void __launch_bounds__(kShadeThreads, 1280 / kShadeThreads) k_wf_shad
   }
 }
 
-// The tail of a frame whose remaining paths are few -- the radiance cache's
-// training paths after every other path ended at its first bounce: one
-// thread finishes each path of wave `wave`'s active list, tracing its pending
+// The tail of a frame whose remaining paths are few (small frames, late waves,
+// the radiance cache's training paths after every other path ended at its
+// first bounce): each path of wave `wave`'s active list is finished here by one
+// thread, or by two where all of them fit the grid so, tracing its pending
 // shadow and bounce rays with the same resumable DDA the queue tracer runs
 // (dda_walk.cuh: same walk, hits and counters) and shading each vertex as
 // k_wf_shade does, until the path ends.  The per-wave form would launch a
@@ -794,10 +795,19 @@ __global__ void __launch_bounds__(kShadeThreads, 1280 / kShadeThreads) k_wf_shad
 // sequence.  Same per-path arithmetic and RNG draws, so the same image.
 // Few paths are spread over all warps, a few lanes each: lanes on different
 // walks take turns.
+// Bound by the latency of a path's walks, one after another.  Its shadow and
+// bounce ray of a vertex are independent: with two lanes per path they walk
+// together, and the odd lane leaves the path's state to the even one.  That pays
+// while all paths fit the grid at once (kTailPairLimit per warp, 47 K); with more,
+// a lane per path finishes sooner.  Path trace in ms, one lane / two where they fit
+// / two always: 320x180 .122 / .111 / .117; 320x180 with 6 bounces .204 / .171 /
+// .171; 400x225 .184 / .180 / .195; 1283x721 with 6 bounces .687 / .665 / .663;
+// a 1080p cache frame (130 K paths) .980 / .975 / .997.
 // (A per-lane state machine -- lanes stepping their walks together, each
 // shading when its own ray ends and then taking the next path -- ran 447
 // against 305 us per 1080p cache frame: some lane shades in nearly every pass,
 // so the warp runs the shading code far more often than once per bounce.)
+constexpr int kTailPairLimit = 16;
 template <class J, bool kWide>
 __global__ void __launch_bounds__(128, 5) k_wf_tail(J jobs, WfDev b, int wave, unsigned long long* stats) {
   frame_begin();
@@ -805,61 +815,65 @@ __global__ void __launch_bounds__(128, 5) k_wf_tail(J jobs, WfDev b, int wave, u
   const int n = b.ctr[4 * wave + 2];
   const uint32_t* list = active_of(b, wave);
   // few paths are spread over all warps (as in k_wf_trace); every block runs every round
+  const unsigned full = 0xffffffffu;
   const int nwarps = (int)(gridDim.x * (blockDim.x >> 5)), warp = (int)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5));
-  const int lanes = min(32, max(1, (n + nwarps - 1) / nwarps)), lane = threadIdx.x & 31;
+  const bool pair = n <= kTailPairLimit * nwarps;
+  const int lane = threadIdx.x & 31, slot = pair ? lane >> 1 : lane;
+  const int per = min(pair ? 16 : 32, max(1, (n + nwarps - 1) / nwarps));
+  const bool owner = !pair || (lane & 1) == 0;    // of the path's state; the other lane of a pair walks its shadow rays
+  const int ray0 = pair && owner ? 1 : 0, ray1 = pair && !owner ? 1 : 2;   // this lane's rays: 0 shadow, 1 bounce
   DCount c{0u, 0u, 0u, 0u};
-  for (int base = 0; base < n; base += nwarps * lanes) {
-    const int i = lane < lanes ? base + warp * lanes + lane : n;
+  for (int base = 0; base < n; base += nwarps * per) {
+    const int i = slot < per ? base + warp * per + slot : n;
     bool fin_train = false;
-    uint32_t ti = 0u;
+    uint32_t ti = 0u, g = 0u, lp = 0u;
     F3 rfin = f3(0.0f, 0.0f, 0.0f);
-    int jc = 0;
-    if (i < n) {
-      const uint32_t g = list[i];
-      const int j = jobs.job_of(g);
-      jc = j;
-      const uint32_t lp = g - jobs.first(j);
-      const int W = jobs.width(j);
-      const CacheDev& cc = jobs.cache(j);
-      const int role = cache_role(cc, lp, W);
-      const Uni& u = jobs.uni(j);
-      const DScene S = jobs.scene(j);
-      for (int w = wave;; w++) {
-        const float4 s0 = b.S0[g];
-        const float4 s1 = b.S1[g];
-        const float4 s2 = b.S2[g];
-        const float4 r0 = b.R0[g];
-        const float4 r1 = b.R1[g];
-        F3 radiance = xyz(s0);
-        F3 tp = xyz(s1);
-        uint32_t rng = __float_as_uint(s0.w);
-        const uint32_t mat1bits = __float_as_uint(s1.w);
-        const uint32_t flags = __float_as_uint(s2.w);
-        const F3 surf = xyz(r0);
-        if (flags & kFlagShadow) {   // the previous vertex's sun shadow ray
-          const float4 r2 = b.R2[g];
-          const F3 ld = xyz(r2);
-          Walk<kWide> d;
-          d.init(S, surf, ld, r2.w);
-          c.rays++;
-          while (!d.done()) {
-            d.template walk_run<5>(S);
-            if (!d.walking()) d.transition(S, ld, c);
-          }
-          d.finish(S, c);
-          if (!(d.tHit >= 0.0f)) radiance = radiance + xyz(s2);
-        }
-        bool done = (flags & kFlagTerminal) != 0u;
-        if (!done) {
-          const F3 rd = xyz(r1);
-          Walk<kWide> d;
-          d.init(S, surf, rd, 1e4f);
+    int j = 0, role = kRolePlain;
+    bool live = i < n;
+    if (live) {
+      g = list[i];
+      j = jobs.job_of(g);
+      lp = g - jobs.first(j);
+      role = cache_role(jobs.cache(j), lp, jobs.width(j));
+    }
+    const DScene S = jobs.scene(j);
+    for (int w = wave; __any_sync(full, live); w++) {
+      uint32_t flags = 0u;
+      F3 surf = f3(0.0f, 0.0f, 0.0f), rd = surf;
+      bool lit = false;                            // the shadow ray met nothing
+      Walk<kWide> d;
+      if (live) {
+        flags = __float_as_uint(b.S2[g].w);
+        surf = xyz(b.R0[g]);
+#pragma unroll 1
+        for (int ray = ray0; ray < ray1; ray++) {
+          if (!(ray == 0 ? (flags & kFlagShadow) != 0u : (flags & kFlagTerminal) == 0u)) continue;
+          const float4 r = ray == 0 ? b.R2[g] : b.R1[g];
+          rd = xyz(r);
+          d.init(S, surf, rd, ray == 0 ? r.w : 1e4f);
           c.rays++;
           while (!d.done()) {
             d.template walk_run<5>(S);
             if (!d.walking()) d.transition(S, rd, c);
           }
           d.finish(S, c);
+          if (ray == 0) lit = !(d.tHit >= 0.0f);
+        }
+      }
+      if (pair) lit = __shfl_xor_sync(full, (int)lit, 1) != 0;   // the owner's answer from its pair
+      if (live && owner) {
+        const float4 s0 = b.S0[g];
+        const float4 s1 = b.S1[g];
+        F3 radiance = xyz(s0);
+        F3 tp = xyz(s1);
+        uint32_t rng = __float_as_uint(s0.w);
+        const uint32_t mat1bits = __float_as_uint(s1.w);
+        const int W = jobs.width(j);
+        const CacheDev& cc = jobs.cache(j);
+        const Uni& u = jobs.uni(j);
+        if (lit) radiance = radiance + xyz(b.S2[g]);   // the previous vertex's sun
+        bool done = (flags & kFlagTerminal) != 0u;
+        if (!done) {
           if (d.tHit < 0.0f) {
             radiance = radiance + tp * sky_color(u, rd, false);
             done = true;
@@ -876,11 +890,14 @@ __global__ void __launch_bounds__(128, 5) k_wf_tail(J jobs, WfDev b, int wave, u
         if (done) {
           finalize(jobs.outs(j), lp, radiance, mat1bits, jobs.clamp(j));
           if (role == kRoleTrain) { fin_train = true; ti = train_index(cc, lp, W); rfin = radiance; }
-          break;
+          live = false;
         }
       }
+      // the pair takes the owner's path state, written above
+      if (pair) live = __shfl_sync(full, (int)live, lane & 30) != 0;
+      __syncwarp();
     }
-    if (any_cache) cache_emit_samples(jobs.cache(jc), fin_train, ti, rfin);
+    if (any_cache) cache_emit_samples(jobs.cache(j), fin_train, ti, rfin);
   }
   if (stats) block_flush_stats(stats, c, 0u);   // kStatRays..kStatVReads
 }
@@ -1147,12 +1164,12 @@ cudaError_t wf_run_waves(const J& jobs, uint32_t P, int waves, const WavefrontBu
 // waves it replaces, at a lower rate per ray; so the line lies at a number of
 // paths, later the more pixels there are.  Path-trace pass in ms by tail wave
 // (pixels, bounces: none / 1 / 2 / 3 / 4 / 5):
-//   58 K, 2: .183 / .125 / .149 / .167      58 K, 6: .400 / .208 / .246 / .282 / .301
-//  130 K, 2: .299 / .285 / .260 / .283     130 K, 6: .454 / .250 / .292 / .327 / .354
-//  230 K, 2: .333 / .341 / .347 / .316     230 K, 4: .372 / .328 / .287 / .316 / .330
-//  518 K, 2: .472 / .623 / .534 / .469     518 K, 6: .702 / .784 / .698 / .640 / .602 / .633
-//  925 K, 6: .830 / 1.10 / .908 / .765 / .734 / .762
-//  2.1 M, 2: 1.212 / 2.00 / 1.62 / 1.252   2.1 M, 6: 1.539 / 2.65 / 2.24 / 1.78 / 1.517 / 1.471
+//   58 K, 2: .180 / .111 / .133 / .160      58 K, 6: .388 / .171 / .214 / .258 / .289
+//  130 K, 2: .286 / .284 / .249 / .264     130 K, 6: .429 / .243 / .280 / .295 / .322
+//  230 K, 2: .324 / .335 / .326 / .301     230 K, 4: .348 / .317 / .271 / .274 / .306
+//  518 K, 2: .442 / .592 / .497 / .436     518 K, 6: .652 / .745 / .666 / .594 / .535 / .569
+//  925 K, 6: .788 / 1.06 / .862 / .718 / .665 / .707
+//  2.1 M, 2: 1.148 / 1.96 / 1.56 / 1.175   2.1 M, 6: 1.453 / 2.57 / 2.16 / 1.69 / 1.424 / 1.380
 // (The tail's grid holds 95 K paths at once; a few more cost it a second round.)
 // Cache-assisted frames (every path but the training paths ends at wave 1)
 // always take wave 2, and no job with the cache can take wave 1.
