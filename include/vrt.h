@@ -113,10 +113,10 @@ typedef struct VrtTuning {
                                  1: (4,4,9), 2: (3,4,8), 3: (4,3,9), 4: (2,4,9),
                                  5: (8,1,9), 6: (4,3,10), 7: (3,6,9), 8: (3,6,8) */
   int atrous_tile_rows;       /* 0, 8 or 16: accepted and returned; the a-trous
-                                 pass has one tile shape (32 x 32 pixels)      */
+                                 pass picks its tiles by the image's size      */
   int tail_wave;              /* first wave whose remaining paths each finish on
-                                 one thread (their rays traced in turn, not in
-                                 per-wave launches); 0 = never, -1 = automatic
+                                 a thread or two of one launch, not in launches
+                                 per wave; 0 = never, -1 = automatic
                                  (wave 2 for a cache-assisted session, or for a
                                  batch whose every job is cache-assisted; else by
                                  pixels and bounces); the image is the same either

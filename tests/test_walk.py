@@ -113,7 +113,7 @@ def _odd_rays(n, ext, seed):
 
 
 @pytest.mark.parametrize("grid", [8, 104, 256])
-@pytest.mark.parametrize("n", [1, 31, 33, 4097, 600_001, 1_100_003])
+@pytest.mark.parametrize("n", [1, 31, 33, 4097, 13_999, 14_001, 140_001, 600_001, 1_100_003])
 def test_ray_batch_matches_oracle(vrt, orc, ctx, grid, n):
     vox, _ = vrt.generate_scene(vrt.VRT_SCENE_RANDOM, grid, 3)
     b, m = orc.build_bricks(vox, grid)

@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(256) k_pathtrace(DScene S, Uni u, float fclamp
 // the runs out.  Bound by instruction issue, like the queue tracer; against one
 // thread per ray on the nested loops, 2 M incoherent rays at 256^3 took 470 ->
 // 256 us (call with its wait), 1.2 M at 128^3 256 -> 166, 64 rays 27 -> 13, 1000
-// 27 -> 19; 20 K - 100 K rays, where the longest walk decides, 34 - 41 -> 35 - 43.
+// 27 -> 19.
 constexpr int kRayThreads = 128, kRayRefill = 12, kRayMaxRun = 256;
 
 template <bool kWide>
@@ -164,6 +164,30 @@ __global__ void __launch_bounds__(kRayThreads, 9) k_trace_rays(DScene S, const f
   }
 }
 
+// The same batch with one thread per ray on the nested loops.  A ray's walk is
+// latency there as here, but its lane never waits for the warp's transitions.
+__global__ void __launch_bounds__(256) k_trace_rays_nested(DScene S, const float* __restrict__ o,
+                                                           const float* __restrict__ d,
+                                                           const float* __restrict__ tmax, int n,
+                                                           VrtHit* __restrict__ out) {
+  extern __shared__ uint32_t s_occ[];
+  const uint32_t* occ = stage_occupancy<true>(S, s_occ);
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  DCount cnt{0u, 0u, 0u, 0u};
+  const F3 ro = f3(o[3 * (size_t)i], o[3 * (size_t)i + 1], o[3 * (size_t)i + 2]);
+  const F3 rd = f3(d[3 * (size_t)i], d[3 * (size_t)i + 1], d[3 * (size_t)i + 2]);
+  const DHit h = trace<true>(S, occ, ro, rd, tmax[i], cnt);
+  VrtHit r;
+  r.t = h.t; r.n[0] = h.n.x; r.n[1] = h.n.y; r.n[2] = h.n.z; r.mat = h.mat;
+  r.voxel[0] = h.vx; r.voxel[1] = h.vy; r.voxel[2] = h.vz;
+  r.face = h.t >= 0.0f ? face_of(h.n) : -1;
+  r.steps = cnt.outer + cnt.inner;
+  r.bytes = 4u * (cnt.outer + cnt.inner + cnt.vreads);
+  r.pad = 0u;
+  out[i] = r;
+}
+
 cudaError_t launch_pathtrace(const SceneDev& s, const VrtUniforms& u, float fclamp, int W, int H,
                              const PathOut& out, cudaStream_t st) {
   const size_t smem = occ_words(s.BG) * sizeof(uint32_t);
@@ -183,6 +207,20 @@ cudaError_t launch_pathtrace(const SceneDev& s, const VrtUniforms& u, float fcla
 cudaError_t launch_trace_rays(const SceneDev& s, const float* o, const float* d, const float* tmax, int n,
                               VrtHit* out, cudaStream_t st) {
   if (n <= 0) return cudaSuccess;
+  // Between the two, where one thread per ray about fills the GPU and the longest walk decides, the nested
+  // loops are faster: us per call, nested / walk, in worlds of 64^3, 128^3 and 256^3: 12 K rays 33 / 32, 38 / 34,
+  // 44 / 40; 20 K 32 / 34, 37 / 41, 45 / 45; 80 K 37 / 48, 41 / 44, 50 / 52; 120 K 44 / 45, 43 / 43, 59 / 56;
+  // 160 K 52 / 51, 52 / 47, 63 / 59.  Worlds of
+  // 8^3 bricks end a walk so soon that the line lies where the walk's refills begin (400 K rays 81 / 85).
+  const size_t smem = occ_words(s.BG) * sizeof(uint32_t);
+  if (n >= 14000 && n <= (s.BG <= 8 ? 500000 : 140000) && smem <= kMaxSmemOccBytes) {
+    if (smem > 48 * 1024) {
+      cudaError_t e = cudaFuncSetAttribute(k_trace_rays_nested, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (e != cudaSuccess) return e;
+    }
+    k_trace_rays_nested<<<(unsigned)((n + 255) / 256), 256, smem, st>>>(to_dscene(s), o, d, tmax, n, out);
+    return cudaGetLastError();
+  }
   // Rays per warp.  Few rays are spread over all warps the GPU holds (9 blocks
   // on each of 148 SMs), down to one per warp, since lanes on different paths
   // take turns; from 32 per warp on, one per lane until the rays fill the GPU

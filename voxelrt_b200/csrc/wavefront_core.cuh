@@ -1126,7 +1126,7 @@ cudaError_t wf_run_waves(const J& jobs, uint32_t P, int waves, const WavefrontBu
   nl++;
   int timed = 0;
   for (int w = 0; w < waves; w++) {
-    if (tail_from > 0 && w == tail_from) {   // the remaining paths, one thread each
+    if (tail_from > 0 && w == tail_from) {   // the remaining paths, a thread or two each
       // a resident grid of 128-thread blocks (a block's round waits for its slowest path); 5 per SM (96
       // registers): 0.125 ms of path trace at 58 K pixels and 1.050 of a 1080p cache frame, against 0.133
       // and 1.060 at 6, 0.146 and 1.082 at 8
@@ -1158,7 +1158,7 @@ cudaError_t wf_run_waves(const J& jobs, uint32_t P, int waves, const WavefrontBu
   return cudaGetLastError();
 }
 
-// The wave whose remaining paths finish one thread each when the tuning leaves
+// The wave whose remaining paths finish in k_wf_tail when the tuning leaves
 // it open (0: none).  A wave has a floor of 25-35 us of trace and 5-8 of
 // shading -- its longest walk, whatever its size -- which k_wf_tail pays once for all the
 // waves it replaces, at a lower rate per ray; so the line lies at a number of
