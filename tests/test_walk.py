@@ -182,3 +182,25 @@ def test_stored_albedo_is_the_material_byte():
     a = np.arange(256, dtype=np.float32) * s
     q = np.clip(np.sqrt(a * a), np.float32(0.0), np.float32(1.0))
     np.testing.assert_array_equal(np.floor(q * np.float32(255.0) + np.float32(0.5)).astype(np.int64), np.arange(256))
+
+
+# Directions whose components lie below the bound of the reciprocals (1e-8), two or three at a time, from up to a
+# world outside and without a bound on t: the point on the ray then lags far behind the walk's cell.
+@pytest.mark.parametrize("grid", [16, 64])
+def test_short_directions_match_oracle(vrt, orc, ctx, grid):
+    n, ext = 1_500_000, grid / 16.0
+    r = np.random.default_rng(grid)
+    vox, _ = vrt.generate_scene(vrt.VRT_SCENE_RANDOM, grid, 3)
+    b, m = orc.build_bricks(vox, grid)
+    sc = vrt.Scene(ctx, vox, grid)
+    o = (r.random((n, 3)) * 3 * ext - ext).astype(np.float32)
+    d = (np.exp(r.uniform(np.log(1e-10), np.log(1e-8), (n, 3))) * r.choice([-1.0, 1.0], (n, 3))).astype(np.float32)
+    long = np.flatnonzero(r.random(n) < 0.3)
+    d[long, r.integers(0, 3, len(long))] = np.exp(r.uniform(np.log(1e-8), np.log(1e-6), len(long))).astype(np.float32)
+    t = np.full(n, 1e30, np.float32)
+    got, want = sc.trace_rays(o, d, t), orc.trace(vox, b, m, grid, o, d, t)
+    for f in ("t", "n"):
+        assert np.array_equal(got[f].view(np.uint32), want[f].view(np.uint32)), f
+    for f in ("mat", "voxel", "face", "steps", "bytes"):
+        assert np.array_equal(got[f], want[f]), f
+    sc.close()

@@ -47,8 +47,9 @@ VRT_DI F3 hit_normal(int vax, F3 rd) {
             face_normal_component(vax == 2, sz));
 }
 
-// Walk states.  kWalkOdd: a direction component of 0 or NaN, or values so
-// large that a point on the ray may lie far from its cell.
+// Walk states.  kWalkOdd: a direction component below the bound at which
+// safe_inv clamps its reciprocal (0 and NaN among them), or values so large that
+// a point on the ray may lie far from its cell.
 enum : int { kWalkVoxel = 1, kWalkOdd = 2, kWalkOcc = 4, kWalkOut = 8, kWalkDone = 16, kWalkWaits = 4 };
 
 constexpr uint32_t kCntB = 1u << 22, kCntV = 1u << 23;
@@ -104,7 +105,9 @@ struct Walk {
     nb = 0u;
     if (tEnter > tExit) { st = kWalkDone; return; }
     const float ax = fabsf(rd.x), ay = fabsf(rd.y), az = fabsf(rd.z);
-    const bool plain = ax > 0.0f && ay > 0.0f && az > 0.0f && ax < 8.0f && ay < 8.0f && az < 8.0f &&
+    // A clamped reciprocal lets the point on the ray lag whole worlds behind the walk's cell, where descend()'s
+    // comparison of linear indices could take it for another one.
+    const bool plain = ax >= 1e-8f && ay >= 1e-8f && az >= 1e-8f && ax < 8.0f && ay < 8.0f && az < 8.0f &&
                        fabsf(ro.x) < 1048576.0f && fabsf(ro.y) < 1048576.0f && fabsf(ro.z) < 1048576.0f;
     st = plain ? 0 : kWalkOdd;
     t = tEnter;
