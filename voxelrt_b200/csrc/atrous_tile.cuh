@@ -164,7 +164,7 @@ VRT_DI int stage_tile(float4* sm, const AtrousImage& I, int x0, int y0, int rows
       c[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
       if ((unsigned)qy < (unsigned)I.H && (unsigned)(qx + k) < (unsigned)I.W) {
         const size_t q = (size_t)qy * I.W + (qx + k);
-        g[k] = __ldg(I.gbuf + q);
+        g[k] = I.gbuf[q];
         c[k] = load_px(I.src, I.src_f32, q);
       }
     }

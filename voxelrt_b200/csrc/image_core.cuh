@@ -6,21 +6,22 @@
 
 namespace vrt {
 
+// The images are read with ordinary loads: the kernel ahead may still write them when the reader's blocks are
+// resident (frame_begin).
 VRT_DI float4 load_px(const void* base, bool f32, size_t p) {
-  if (f32) return __ldg(reinterpret_cast<const float4*>(base) + p);
-  return unpack_h4(__ldg(reinterpret_cast<const uint2*>(base) + p));
+  if (f32) return reinterpret_cast<const float4*>(base)[p];
+  return unpack_h4(reinterpret_cast<const uint2*>(base)[p]);
 }
 
 // temporal.wgsl:17-77 for pixel (gx, gy): reproject through prevViewProj,
 // validate depth (8% + 2 cm) and normal (dot > 0.85), blend with the
 // bilinearly fetched history (WebGPU linear filter: texel centres at +0.5,
 // clamp to edge).  Returns (colour, history length).
-VRT_DI float4 temporal_pixel(const Uni& u, int W, int H, int gx, int gy, const uint2* __restrict__ rad,
-                             const float4* __restrict__ gcur, const void* __restrict__ accPrev, bool accF32,
-                             const float4* __restrict__ gprev) {
+VRT_DI float4 temporal_pixel(const Uni& u, int W, int H, int gx, int gy, const uint2* rad, const float4* gcur,
+                             const void* accPrev, bool accF32, const float4* gprev) {
   const size_t p = (size_t)gy * W + gx;
-  const float4 c4 = unpack_h4(__ldg(rad + p));
-  const float4 g = __ldg(gcur + p);
+  const float4 c4 = unpack_h4(rad[p]);
+  const float4 g = gcur[p];
   const bool temporalOn = (u.params0[2] & 1u) != 0u;
   if (g.w < 0.0f || !temporalOn) return make_float4(c4.x, c4.y, c4.z, 1.0f);
   const float uvx = ((float)gx + 0.5f) / (float)W;
@@ -36,7 +37,7 @@ VRT_DI float4 temporal_pixel(const Uni& u, int W, int H, int gx, int gy, const u
     const float puy = (-ndy) * 0.5f + 0.5f;
     if (pux > 0.0f && puy > 0.0f && pux < 1.0f && puy < 1.0f) {
       const int ppx = min((int)(pux * (float)W), W - 1), ppy = min((int)(puy * (float)H), H - 1);
-      const float4 pg = __ldg(gprev + ((size_t)ppy * W + ppx));
+      const float4 pg = gprev[(size_t)ppy * W + ppx];
       const F3 dv = wp - f3(u.prevCamPos[0], u.prevCamPos[1], u.prevCamPos[2]);
       const float expectedT = __fsqrt_rn(dot3(dv, dv));
       const bool depthOk = pg.w > 0.0f && fabsf(pg.w - expectedT) < 0.08f * expectedT + 0.02f;
@@ -83,11 +84,11 @@ VRT_DI float b3_weight(int d) { return d == 0 ? 0.375f : ((d == 1 || d == -1) ? 
 // skipped.  The two exponentials are evaluated as one exp of the summed
 // exponents with per-pixel reciprocals (within WGSL's accuracy for '/' and
 // exp); taps of zero normal weight add nothing and are skipped.
-VRT_DI float4 atrous_pixel(int W, int H, int px, int py, const void* __restrict__ src, bool srcF32,
-                           const float4* __restrict__ gbuf, int step) {
+VRT_DI float4 atrous_pixel(int W, int H, int px, int py, const void* src, bool srcF32, const float4* gbuf,
+                           int step) {
   const size_t p = (size_t)py * W + px;
   const float4 center = load_px(src, srcF32, p);
-  const float4 g = __ldg(gbuf + p);
+  const float4 g = gbuf[p];
   if (g.w < 0.0f) return center;
   const float history = fmax_(center.w, 1.0f);
   const float lumC = luminance(center.x, center.y, center.z);
@@ -106,7 +107,7 @@ VRT_DI float4 atrous_pixel(int W, int H, int px, int py, const void* __restrict_
       const int qx = px + dx * step, qy = py + dy * step;
       if (qx < 0 || qy < 0 || qx >= W || qy >= H) continue;
       const size_t q = (size_t)qy * W + qx;
-      const float4 gq = __ldg(gbuf + q);
+      const float4 gq = gbuf[q];
       if (gq.w < 0.0f) continue;
       const float nd = fmax_(__fmaf_rn(g.z, gq.z, __fmaf_rn(g.y, gq.y, g.x * gq.x)), 0.0f);
       const float n2 = nd * nd, n4 = n2 * n2, n8 = n4 * n4, n16 = n8 * n8, n32 = n16 * n16;

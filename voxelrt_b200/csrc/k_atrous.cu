@@ -16,8 +16,8 @@ namespace vrt {
 // 104 / 107, 1920x1080 201 / 197: the line is at two full waves of 32-row tiles
 // (3 on each of 148 SMs).  8 rows: no better at any size.
 template <int S, int R, bool kSrcF32>
-__global__ void __launch_bounds__(8 * R, 96 / R) k_atrous(int W, int H, const void* __restrict__ src,
-                                                          const float4* __restrict__ gbuf, uint2* __restrict__ dst) {
+__global__ void __launch_bounds__(8 * R, 96 / R) k_atrous(int W, int H, const void* src, const float4* gbuf,
+                                                          uint2* __restrict__ dst) {
   frame_begin();
   extern __shared__ float4 sm[];
   atrous_tile<S, R>(sm, AtrousImage{W, H, src, kSrcF32, gbuf, dst}, blockIdx.x * kAtrousTile, blockIdx.y * R);

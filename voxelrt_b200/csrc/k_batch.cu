@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(256) k_b_present(MultiJob J, uint32_t P, const
   const uint32_t lp = g - jd.first;
   const bool denoise = (jd.u.params0[2] & 2u) != 0u;
   const float4 il = denoise ? load_px(jd.den0, false, lp) : load_px(jd.acc_cur, jd.acc_f32 != 0, lp);
-  jd.ldr[lp] = present_pixel(jd.u.params1[2], il, __ldg(jd.out.alb8 + lp), lut);
+  jd.ldr[lp] = present_pixel(jd.u.params1[2], il, jd.out.alb8[lp], lut);
 }
 
 cudaError_t launch_batch_frame(const void* d_jobs, const uint32_t* d_firsts, int n, int max_bg, uint32_t P, int waves,

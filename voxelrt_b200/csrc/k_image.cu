@@ -18,9 +18,9 @@ namespace vrt {
 // history (WebGPU linear filter: texel centres at +0.5, clamp to edge).
 // ---------------------------------------------------------------------------
 template <bool kAccF32>
-__global__ void __launch_bounds__(256) k_temporal(Uni u, int W, int H, const uint2* __restrict__ rad,
-                                                  const float4* __restrict__ gcur, const void* __restrict__ accPrev,
-                                                  const float4* __restrict__ gprev, void* __restrict__ accOut) {
+__global__ void __launch_bounds__(256) k_temporal(Uni u, int W, int H, const uint2* rad, const float4* gcur,
+                                                  const void* accPrev, const float4* gprev,
+                                                  void* __restrict__ accOut) {
   frame_begin();
   const int gx = blockIdx.x * 32 + (threadIdx.x & 31);
   const int gy = blockIdx.y * 8 + (threadIdx.x >> 5);
@@ -36,8 +36,8 @@ __global__ void __launch_bounds__(256) k_temporal(Uni u, int W, int H, const uin
 // when a buffer is not 16-byte aligned).
 template <bool kFinF32>
 __global__ void __launch_bounds__(256) k_present(float exposure, uint32_t P, uint32_t n4,
-                                                 const void* __restrict__ fin, const uint32_t* __restrict__ alb8,
-                                                 uint32_t* __restrict__ ldr, const float* __restrict__ lut) {
+                                                 const void* fin, const uint32_t* alb8, uint32_t* __restrict__ ldr,
+                                                 const float* __restrict__ lut) {
   frame_begin();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n4) {
@@ -45,16 +45,16 @@ __global__ void __launch_bounds__(256) k_present(float exposure, uint32_t P, uin
     if (kFinF32) {
       const float4* f = reinterpret_cast<const float4*>(fin) + 4u * (size_t)i;
 #pragma unroll
-      for (int k = 0; k < 4; k++) il[k] = __ldg(f + k);
+      for (int k = 0; k < 4; k++) il[k] = f[k];
     } else {
       const uint4* f = reinterpret_cast<const uint4*>(fin) + 2u * (size_t)i;
-      const uint4 a = __ldg(f), b = __ldg(f + 1);
+      const uint4 a = f[0], b = f[1];
       il[0] = unpack_h4(make_uint2(a.x, a.y));
       il[1] = unpack_h4(make_uint2(a.z, a.w));
       il[2] = unpack_h4(make_uint2(b.x, b.y));
       il[3] = unpack_h4(make_uint2(b.z, b.w));
     }
-    const uint4 al = __ldg(reinterpret_cast<const uint4*>(alb8) + i);
+    const uint4 al = reinterpret_cast<const uint4*>(alb8)[i];
     uint4 o;
     o.x = present_pixel(exposure, il[0], al.x, lut);
     o.y = present_pixel(exposure, il[1], al.y, lut);
@@ -64,7 +64,7 @@ __global__ void __launch_bounds__(256) k_present(float exposure, uint32_t P, uin
   } else {
     const size_t p = 4u * (size_t)n4 + (i - n4);
     if (p >= P) return;
-    ldr[p] = present_pixel(exposure, load_px(fin, kFinF32, p), __ldg(alb8 + p), lut);
+    ldr[p] = present_pixel(exposure, load_px(fin, kFinF32, p), alb8[p], lut);
   }
 }
 

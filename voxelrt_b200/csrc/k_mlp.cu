@@ -230,10 +230,10 @@ __device__ __forceinline__ int image_index(int i) {
 static_assert(kWEnd == kParams * 2, "the weight image holds every parameter once");
 
 // Copies the weight image (kWEnd bytes) into shared memory, 16 bytes per access.
-__device__ __forceinline__ void load_weights(uint8_t* smem, const uint16_t* __restrict__ w) {
+__device__ __forceinline__ void load_weights(uint8_t* smem, const uint16_t* w) {
   const uint4* src = reinterpret_cast<const uint4*>(w);
   uint4* dst = reinterpret_cast<uint4*>(smem);
-  for (int i = threadIdx.x; i < kWEnd / 16; i += blockDim.x) dst[i] = __ldg(src + i);
+  for (int i = threadIdx.x; i < kWEnd / 16; i += blockDim.x) dst[i] = src[i];
 }
 
 struct Ctl {
@@ -359,7 +359,7 @@ __device__ __forceinline__ void store_row_where(uint8_t* tile, const uint8_t* ac
 
 // Writes the encoded input of sample `src` (zeros when idx >= n) into row
 // `row` of the input tile.
-__device__ __forceinline__ void stage_input(uint8_t* tile, int row, const float* __restrict__ q9, int n, int idx,
+__device__ __forceinline__ void stage_input(uint8_t* tile, int row, const float* q9, int n, int idx,
                                             float extent, int src) {
   float f[kIn];
   if (idx < n) {
@@ -493,7 +493,7 @@ __global__ void __launch_bounds__(256, 2) k_mlp_infer(const __grid_constant__ Ml
       const int idx = (pair_tile + u * vctas) * 128 + t;
       if (idx < n) {
 #pragma unroll
-        for (int j = 0; j < 9; j++) q[u][j] = __ldg(tk.q9 + (size_t)idx * 9 + j);
+        for (int j = 0; j < 9; j++) q[u][j] = tk.q9[(size_t)idx * 9 + j];
       }
     }
   };
@@ -583,8 +583,8 @@ __global__ void __launch_bounds__(256, 1) k_mlp_grad(const __grid_constant__ Mlp
   using namespace mlp;
   const MlpTask& tk = ts.t[task_of(ts, blockIdx.x)];
   const int cb = blockIdx.x - tk.cta0;
-  const float* __restrict__ q9 = tk.q9;
-  const float* __restrict__ y3 = tk.y3;
+  const float* q9 = tk.q9;
+  const float* y3 = tk.y3;
   const float extent = tk.extent;
   int n, pop;
   bool draw;
@@ -619,9 +619,9 @@ __global__ void __launch_bounds__(256, 1) k_mlp_grad(const __grid_constant__ Mlp
     if (tile_ < tiles && idx_ < n) {
       const int src_ = sample_source(idx_, pop, draw, seed);
 #pragma unroll
-      for (int j = 0; j < 9; j++) qn[j] = __ldg(q9 + (size_t)src_ * 9 + j);
+      for (int j = 0; j < 9; j++) qn[j] = q9[(size_t)src_ * 9 + j];
 #pragma unroll
-      for (int j = 0; j < 3; j++) yn[j] = __ldg(y3 + (size_t)src_ * 3 + j);
+      for (int j = 0; j < 3; j++) yn[j] = y3[(size_t)src_ * 3 + j];
     }
   };
   fetch(cb);

@@ -314,7 +314,11 @@ VRT_DI F3 cosine_hemisphere(F3 n, uint32_t& rng) {
 // frame_begin, before it reads or writes memory: all threads wait until the
 // kernels ahead are complete and their writes visible, then allow the next kernel's
 // blocks onto the SMs.  A kernel so launched is complete only after its own
-// wait, so the order of the whole stream holds.
+// wait, so the order of the whole stream holds.  What another such kernel writes
+// (images, path state, weights, queries, samples) it reads with ordinary loads: the non-coherent path
+// (__ldg, const __restrict__ parameters) asks for memory that nothing writes as long as the reader is resident,
+// and such loads need not stay below the wait.  It is left for the scene, whose
+// edits are ordinary launches, and for tables uploaded ahead of the frame.
 VRT_DI void frame_begin() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
