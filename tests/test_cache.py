@@ -174,3 +174,30 @@ def test_cache_jobs_in_a_batch_match_alone(vrt, plain_beside, tail):
             np.testing.assert_array_equal(inb[i].albedo(), alone[i].albedo())
     st = batch.stats()
     assert st.cache_queries > 0 and st.cache_samples > 0
+
+
+@pytest.mark.parametrize("plain_beside", [False, True])
+def test_tail_from_wave_1_leaves_cache_frames(vrt, plain_beside):
+    """A tail wave of 1 set on a session or batch with the cache on: its paths still end in queries, and the first
+    frame's image is the one of the wave-by-wave form."""
+    W, H = 160, 90
+    vox, spawn, ctx, sc, _ = _setup(vrt, 16, 16)
+    u = vrt.make_uniforms(spawn, None, vrt.Lighting(), 4, 2, 0, W, H)
+    got = []
+    for tail in (0, 1):
+        s = vrt.Session(ctx, sc, W, H, firefly_clamp=10.0, keep_radiance_f32=True)
+        views = [vrt.Session(ctx, sc, W, H, firefly_clamp=10.0, keep_radiance_f32=True, path_kernel="batch_only")
+                 for _ in range(2 if plain_beside else 1)]
+        for t in (s, views[0]):
+            t.set_cache(seed=7)
+        batch = vrt.Batch(ctx, views)
+        for t in (s, batch):
+            t.set_tuning(tail_wave=tail)
+        s.frame(u)
+        batch.frame([u] * len(views))
+        st = s.stats()
+        got.append([st.cache_queries, st.rays, batch.stats().cache_queries] +
+                   [t.radiance_f32().tobytes() for t in (s, *views)])
+        batch.close()
+    assert got[0][0] > 0
+    assert got[0] == got[1]

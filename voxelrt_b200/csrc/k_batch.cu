@@ -97,7 +97,7 @@ cudaError_t launch_batch_frame(const void* d_jobs, const uint32_t* d_firsts, int
   J.n = n;
   J.cache_jobs = ncl;
   J.max_bg = max_bg;
-  const int tail = tune.tail_wave >= 0 ? tune.tail_wave : auto_tail(P, waves, ncl > 0, ncl > 0 && ncl == n);
+  const int tail = frame_tail(tune, P, waves, ncl > 0, ncl > 0 && ncl == n);
   cudaError_t e = wf_launch_frame(J, P, waves, wb, tune, stats, st, launches, nullptr, 0, nullptr, n, tail);
   if (e != cudaSuccess) return e;
   // the cache jobs' inference, resolve and training, all jobs per launch

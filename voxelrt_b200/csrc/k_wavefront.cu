@@ -81,7 +81,7 @@ cudaError_t launch_wavefront(const SceneDev& s, const VrtUniforms& uu, float fcl
   // cache-assisted frames run as many waves as their training paths need
   const int waves = (job.cc.on ? (int)job.cc.train_bounces : (int)job.u.params0[1]) + 2;
   const bool cc = job.cc.on != 0;
-  const int tail = tune.tail_wave >= 0 ? tune.tail_wave : auto_tail((uint32_t)(W * H), waves, cc, cc);
+  const int tail = frame_tail(tune, (uint32_t)(W * H), waves, cc, cc);
   cudaError_t e = wf_launch_frame(job, (uint32_t)(W * H), waves, wb, tune, out.stats, st, launches, trace_ev,
                                   max_timed_waves, timed_waves, 1, tail);
   if (e != cudaSuccess || !job.cc.on) return e;

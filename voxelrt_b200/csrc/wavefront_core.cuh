@@ -1172,7 +1172,7 @@ cudaError_t wf_run_waves(const J& jobs, uint32_t P, int waves, const WavefrontBu
 //  2.1 M, 2: 1.148 / 1.96 / 1.56 / 1.175   2.1 M, 6: 1.453 / 2.57 / 2.16 / 1.69 / 1.424 / 1.380
 // (The tail's grid holds 95 K paths at once; a few more cost it a second round.)
 // Cache-assisted frames (every path but the training paths ends at wave 1)
-// always take wave 2, and no job with the cache can take wave 1.
+// always take wave 2, and with the cache on no frame takes wave 1 (frame_tail).
 inline int auto_tail(uint32_t P, int waves, bool any_cache, bool all_cache) {
   if (all_cache) return 2;
   const bool deep = waves > 4;   // 3 bounces or more
@@ -1184,6 +1184,13 @@ inline int auto_tail(uint32_t P, int waves, bool any_cache, bool all_cache) {
   else if (P <= 1500000u) w = 4;
   else w = 5;
   return w < waves ? w : 0;
+}
+
+// The tail wave of a frame: as tuned, else automatic.  A path that the cache ends turns into a query in
+// wave 1's shading, which the tail does not do, so with any such path in the frame the tail begins at wave 2.
+inline int frame_tail(const WavefrontTuning& tune, uint32_t P, int waves, bool any_cache, bool all_cache) {
+  const int w = tune.tail_wave >= 0 ? tune.tail_wave : auto_tail(P, waves, any_cache, all_cache);
+  return any_cache && w == 1 ? 2 : w;
 }
 
 // The plain path's wave sequence (with the radiance cache's counter reset
