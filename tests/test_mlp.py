@@ -184,3 +184,45 @@ def test_bounded_wait_runs_out_and_context_survives(vrt, cache):
     out = torch.zeros(900, dtype=torch.float32, device="cuda")
     cache.infer(_cuda(q), out)
     assert torch.isfinite(out).all()
+
+
+@pytest.mark.parametrize("tiny", [1e-20, 1e-23])
+def test_gradient_through_tiny_activations(vrt, orc, cache, tiny):
+    """A positive pre-activation below half of bf16's least value (tiny * 1e-21) is stored as next to nothing, but the
+    ReLU's derivative there is 1.  Tolerance: that of test_mlp_gradient_matches_oracle."""
+    import torch
+    from oracle import mlp_ref as M
+    rng = np.random.default_rng(3)
+    q, y = _queries(rng, 700)
+    ws = [rng.normal(size=s).astype(np.float32) * np.float32(0.1) for s in M.SHAPES]
+    ws[3][:, 3:] = 0.0
+    ws[0][:, 3] = 0.0
+    ws[0][78, 3] = tiny                        # feature 78 is the constant 1
+    ws[1][:, 7] = 0.0
+    ws[1][3, 7] = 1e-21
+    ws[2][7, :] = 1.0
+    p = M.pack(ws).astype(np.float32)
+    cache.set_params(p)
+    g = torch.zeros(M.N_PARAMS, dtype=torch.float32, device="cuda")
+    cache.gradient(_cuda(q), _cuda(y), g)
+    got, want = M.unpack(g.cpu().numpy())[1], M.unpack(M.gradient(M.encode(q, EXTENT), y, p)[1])[1]
+    assert np.abs(want[:, 7]).max() > 0.1 * np.abs(want).max()
+    assert np.all(np.abs(got - want) <= 2e-3 * np.abs(want).max() + 1e-2 * np.abs(want))
+
+
+def test_gradient_with_a_nan_query(vrt, cache):
+    """The pre-activations of a NaN query are NaN and count as 0: its sample adds to the loss and to no gradient but
+    that of the weights its NaN feature meets.  So the sum over 257 samples with it is the sum over the 256 without it
+    (both means carry two fp32 roundings)."""
+    import torch
+    q, y = _queries(np.random.default_rng(4), 257)
+    q[256, 3] = np.nan                          # feature 72
+    out = []
+    for n in (256, 257):
+        g = torch.zeros(14336, dtype=torch.float32, device="cuda")
+        loss = cache.gradient(_cuda(q[:n]), _cuda(y[:n]), g)
+        assert np.isfinite(loss)
+        out.append(g.cpu().numpy().astype(np.float64) * n)
+    keep = np.ones(14336, bool)
+    keep[72 * 64:73 * 64] = False
+    np.testing.assert_allclose(out[1][keep], out[0][keep], rtol=4 * 2.0 ** -24, atol=0)

@@ -212,6 +212,29 @@ __device__ __forceinline__ void store_row_relu(uint8_t* tile, int row, int C, co
     *reinterpret_cast<uint4*>(tile + umma::canon_off(row, 8 * cg, C)) = pack8_relu(v + 8 * cg);
 }
 
+// Row `row` of a 64-column activation tile of the training kernel: h > 0 ? h : 0
+// in bf16 (a NaN becomes 0, unlike pack8_relu's), in which a positive h is never
+// stored as 0, since the backward pass takes the ReLU's derivative from here.  The added
+// half of bf16's least value (2^-134) sees to that: it lifts every positive h over
+// the tie and leaves 0 on it (rounded to even, 0), and above 2^-109 it is lost
+// in the sum.
+__device__ __forceinline__ void store_row_hidden(uint8_t* tile, int row, const float* v) {
+  const float2 half = make_float2(0x1p-134f, 0x1p-134f);
+  const __nv_bfloat162 zero = __floats2bfloat162_rn(0.0f, 0.0f);
+#pragma unroll
+  for (int cg = 0; cg < kHid / 8; cg++) {
+    uint4 r;
+    uint32_t* w = &r.x;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const float2 x = f2_add(make_float2(v[8 * cg + 2 * i], v[8 * cg + 2 * i + 1]), half);
+      const __nv_bfloat162 h = __hmax2(__floats2bfloat162_rn(x.x, x.y), zero);   // of 0 and a NaN: 0
+      w[i] = *reinterpret_cast<const uint32_t*>(&h);
+    }
+    *reinterpret_cast<uint4*>(tile + umma::canon_off(row, 8 * cg, kHid)) = r;
+  }
+}
+
 // The bf16 weight copy is kept in global memory as the kernels' shared-memory
 // image of the weights: for each layer W^T (rows N_out, columns K_in) in the
 // canonical no-swizzle layout at byte offset kWf<l>, kWEnd bytes in all.
@@ -329,7 +352,7 @@ __device__ __forceinline__ void forward_tile(uint8_t* smem, uint32_t tbase, Ctl&
     sync_mma(c);
     float h[kHid];
     tmem_row<kHid>(tbase, tcol, h);
-    store_row_relu(smem + aout[l] + g * gstride, r, kHid, h);
+    store_row_hidden(smem + aout[l] + g * gstride, r, h);
     publish();
   }
   if (t == 0)
@@ -341,7 +364,7 @@ __device__ __forceinline__ void forward_tile(uint8_t* smem, uint32_t tbase, Ctl&
 // Row `row` of a 64-column tile from the input gradients dx, zero where the
 // layer's activation (row `row` of `act`) is zero: the ReLU's derivative, taken
 // from the stored activations two at a time instead of from a mask of the
-// pre-activations (the stored value of a positive pre-activation is positive).
+// pre-activations (store_row_hidden keeps a positive one positive).
 __device__ __forceinline__ void store_row_where(uint8_t* tile, const uint8_t* act, int row, const float* dx) {
   const __nv_bfloat162 zero = __floats2bfloat162_rn(0.0f, 0.0f);
 #pragma unroll
