@@ -226,3 +226,26 @@ def test_gradient_with_a_nan_query(vrt, cache):
     keep = np.ones(14336, bool)
     keep[72 * 64:73 * 64] = False
     np.testing.assert_allclose(out[1][keep], out[0][keep], rtol=4 * 2.0 ** -24, atol=0)
+
+
+@pytest.mark.parametrize("shift", [0, 4, 6])
+def test_gradient_into_any_alignment(vrt, cache, shift):
+    """The caller's array at byte offsets that a kernel can (0, 4) and cannot (6) store floats to."""
+    import ctypes as C
+
+    import torch
+    q, y = (_cuda(a) for a in _queries(np.random.default_rng(6), 300))
+    want = torch.zeros(14336, dtype=torch.float32, device="cuda")
+    loss = cache.gradient(q, y, want)
+    buf = torch.full((14336 * 4 + 16,), 0x55, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    for with_loss in (True, False):
+        got = C.c_float()
+        code = vrt.lib.vrt_mlp_gradient_device(cache.h, C.c_void_p(q.data_ptr()), C.c_void_p(y.data_ptr()), 300,
+                                               C.c_float(EXTENT), C.c_void_p(buf.data_ptr() + shift),
+                                               C.byref(got) if with_loss else None)
+        assert code == 0, vrt.lib.vrt_last_error_string().decode()
+        b = buf.cpu().numpy()
+        assert b[shift:shift + 14336 * 4].tobytes() == want.cpu().numpy().tobytes()
+        assert np.all(b[:shift] == 0x55) and np.all(b[shift + 14336 * 4:] == 0x55)
+        assert not with_loss or got.value == loss

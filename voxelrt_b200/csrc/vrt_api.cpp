@@ -2059,8 +2059,18 @@ int vrt_mlp_gradient_device(VrtMlp* m, const float* d_q9, const float* d_y3, int
                             float* loss_out) {
   if (!m || n < 1 || !d_q9 || !d_y3 || !(extent > 0.0f)) return fail(VRT_ERR_INVALID, "bad argument");
   if (int r = set_dev(m->ctx)) return r;
-  if (int r = mlp_grad_impl(m, d_q9, d_y3, n, extent, d_grad ? d_grad : m->grad, loss_out, false)) return r;
-  return loss_out ? VRT_OK : mlp_check_err(m);
+  // The reduction writes the caller's array itself where it lies on this device and is aligned; any other
+  // array (misaligned, on the host, on another device) takes a copy, which accepts or refuses it.
+  bool direct = false;
+  if (d_grad && ((uintptr_t)d_grad & 3u) == 0u) {
+    cudaPointerAttributes at;
+    CUDA_TRY(cudaPointerGetAttributes(&at, d_grad));
+    direct = at.type == cudaMemoryTypeDevice && at.device == m->ctx->device;
+  }
+  if (int r = mlp_grad_impl(m, d_q9, d_y3, n, extent, direct ? d_grad : m->grad, loss_out, false)) return r;
+  if (d_grad && !direct)
+    CUDA_TRY(cudaMemcpyAsync(d_grad, m->grad, (size_t)m->P * 4, cudaMemcpyDeviceToDevice, m->ctx->stream));
+  return loss_out && (direct || !d_grad) ? VRT_OK : mlp_check_err(m);
 }
 
 int vrt_mlp_train_device(VrtMlp* m, const float* d_q9, const float* d_y3, int n, float extent, float lr, int steps,
