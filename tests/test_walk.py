@@ -204,3 +204,24 @@ def test_short_directions_match_oracle(vrt, orc, ctx, grid):
     for f in ("mat", "voxel", "face", "steps", "bytes"):
         assert np.array_equal(got[f], want[f]), f
     sc.close()
+
+
+def test_host_entry_survives_device_pointers(vrt, ctx):
+    """vrt_trace_rays takes host arrays; device pointers get the runtime's answer at every batch size, and host arrays
+    are answered as before afterwards."""
+    import ctypes as C
+
+    import torch
+    vox, _ = vrt.generate_scene(vrt.VRT_SCENE_RANDOM, 64, 3)
+    sc = vrt.Scene(ctx, vox, 64)
+    o, d, t = _odd_rays(64, 4.0, 5)
+    want = sc.trace_rays(o, d, t).tobytes()
+    dev = torch.zeros(20_000 * 12, dtype=torch.float32, device="cuda")
+    host = np.zeros(20_000 * 12, np.float32)
+    torch.cuda.synchronize()
+    p, q = C.c_void_p(dev.data_ptr()), C.c_void_p(host.ctypes.data)
+    for args in ((p, q, q, q), (q, p, q, q), (q, q, p, q), (q, q, q, p)):
+        few, many = (vrt.lib.vrt_trace_rays(sc.h, *args[:3], n, args[3]) for n in (64, 20_000))
+        assert few == many
+    assert sc.trace_rays(o, d, t).tobytes() == want
+    sc.close()

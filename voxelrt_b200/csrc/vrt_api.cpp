@@ -403,6 +403,12 @@ int vrt_trace_rays_device(VrtScene* s, const float* o, const float* d, const flo
 
 constexpr int kRayStage = 16384;   // rays of the staged path (1.2 MB of pinned memory per context)
 
+// Whether the host itself can read and write p (the runtime knows it as no device allocation).
+static bool host_memory(const void* p) {
+  cudaPointerAttributes at;
+  return cudaPointerGetAttributes(&at, p) == cudaSuccess && at.type != cudaMemoryTypeDevice;
+}
+
 int vrt_trace_rays(VrtScene* s, const float* o, const float* d, const float* tmax, int n, VrtHit* out) {
   if (!s || n < 0) return fail(VRT_ERR_INVALID, "bad argument");
   if (n == 0) return VRT_OK;
@@ -412,8 +418,9 @@ int vrt_trace_rays(VrtScene* s, const float* o, const float* d, const float* tma
   const size_t bo = (size_t)n * 12, bt = (size_t)n * 4, bh = (size_t)n * sizeof(VrtHit);
   // Small batches through pinned memory that the kernel reads and writes itself: one launch and one
   // wait, where an allocation and four copies took most of the call (64 rays 61 -> 32 us, 5000 rays
-  // 132 -> 72, 16384 rays 239 -> 195).  Past kRayStage the copies themselves decide.
-  if (n <= kRayStage) {
+  // 132 -> 72, 16384 rays 239 -> 195).  Past kRayStage the copies themselves decide.  Device pointers,
+  // which are none of this entry's, are left to the copies to refuse.
+  if (n <= kRayStage && host_memory(o) && host_memory(d) && host_memory(tmax) && host_memory(out)) {
     VrtCtx* c = s->ctx;
     if (!c->ray_stage)
       CUDA_TRY(cudaHostAlloc((void**)&c->ray_stage, (size_t)kRayStage * (28 + sizeof(VrtHit)),
