@@ -225,3 +225,26 @@ def test_host_entry_survives_device_pointers(vrt, ctx):
         assert few == many
     assert sc.trace_rays(o, d, t).tobytes() == want
     sc.close()
+
+
+def test_ray_batches_of_several_threads(vrt, ctx):
+    """Threads that query one world at once, with batches of the sizes that go through the context's pinned memory:
+    each gets its own rays' hits."""
+    import threading
+    vox, _ = vrt.generate_scene(vrt.VRT_SCENE_RANDOM, 64, 3)
+    sc = vrt.Scene(ctx, vox, 64)
+    rays = [_odd_rays(n, 4.0, n) for n in (1, 64, 700, 5000, 16_384, 16_385)]
+    want = [sc.trace_rays(*r).tobytes() for r in rays]
+    wrong = []
+
+    def work(k):
+        for _ in range(60):
+            if sc.trace_rays(*rays[k]).tobytes() != want[k]:
+                wrong.append(k)
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(len(rays))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
+    sc.close()

@@ -68,6 +68,7 @@ struct VrtCtx {
   uint64_t used = 0;
   float* present_lut = nullptr;   // kPresentLut floats, built on the stream at creation
   char* ray_stage = nullptr;      // pinned staging of small ray batches (vrt_trace_rays), on first use
+  std::mutex ray_mutex;           // held by the call that uses it
 };
 
 struct VrtScene {
@@ -419,9 +420,11 @@ int vrt_trace_rays(VrtScene* s, const float* o, const float* d, const float* tma
   // Small batches through pinned memory that the kernel reads and writes itself: one launch and one
   // wait, where an allocation and four copies took most of the call (64 rays 61 -> 32 us, 5000 rays
   // 132 -> 72, 16384 rays 239 -> 195).  Past kRayStage the copies themselves decide.  Device pointers,
-  // which are none of this entry's, are left to the copies to refuse.
-  if (n <= kRayStage && host_memory(o) && host_memory(d) && host_memory(tmax) && host_memory(out)) {
-    VrtCtx* c = s->ctx;
+  // which are none of this entry's, are left to the copies to refuse; and a call that finds the staging
+  // taken by another thread's copies through memory of its own.
+  VrtCtx* c = s->ctx;
+  std::unique_lock<std::mutex> stage(c->ray_mutex, std::defer_lock);
+  if (n <= kRayStage && host_memory(o) && host_memory(d) && host_memory(tmax) && host_memory(out) && stage.try_lock()) {
     if (!c->ray_stage)
       CUDA_TRY(cudaHostAlloc((void**)&c->ray_stage, (size_t)kRayStage * (28 + sizeof(VrtHit)),
                              cudaHostAllocMapped | cudaHostAllocPortable));
