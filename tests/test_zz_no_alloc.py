@@ -15,6 +15,7 @@ also check that the device's free memory does not change across calls.  This
 file is collected last so a failure here cannot hide the other tests' results.
 """
 import ctypes as C
+import math
 
 import numpy as np
 import pytest
@@ -131,3 +132,30 @@ def test_noalloc_tiles(vrt, orc, W, H, acc_f32, form):
     nan = np.isnan(want.view(np.float16))
     assert np.array_equal(nan, np.isnan(got.view(np.float16)))
     assert np.array_equal(got[~nan], want[~nan])
+
+
+# Odd values in every tile while the normals stay on the axes, and tiles of nothing but one odd value; distances too.
+@pytest.mark.parametrize("value", [-2.0, -0.0, np.inf, np.nan, 1e25])
+@pytest.mark.parametrize("W,H,share", [(33, 17, 1.0), (65, 47, 0.3), (970, 965, 0.002)])
+def test_noalloc_odd_values(vrt, orc, W, H, share, value):
+    import torch
+    from voxelrt_b200._lib import lib
+
+    r = np.random.default_rng(W)
+    gb = np.zeros((H, W, 4), np.float32)
+    np.put_along_axis(gb, r.integers(0, 3, (H, W, 1)), 1.0, axis=2)
+    gb[..., 3] = np.where(r.random((H, W)) < 0.1, -1.0, 2.0 + 0.1 * r.random((H, W)))
+    acc = np.zeros((H, W, 4), np.float32)
+    acc[..., :3] = np.where(r.random((H, W, 1)) < 0.3, 0.0, np.exp(r.normal(size=(H, W, 3))))
+    acc[..., 3] = r.integers(0, 65, (H, W))
+    acc[..., :3][r.random((H, W)) < share] = value
+    if np.isinf(value) or np.isnan(value):
+        gb[(r.random((H, W)) < share / 4) & (gb[..., 3] > 0), 3] = value
+    for tilted in (False, True):
+        if tilted:
+            gb[r.random((H, W)) < 0.3, :3] = np.float32(1.0 / math.sqrt(3.0))
+        got, _, _ = _run_noalloc(lib, torch, torch.device("cuda:0"), acc, True, gb, W, H)
+        want = _oracle_chain(orc, acc, True, gb, W, H)
+        nan = np.isnan(want.view(np.float16))
+        assert np.array_equal(nan, np.isnan(got.view(np.float16)))
+        assert np.array_equal(got[~nan], want[~nan])

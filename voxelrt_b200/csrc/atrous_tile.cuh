@@ -1,6 +1,10 @@
 // atrous_tile.cuh -- one a-trous iteration (atrous.wgsl:26-83) over a tile of
 // 32 x R output pixels (R = 32, or 16 for small images), shared by the single-image kernel (k_atrous.cu) and
-// the batched one (k_batch.cu).
+// the batched one (k_batch.cu): 5x5 B3-spline taps at the step, weights
+// normal^32 * exp(-(|dt| / (0.05 t + 0.01) + |dL| / sigmaL)),
+// sigmaL = max(0.08, 2/sqrt(max(history,1))); sky, out-of-image taps and taps of
+// zero normal weight skipped.  The two exponentials are one exp of the summed
+// exponents with per-pixel reciprocals (within WGSL's accuracy for '/' and exp).
 //
 // Bound by arithmetic: 24 taps per pixel of up to 30 fp32 operations (a power
 // of 32, an exponential, four sums), all of them part of the bit-exact
@@ -21,10 +25,10 @@
 //    sky, a zero normal weight) adds a product with a weight of 0.  That
 //    changes no bit while every staged colour is finite and not negative (nor
 //    -0) and normals' components are at most 1.01; a tile with any other value
-//    takes the per-pixel form (atrous_pixel), which does skip.
+//    takes the form that keeps the sums of a skipped tap by a select (kOdd).
 //  * The exponent is clamped at 87 instead of selecting 0 past it: the weight
 //    is then at most 1.7e-38, which no sum can see while colours stay below
-//    1e20 (same check).
+//    1e20 (same check; kOdd selects).
 // floor() is a rounded-down addition of 1.5 * 2^23, exact for these exponents
 // and without conversions; the signs in exp's polynomial are arranged for the
 // negated argument, each product and sum rounding as in exp_nonpos_.
@@ -92,21 +96,27 @@ struct CentrePair {
 
 // The tap `t` at kernel weight wk (passed negated: the exponential below
 // comes out negated too).
-template <bool kUnit>
+template <bool kUnit, bool kOdd>
 VRT_DI void tap_pair(CentrePair& c, const TapPair& t, float nwk) {
   float2 wn;   // -(kernel weight x normal weight)
+  bool skip0 = false, skip1 = false;   // kOdd: the definition skips the tap
   if (kUnit) {
-    wn = f2(c.x.x == t.x.x ? nwk : 0.0f, c.x.y == t.x.y ? nwk : 0.0f);
+    skip0 = c.x.x != t.x.x;
+    skip1 = c.x.y != t.x.y;
+    wn = f2(skip0 ? 0.0f : nwk, skip1 ? 0.0f : nwk);
   } else {
     float2 nd = f2_fma(c.z, t.z, f2_fma(c.y, t.y, f2_mul(c.x, t.x)));
-    nd = f2(fmaxf(nd.x, 0.0f), fmaxf(nd.y, 0.0f));
+    nd = kOdd ? f2(fmax_(nd.x, 0.0f), fmax_(nd.y, 0.0f)) : f2(fmaxf(nd.x, 0.0f), fmaxf(nd.y, 0.0f));
     const float2 n2 = f2_mul(nd, nd), n4 = f2_mul(n2, n2), n8 = f2_mul(n4, n4), n16 = f2_mul(n8, n8),
                  n32 = f2_mul(n16, n16);
     wn = f2_mul(n32, f2(nwk, nwk));
+    skip0 = n32.x == 0.0f || t.w.x < 0.0f;
+    skip1 = n32.y == 0.0f || t.w.y < 0.0f;
   }
   const float2 dt = f2_sub(c.w, t.w), dl = f2_sub(c.l, t.l);
   float2 v = f2_fma(f2(fabsf(dt.x), fabsf(dt.y)), c.invD, f2(fabsf(dl.x) * c.invS.x, fabsf(dl.y) * c.invS.y));
-  v = f2(fminf(v.x, 87.0f), fminf(v.y, 87.0f));
+  const bool far0 = !(v.x < 87.0f), far1 = !(v.y < 87.0f);
+  if (!kOdd) v = f2(fminf(v.x, 87.0f), fminf(v.y, 87.0f));
   // exp_nonpos_(-v), negated
   const float2 k2 = f2_add_rd(f2_fma(v, f2(-1.44269502f, -1.44269502f), f2(0.5f, 0.5f)), f2(12582912.0f, 12582912.0f));
   const float2 kf = f2_sub(k2, f2(12582912.0f, 12582912.0f));
@@ -119,21 +129,22 @@ VRT_DI void tap_pair(CentrePair& c, const TapPair& t, float nwk) {
   p = f2_fma(r, p, f2(-0.5f, -0.5f));
   p = f2_fma(r, p, f2(1.0f, 1.0f));
   p = f2_fma(r, p, f2(-1.0f, -1.0f));
-  const float2 e = f2(__int_as_float(__float_as_int(p.x) + (__float_as_int(k2.x) << 23)),
-                      __int_as_float(__float_as_int(p.y) + (__float_as_int(k2.y) << 23)));
+  float2 e = f2(__int_as_float(__float_as_int(p.x) + (__float_as_int(k2.x) << 23)),
+                __int_as_float(__float_as_int(p.y) + (__float_as_int(k2.y) << 23)));
+  if (kOdd) e = f2(far0 ? -0.0f : e.x, far1 ? -0.0f : e.y);
   const float2 w = f2_mul(wn, e);
+  if (kOdd) {
+    const float2 r2 = f2_fma(t.r, w, c.sr), g2 = f2_fma(t.g, w, c.sg), b2 = f2_fma(t.b, w, c.sb);
+    if (!skip0) { c.sr.x = r2.x; c.sg.x = g2.x; c.sb.x = b2.x; c.ws.x = c.ws.x + w.x; }
+    if (!skip1) { c.sr.y = r2.y; c.sg.y = g2.y; c.sb.y = b2.y; c.ws.y = c.ws.y + w.y; }
+    return;
+  }
   c.sr = f2_fma(t.r, w, c.sr);
   c.sg = f2_fma(t.g, w, c.sg);
   c.sb = f2_fma(t.b, w, c.sb);
   // scalar: a packed add of the packed product would be fused with it
   c.ws.x = c.ws.x + w.x;
   c.ws.y = c.ws.y + w.y;
-}
-
-// atrous_pixel out of line, for the tiles it is left to.
-static __device__ __noinline__ float4 atrous_pixel_plain(int W, int H, int px, int py, const void* src, bool src_f32,
-                                                         const float4* gbuf, int step) {
-  return atrous_pixel(W, H, px, py, src, src_f32, gbuf, step);
 }
 
 // Image of one iteration.
@@ -211,8 +222,9 @@ VRT_DI void load_alpha(const AtrousImage& I, int px, int y, float (&alpha)[kPair
 }
 
 // kPairs pairs of this thread: pixels px, px + 1 of image rows y + q S, staged
-// in rows ly + q S (the halo's corner is row 0) at pair column pc.
-template <int S, int R, bool kUnit, int kPairs>
+// in rows ly + q S (the halo's corner is row 0) at pair column pc.  kOdd: the
+// staged tile holds a value that asks for it.
+template <int S, int R, bool kUnit, int kPairs, bool kOdd>
 VRT_DI void filter_pairs(const float4* sm, const AtrousImage& I, int ne, int pc, int ly, int px, int y,
                          const float (&alpha)[kPairs][2]) {
   using G = AtrousGeom<S, R>;
@@ -268,8 +280,8 @@ VRT_DI void filter_pairs(const float4* sm, const AtrousImage& I, int ne, int pc,
           tp = prev;
         }
         const float wx = b3_weight(dx);
-        if (j < 5 && (dx != 0 || j != 2)) tap_pair<kUnit>(c[0], tp, -(wx * w0));
-        if (kPairs > 1 && j > 0 && (dx != 0 || j != 3)) tap_pair<kUnit>(c[kPairs - 1], tp, -(wx * w1));
+        if (j < 5 && (dx != 0 || j != 2)) tap_pair<kUnit, kOdd>(c[0], tp, -(wx * w0));
+        if (kPairs > 1 && j > 0 && (dx != 0 || j != 3)) tap_pair<kUnit, kOdd>(c[kPairs - 1], tp, -(wx * w1));
       }
     }
   }
@@ -305,30 +317,21 @@ VRT_DI void atrous_tile(float4* sm, const AtrousImage& I, int x0, int y0) {
   float alpha[2][2];
   load_alpha<S, 2>(I, x0 + 2 * pc, y0 + ya, alpha);
   const int flags = stage_tile<S, R, true>(sm, I, x0 - G::HX, y0 - G::HX, G::EH);
-  bool odd = __syncthreads_or(flags & kTileOdd) != 0;
+  const bool odd = __syncthreads_or(flags & kTileOdd) != 0;
   const bool full = __syncthreads_or(flags & kTileFullNormals) != 0;
-  if (!odd && !full) {
-    filter_pairs<S, R, true, 2>(sm, I, G::NE, pc, ya, x0 + 2 * pc, y0 + ya, alpha);
+  if (!full) {
+    if (!odd) filter_pairs<S, R, true, 2, false>(sm, I, G::NE, pc, ya, x0 + 2 * pc, y0 + ya, alpha);
+    else filter_pairs<S, R, true, 2, true>(sm, I, G::NE, pc, ya, x0 + 2 * pc, y0 + ya, alpha);
     return;
   }
   for (int half = 0; half < 2; half++) {   // R / 2 rows, one pair per thread
     const int yh = y0 + (R / 2) * half;
-    if (!odd) {
-      const int f = stage_tile<S, R, false>(sm, I, x0 - G::HX, yh - G::HX, G::HH);
-      odd = __syncthreads_or(f) != 0;
-    }
-    if (!odd) {
-      float a1[1][2];
-      load_alpha<S, 1>(I, x0 + 2 * pc, yh + rs, a1);
-      filter_pairs<S, R, false, 1>(sm, I, G::HE, pc, rs, x0 + 2 * pc, yh + rs, a1);
-    } else {
-      for (int k = 0; k < 2; k++) {
-        const int x = x0 + 2 * pc + k, y = yh + rs;
-        if (x >= I.W || y >= I.H) continue;
-        const float4 v = atrous_pixel_plain(I.W, I.H, x, y, I.src, I.src_f32, I.gbuf, S);
-        I.dst[(size_t)y * I.W + x] = pack_h4(v.x, v.y, v.z, v.w);
-      }
-    }
+    const int f = stage_tile<S, R, false>(sm, I, x0 - G::HX, yh - G::HX, G::HH);
+    const bool oddh = __syncthreads_or(f & kTileOdd) != 0;
+    float a1[1][2];
+    load_alpha<S, 1>(I, x0 + 2 * pc, yh + rs, a1);
+    if (!oddh) filter_pairs<S, R, false, 1, false>(sm, I, G::HE, pc, rs, x0 + 2 * pc, yh + rs, a1);
+    else filter_pairs<S, R, false, 1, true>(sm, I, G::HE, pc, rs, x0 + 2 * pc, yh + rs, a1);
     __syncthreads();   // the half's taps are read before the next half is staged
   }
 }

@@ -1,5 +1,5 @@
 // image_core.cuh -- per-pixel bodies of the image-space passes (temporal,
-// a-trous, present), shared by the single-session kernels (k_image.cu) and the
+// present; a-trous: atrous_tile.cuh), shared by the single-session kernels (k_image.cu) and the
 // batched kernels (k_batch.cu).
 #pragma once
 #include "vrt_device.cuh"
@@ -77,54 +77,6 @@ VRT_DI void store_px(void* base, bool f32, size_t p, float4 v) {
 
 // B3-spline taps (atrous.wgsl:26): 3/8, 1/4, 1/16 for |d| = 0, 1, 2.
 VRT_DI float b3_weight(int d) { return d == 0 ? 0.375f : ((d == 1 || d == -1) ? 0.25f : 0.0625f); }
-
-// atrous.wgsl:26-83 for pixel (px, py): 5x5 B3-spline taps at `step`,
-// weights normal^32 * exp(-(|dt| / (0.05 t + 0.01) + |dL| / sigmaL)),
-// sigmaL = max(0.08, 2/sqrt(max(history,1))); sky and out-of-image taps
-// skipped.  The two exponentials are evaluated as one exp of the summed
-// exponents with per-pixel reciprocals (within WGSL's accuracy for '/' and
-// exp); taps of zero normal weight add nothing and are skipped.
-VRT_DI float4 atrous_pixel(int W, int H, int px, int py, const void* src, bool srcF32, const float4* gbuf,
-                           int step) {
-  const size_t p = (size_t)py * W + px;
-  const float4 center = load_px(src, srcF32, p);
-  const float4 g = gbuf[p];
-  if (g.w < 0.0f) return center;
-  const float history = fmax_(center.w, 1.0f);
-  const float lumC = luminance(center.x, center.y, center.z);
-  const float sigmaL = fmax_(0.08f, 2.0f / __fsqrt_rn(history));
-  float sr = (center.x * 0.375f) * 0.375f;
-  float sg = (center.y * 0.375f) * 0.375f;
-  float sb = (center.z * 0.375f) * 0.375f;
-  float wSum = 0.140625f;
-  const float invD = 1.0f / (0.05f * g.w + 0.01f);
-  const float invS = 1.0f / sigmaL;
-#pragma unroll
-  for (int dy = -2; dy <= 2; dy++) {
-#pragma unroll
-    for (int dx = -2; dx <= 2; dx++) {
-      if (dx == 0 && dy == 0) continue;
-      const int qx = px + dx * step, qy = py + dy * step;
-      if (qx < 0 || qy < 0 || qx >= W || qy >= H) continue;
-      const size_t q = (size_t)qy * W + qx;
-      const float4 gq = gbuf[q];
-      if (gq.w < 0.0f) continue;
-      const float nd = fmax_(__fmaf_rn(g.z, gq.z, __fmaf_rn(g.y, gq.y, g.x * gq.x)), 0.0f);
-      const float n2 = nd * nd, n4 = n2 * n2, n8 = n4 * n4, n16 = n8 * n8, n32 = n16 * n16;
-      if (n32 == 0.0f) continue;
-      const float4 cq = load_px(src, srcF32, q);
-      const float wKernel = b3_weight(dx) * b3_weight(dy);
-      const float e = exp_nonpos_(-__fmaf_rn(fabsf(g.w - gq.w), invD, fabsf(lumC - luminance(cq.x, cq.y, cq.z)) * invS));
-      const float w = (wKernel * n32) * e;
-      sr = __fmaf_rn(cq.x, w, sr);
-      sg = __fmaf_rn(cq.y, w, sg);
-      sb = __fmaf_rn(cq.z, w, sb);
-      wSum = wSum + w;
-    }
-  }
-  const float den = fmax_(wSum, 1e-6f);
-  return make_float4(sr / den, sg / den, sb / den, center.w);
-}
 
 // present.wgsl:40-55 for one channel: v = illum * sqrtAlb^2 * exposure ->
 // ACES -> clamp -> pow(1/2.2) -> rgba8unorm code.

@@ -4,11 +4,14 @@
 
 namespace vrt {
 
-// Three iterations, against the form before (one pixel per thread, tiles staged
-// by TMA; odd widths unstaged): 1920x1080 297 -> 197 us, with normals off the
-// axes 300 -> 277; 1283x721 180 -> 104; 640x360 56 -> 43; 320x180, where the
-// taps' latency decides, 31 -> 32.  24 resident warps per SM (80 registers); 32
-// (64 registers, spilling) measure the same.  Issue slots 64% busy, FMA pipe
+// Three iterations back to back, against the form before (one pixel per thread,
+// tiles staged by TMA; odd widths unstaged): 1920x1080 260 -> 173 us, with
+// normals off the axes 260 -> 239; 641x361 60 -> 42.  Tiles that hold a negative, infinite or NaN
+// colour keep the sums of skipped taps by selects: with one such pixel in a
+// thousand 1920x1080 takes 183 (negative) to 196 us (NaN, infinite), 260 and 269 before, and
+// 177 with 30% of the colours -0.  (One thread per pixel
+// on the unstaged image for those tiles took 529 and 605.)  24 resident warps per SM (80 registers);
+// 32 (64 registers, spilling) measure the same.  Issue slots 64% busy, FMA pipe
 // 51% (a packed instruction holds it twice as long).
 //
 // Tiles of 32 rows read less halo; 16 rows make twice the blocks.  Measured at
