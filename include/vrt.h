@@ -104,8 +104,8 @@ enum {
 /* Launch-shape knobs of the wavefront path tracer; 0 keeps the default. */
 typedef struct VrtTuning {
   int refill_min;             /* idle lanes of a warp that trigger a refill    */
-  int trace_blocks_per_sm;    /* persistent DDA blocks (of 128 threads) per SM
-                                 (0 = max)                                     */
+  int trace_blocks_per_sm;    /* persistent DDA blocks per SM, counted as blocks
+                                 of 256 threads (0 = max)                      */
   int shade_blocks_per_sm;    /* shading kernel blocks per SM                  */
   int trace_variant;          /* tracer variant: (rounds of transitions per pass
                                  of the warp bookkeeping, DDA steps per round,

@@ -248,3 +248,22 @@ def test_ray_batches_of_several_threads(vrt, ctx):
         t.join()
     assert not wrong
     sc.close()
+
+
+def test_trace_blocks_count_256_threads(vrt, ctx):
+    """A tuning's tracer blocks are counted as blocks of 256 threads: one per SM already holds a warp for each of
+    8 rays per SM, so that twice as many change nothing (a warp that holds two rays walks fewer lane slots)."""
+    import torch
+    W, H = 8, torch.cuda.get_device_properties(0).multi_processor_count
+    vox, spawn = vrt.generate_scene(vrt.VRT_SCENE_FULL, 64, 3)
+    sc = vrt.Scene(ctx, vox, 64)
+    u = vrt.make_uniforms(vrt.camera_spline(spawn, 2), None, vrt.Lighting(), 5, 0, 0, W, H)
+    slots = []
+    for blocks in (1, 2):
+        s = vrt.Session(ctx, sc, W, H)
+        s.set_tuning(trace_blocks_per_sm=blocks, tail_wave=0)
+        s.frame(u)
+        slots.append(s.stats().trace_step_slots)
+        s.close()
+    assert slots[0] == slots[1] > 0
+    sc.close()

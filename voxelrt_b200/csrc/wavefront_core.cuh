@@ -1062,7 +1062,7 @@ template <class J, bool kWide, int kPhases, int kMinB, int kRun, bool kVarMaxT>
 cudaError_t wf_launch_trace(const J& jobs, int blocks_per_sm, int sms, const WfDev& b, int w, int implicit_n,
                             int refill, unsigned long long* stats, cudaStream_t st) {
   auto* fn = k_wf_trace<J, kWide, kPhases, kMinB, kRun, kVarMaxT>;
-  int per = blocks_per_sm;
+  int per = blocks_per_sm * (256 / kTraceThreads);   // the tuning counts blocks of 256 threads
   if (per <= 0) {
     cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, kTraceThreads, 0);
     if (e != cudaSuccess || per < 1) per = 1;
