@@ -1218,10 +1218,11 @@ int vrt_batch_set_tuning(VrtBatch* b, const VrtTuning* t) {
   return VRT_OK;
 }
 
+// Whether a graph captured with one serves the other (atrous_rows picks nothing).
 static bool same_tuning(const WavefrontTuning& a, const WavefrontTuning& c) {
   return a.refill_min == c.refill_min && a.trace_blocks_per_sm == c.trace_blocks_per_sm &&
          a.shade_blocks_per_sm == c.shade_blocks_per_sm && a.trace_variant == c.trace_variant &&
-         a.tail_wave == c.tail_wave && a.atrous_rows == c.atrous_rows;
+         a.tail_wave == c.tail_wave;
 }
 
 }  // extern "C"

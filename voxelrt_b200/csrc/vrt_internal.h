@@ -102,7 +102,7 @@ struct WavefrontTuning {
   int shade_blocks_per_sm = 32;
   int trace_variant = 0;        // shape of the tracer (wf_dispatch_trace): (transition rounds per
                                 // warp-bookkeeping pass, steps per round, min blocks/SM)
-  int atrous_rows = 0;          // kept from the caller's tuning; the a-trous tiles have one shape
+  int atrous_rows = 0;          // kept from the caller's tuning; the a-trous tiles go by the image's size
   int tail_wave = -1;           // first wave whose paths finish one thread each (k_wf_tail); 0 = never;
                                 // -1 = automatic (auto_tail in wavefront_core.cuh)
 };
