@@ -650,13 +650,13 @@ int vrt_session_autotune(VrtSession* s, const VrtUniforms* u, int frames, VrtTun
         if (med < win_ms) { win_ms = med; win = s->tune; }
       }
   s->tune = win;
-  // where the remaining paths finish one thread each: automatic, never, or
-  // from wave 2 / 3 (frames of more than one bounce)
+  // where the remaining paths finish in one launch: automatic, never, or from one of the waves that
+  // auto_tail picks from
   {
     const int nb = s->cache_on ? s->cache_cfg.train_bounces : (int)u->params0[1];
     float best_tail = 1e30f;
     int best_wave = win.tail_wave;
-    for (int tw : {-1, 0, 2, 3}) {
+    for (int tw : {-1, 0, 1, 2, 3, 4, 5}) {
       if (tw > 0 && tw >= nb + 2) continue;
       s->tune.tail_wave = tw;
       if (int r = vrt_pass_pathtrace(s, u)) { s->tune = keep; return r; }   // warm-up
@@ -1418,8 +1418,8 @@ int vrt_batch_autotune(VrtBatch* b, const VrtUniforms* u, int frames, VrtTuning*
         std::sort(ms.begin(), ms.end());
         if (ms[(size_t)frames / 2] < win_ms) { win_ms = ms[(size_t)frames / 2]; win = b->tune; }
       }
-  // where the remaining paths of the batch finish one thread each (0: never)
-  for (int tw : {2, 3, 4}) {
+  // where the remaining paths of the batch finish in one launch (0: never); tuned so far: automatic, or as set
+  for (int tw : {0, 1, 2, 3, 4, 5}) {
     b->tune = win;
     b->tune.tail_wave = tw;
     int r = vrt_batch_frame(b, u);
