@@ -153,7 +153,8 @@ typedef struct VrtFrameStats {
   float ms_cache;             /* cache inference + resolve + training steps    */
   float ms_reuse;             /* ReSTIR frames: reuse passes (inside
                                  ms_pathtrace, which covers all three)         */
-  uint64_t trace_step_slots;  /* wavefront tracer: lane slots of its DDA steps
+  uint64_t trace_step_slots;  /* wavefront tracer, and the launch that finishes
+                                 the remaining paths: lane slots of their DDA steps
                                  (32 x steps per pass x warp passes); the
                                  brick + voxel iterations over this is the
                                  tracer's SIMT (warp execution) efficiency     */

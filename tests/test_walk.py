@@ -267,3 +267,20 @@ def test_trace_blocks_count_256_threads(vrt, ctx):
         s.close()
     assert slots[0] == slots[1] > 0
     sc.close()
+
+
+# Lane step slots are counted wherever a path's rays are walked: no more iterations than slots, at every tail wave.
+@pytest.mark.parametrize("W,H,bounces", [(64, 41, 3), (401, 297, 2), (611, 331, 3)])
+def test_step_slots_cover_the_tail(vrt, ctx, W, H, bounces):
+    vox, spawn = vrt.generate_scene(vrt.VRT_SCENE_VOXELRT, 128, 7)
+    sc = vrt.Scene(ctx, vox, 128)
+    u = vrt.make_uniforms(vrt.camera_spline(spawn, 3), None, vrt.Lighting(), 9, bounces, 0, W, H)
+    for tail in (0, -1, 1, 2):
+        s = vrt.Session(ctx, sc, W, H)
+        s.set_tuning(tail_wave=tail)
+        s.frame(u)
+        st = s.stats()
+        steps = st.dda_outer + st.dda_inner
+        assert steps <= st.trace_step_slots <= 32 * 5 * steps, f"tail wave {tail}"
+        s.close()
+    sc.close()

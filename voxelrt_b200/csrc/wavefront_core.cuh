@@ -808,6 +808,7 @@ __global__ void __launch_bounds__(kShadeThreads, 1280 / kShadeThreads) k_wf_shad
 // against 305 us per 1080p cache frame: some lane shades in nearly every pass,
 // so the warp runs the shading code far more often than once per bounce.)
 constexpr int kTailPairLimit = 16;
+constexpr int kTailRun = 5;   // DDA steps between transitions
 template <class J, bool kWide>
 __global__ void __launch_bounds__(128, 5) k_wf_tail(J jobs, WfDev b, int wave, unsigned long long* stats) {
   frame_begin();
@@ -823,6 +824,7 @@ __global__ void __launch_bounds__(128, 5) k_wf_tail(J jobs, WfDev b, int wave, u
   const bool owner = !pair || (lane & 1) == 0;    // of the path's state; the other lane of a pair walks its shadow rays
   const int ray0 = pair && owner ? 1 : 0, ray1 = pair && !owner ? 1 : 2;   // this lane's rays: 0 shadow, 1 bounce
   DCount c{0u, 0u, 0u, 0u};
+  uint32_t passes = 0u;   // rounds of steps of this warp
   for (int base = 0; base < n; base += nwarps * per) {
     const int i = slot < per ? base + warp * per + slot : n;
     bool fin_train = false;
@@ -842,6 +844,7 @@ __global__ void __launch_bounds__(128, 5) k_wf_tail(J jobs, WfDev b, int wave, u
       F3 surf = f3(0.0f, 0.0f, 0.0f), rd = surf;
       bool lit = false;                            // the shadow ray met nothing
       Walk<kWide> d;
+      uint32_t rounds = 0u;                        // of steps, of this lane
       if (live) {
         flags = __float_as_uint(b.S2[g].w);
         surf = xyz(b.R0[g]);
@@ -853,13 +856,15 @@ __global__ void __launch_bounds__(128, 5) k_wf_tail(J jobs, WfDev b, int wave, u
           d.init(S, surf, rd, ray == 0 ? r.w : 1e4f);
           c.rays++;
           while (!d.done()) {
-            d.template walk_run<5>(S);
+            rounds++;
+            d.template walk_run<kTailRun>(S);
             if (!d.walking()) d.transition(S, rd, c);
           }
           d.finish(S, c);
           if (ray == 0) lit = !(d.tHit >= 0.0f);
         }
       }
+      passes += __reduce_max_sync(full, rounds);   // lanes step together, so the longest walk counts
       if (pair) lit = __shfl_xor_sync(full, (int)lit, 1) != 0;   // the owner's answer from its pair
       if (live && owner) {
         const float4 s0 = b.S0[g];
@@ -899,7 +904,10 @@ __global__ void __launch_bounds__(128, 5) k_wf_tail(J jobs, WfDev b, int wave, u
     }
     if (any_cache) cache_emit_samples(jobs.cache(j), fin_train, ti, rfin);
   }
-  if (stats) block_flush_stats(stats, c, 0u);   // kStatRays..kStatVReads
+  if (stats) {
+    block_flush_stats(stats, c, 0u);   // kStatRays..kStatVReads
+    block_flush_one(stats + kStatTraceSlots, lane == 0 ? passes * (uint32_t)(32 * kTailRun) : 0u);
+  }
 }
 
 // Zeroes the per-frame query and sample counters of every cache job.
