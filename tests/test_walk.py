@@ -284,3 +284,24 @@ def test_step_slots_cover_the_tail(vrt, ctx, W, H, bounces):
         assert steps <= st.trace_step_slots <= 32 * 5 * steps, f"tail wave {tail}"
         s.close()
     sc.close()
+
+
+# Batches on both sides of the lines between the walk and the nested loops, which depend on the world's size.
+@pytest.mark.parametrize("grid,n", [(32, 6_999), (32, 7_001), (32, 1_600_000), (32, 1_600_001), (64, 1_000_000), (64, 1_000_001),
+                                    (80, 320_000), (80, 320_001), (128, 0), (128, 1)])
+def test_ray_batch_lines_match_oracle(vrt, orc, ctx, grid, n):
+    import torch
+    if n < 2:     # at one wave of blocks, and past it
+        n += 1024 * torch.cuda.get_device_properties(0).multi_processor_count
+    vox, _ = vrt.generate_scene(vrt.VRT_SCENE_RANDOM, grid, 3)
+    b, m = orc.build_bricks(vox, grid)
+    sc = vrt.Scene(ctx, vox, grid)
+    o, d, t = _odd_rays(n, grid / 16.0, grid + n)
+    got, want = sc.trace_rays(o, d, t), orc.trace(vox, b, m, grid, o, d, t)
+    for f in ("t", "n"):            # as bits, any NaN equal to any other
+        x, y = got[f], want[f]
+        assert np.array_equal(np.isnan(x), np.isnan(y))
+        assert np.array_equal(x.view(np.uint32)[~np.isnan(x)], y.view(np.uint32)[~np.isnan(y)])
+    for f in ("mat", "voxel", "face", "steps", "bytes"):
+        assert np.array_equal(got[f], want[f]), f
+    sc.close()

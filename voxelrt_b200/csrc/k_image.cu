@@ -158,15 +158,11 @@ __global__ void __launch_bounds__(512) k_build_bricks(const uint32_t* __restrict
   if (threadIdx.x == 0) bricks[bi] = occ ? 1u : 0u;
 }
 
-// Occupancy bitmaps: bit bi of bits = bricks[bi] != 0, and the same over the
-// grid padded by one cell on each side, whose border bits are set (pad).
-__global__ void k_build_bits(const uint32_t* __restrict__ bricks, int BG, uint32_t* __restrict__ bits,
-                             uint32_t* __restrict__ pad) {
+// Occupancy bitmap over the brick grid padded by one cell on each side: a cell's bit is set where its brick's
+// word is not 0, and on the border.
+__global__ void k_build_bits(const uint32_t* __restrict__ bricks, int BG, uint32_t* __restrict__ pad) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int nb = BG * BG * BG, P = BG + 2, np = P * P * P;
-  const bool occ = i < nb && bricks[i] != 0u;
-  const uint32_t word = __ballot_sync(0xffffffffu, occ);
-  if ((threadIdx.x & 31) == 0 && i < ((nb + 31) & ~31)) bits[i >> 5] = word;
+  const int P = BG + 2, np = P * P * P;
   bool pocc = false;
   if (i < np) {
     const int x = i % P - 1, y = (i / P) % P - 1, z = i / (P * P) - 1;
@@ -200,7 +196,7 @@ cudaError_t launch_build_bricks(const SceneDev& s, int bx0, int by0, int bz0, in
 
 cudaError_t launch_build_bits(const SceneDev& s, cudaStream_t st) {
   const int np = (s.BG + 2) * (s.BG + 2) * (s.BG + 2);
-  k_build_bits<<<(np + 255) / 256, 256, 0, st>>>(s.bricks, s.BG, s.bits, s.cells);
+  k_build_bits<<<(np + 255) / 256, 256, 0, st>>>(s.bricks, s.BG, s.cells);
   return cudaGetLastError();
 }
 

@@ -1705,7 +1705,7 @@ static RestirDev restir_dev(const SceneDev& s, const VrtUniforms& u, float fclam
 template <typename K>
 static cudaError_t launch_occ_kernel(K kern_smem, K kern_glob, const SceneDev& s, int W, int H, const RestirDev& R,
                                      cudaStream_t st) {
-  const size_t smem = occ_words(s.BG) * sizeof(uint32_t);
+  const size_t smem = pad_words(s.BG) * sizeof(uint32_t);
   const dim3 grid((W + 15) / 16, (H + 15) / 16);
   if (smem <= kMaxSmemOccBytes) {
     if (smem > 48 * 1024) {

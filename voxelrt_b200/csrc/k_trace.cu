@@ -166,7 +166,8 @@ __global__ void __launch_bounds__(kRayThreads, 9) k_trace_rays(DScene S, const f
 
 // The same batch with one thread per ray on the nested loops.  A ray's walk is
 // latency there as here, but its lane never waits for the warp's transitions.
-__global__ void __launch_bounds__(256) k_trace_rays_nested(DScene S, const float* __restrict__ o,
+template <int kThreads>
+__global__ void __launch_bounds__(kThreads) k_trace_rays_nested(DScene S, const float* __restrict__ o,
                                                            const float* __restrict__ d,
                                                            const float* __restrict__ tmax, int n,
                                                            VrtHit* __restrict__ out) {
@@ -175,8 +176,8 @@ __global__ void __launch_bounds__(256) k_trace_rays_nested(DScene S, const float
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   DCount cnt{0u, 0u, 0u, 0u};
-  const F3 ro = f3(o[3 * (size_t)i], o[3 * (size_t)i + 1], o[3 * (size_t)i + 2]);
-  const F3 rd = f3(d[3 * (size_t)i], d[3 * (size_t)i + 1], d[3 * (size_t)i + 2]);
+  const F3 ro = f3(o[3 * i], o[3 * i + 1], o[3 * i + 2]);
+  const F3 rd = f3(d[3 * i], d[3 * i + 1], d[3 * i + 2]);
   const DHit h = trace<true>(S, occ, ro, rd, tmax[i], cnt);
   VrtHit r;
   r.t = h.t; r.n[0] = h.n.x; r.n[1] = h.n.y; r.n[2] = h.n.z; r.mat = h.mat;
@@ -190,7 +191,7 @@ __global__ void __launch_bounds__(256) k_trace_rays_nested(DScene S, const float
 
 cudaError_t launch_pathtrace(const SceneDev& s, const VrtUniforms& u, float fclamp, int W, int H,
                              const PathOut& out, cudaStream_t st) {
-  const size_t smem = occ_words(s.BG) * sizeof(uint32_t);
+  const size_t smem = pad_words(s.BG) * sizeof(uint32_t);
   dim3 grid((W + 15) / 16, (H + 15) / 16);
   if (smem <= kMaxSmemOccBytes) {
     if (smem > 48 * 1024) {
@@ -207,25 +208,35 @@ cudaError_t launch_pathtrace(const SceneDev& s, const VrtUniforms& u, float fcla
 cudaError_t launch_trace_rays(const SceneDev& s, const float* o, const float* d, const float* tmax, int n,
                               VrtHit* out, cudaStream_t st) {
   if (n <= 0) return cudaSuccess;
-  // Between the two, where one thread per ray about fills the GPU and the longest walk decides, the nested
-  // loops are faster: us per call, nested / walk, in worlds of 64^3, 128^3 and 256^3: 12 K rays 33 / 32, 38 / 34,
-  // 44 / 40; 20 K 32 / 34, 37 / 41, 45 / 45; 80 K 37 / 48, 41 / 44, 50 / 52; 120 K 44 / 45, 43 / 43, 59 / 56;
-  // 160 K 52 / 51, 52 / 47, 63 / 59.  Worlds of
-  // 8^3 bricks end a walk so soon that the line lies where the walk's refills begin (400 K rays 81 / 85).
-  const size_t smem = occ_words(s.BG) * sizeof(uint32_t);
-  if (n >= 14000 && n <= (s.BG <= 8 ? 500000 : 140000) && smem <= kMaxSmemOccBytes) {
+  // Where one thread per ray about fills the GPU and the longest walk decides, the nested loops are the safe
+  // choice: from some 14 K rays to one wave of their blocks (1024 rays an SM).  us per call, nested / walk, means of
+  // three worlds and two batches, in 80^3, 128^3 and 256^3 voxels: 12 K rays 24.9 / 21.3, 30.5 / 26.5, 37.3 / 31.4;
+  // 24 K 25.2 / 25.4, 32.4 / 30.4, 39.0 / 36.9 (single batches up to 0.83 of the nested loops' rate); 64 K
+  // 26.5 / 29.8, 33.6 / 34.9, 44.5 / 44.9; 130 K 33.3 / 36.2, 41.4 / 41.4, 54.8 / 55.1; 185 K 41.9 / 42.8, 51.5 / 47.0,
+  // 67.4 / 61.0.  Small worlds end a walk so soon that its refills and transitions pay only where its long runs
+  // begin: 32^3 at 5 K 14.2 / 12.9, 8 K 14.5 / 15.1, 800 K 75 / 91, 2 M 173 / 172; 64^3 at 800 K 107 / 110, 1.2 M
+  // 153 / 133; 80^3 at 270 K 51.4 / 51.4, 330 K 58.5 / 57.8.
+  const int sms = wf_sm_count(), wave = 1024 * sms;
+  const size_t smem = pad_words(s.BG) * sizeof(uint32_t);
+  const int nested_from = s.BG <= 4 ? 7000 : 14000;
+  const int nested_to = s.BG <= 4 ? 1600000 : (s.BG <= 8 ? 1000000 : (s.BG <= 10 ? 320000 : wave));
+  if (n >= nested_from && n <= nested_to && smem <= kMaxSmemOccBytes) {
+    // past one wave smaller blocks even the end out (800 K rays at 64^3: 110 -> 105 us); within it they lie
+    // unevenly on the SMs (145 K rays at 80^3: 34.5 -> 36.0)
+    const int threads = n <= wave ? 256 : 128;
+    auto* fn = threads == 256 ? k_trace_rays_nested<256> : k_trace_rays_nested<128>;
     if (smem > 48 * 1024) {
-      cudaError_t e = cudaFuncSetAttribute(k_trace_rays_nested, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (e != cudaSuccess) return e;
     }
-    k_trace_rays_nested<<<(unsigned)((n + 255) / 256), 256, smem, st>>>(to_dscene(s), o, d, tmax, n, out);
+    fn<<<(unsigned)((n + threads - 1) / threads), threads, smem, st>>>(to_dscene(s), o, d, tmax, n, out);
     return cudaGetLastError();
   }
   // Rays per warp.  Few rays are spread over all warps the GPU holds (9 blocks
-  // on each of 148 SMs), down to one per warp, since lanes on different paths
+  // on each SM), down to one per warp, since lanes on different paths
   // take turns; from 32 per warp on, one per lane until the rays fill the GPU
   // three times over, then longer runs with refills.
-  const int warps = kRayThreads / 32, resident = 148 * 9 * warps;
+  const int warps = kRayThreads / 32, resident = sms * 9 * warps;
   const int run = n <= 32 * resident ? (n + resident - 1) / resident
                                      : std::min(kRayMaxRun, std::max(32, n / (3 * resident) / 32 * 32));
   const unsigned blocks = (unsigned)(((long long)n + (long long)run * warps - 1) / ((long long)run * warps));

@@ -264,7 +264,7 @@ cudaError_t launch_vb_frame(const VbLaunch& L, cudaStream_t st) {
   D.horizon = make_float3(L.horizon[0], L.horizon[1], L.horizon[2]);
   D.rays = L.rays;
   const int P = L.W * L.H;
-  const size_t smem = occ_words(L.scene.BG) * sizeof(uint32_t);
+  const size_t smem = pad_words(L.scene.BG) * sizeof(uint32_t);
   if (smem <= kMaxSmemOccBytes) {
     if (smem > 48 * 1024) {
       cudaError_t e = cudaFuncSetAttribute(k_vb_paths<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

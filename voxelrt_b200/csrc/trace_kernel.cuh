@@ -7,16 +7,16 @@
 
 namespace vrt {
 
-// Largest occupancy bitmap staged in shared memory (512^3 grid = 32 KB).
-constexpr size_t kMaxSmemOccBytes = 64 * 1024;
+// Largest occupancy bitmap staged in shared memory (640^3 grid; a 512^3 grid's takes 36 KB).
+constexpr size_t kMaxSmemOccBytes = 68 * 1024;
 
-// Stage the 1-bit-per-brick occupancy bitmap in shared memory (kSmem) or use
+// Stage the padded grid's occupancy bitmap in shared memory (kSmem) or use
 // the global copy.  Every thread of the block must call it.
 template <bool kSmem>
 VRT_DI const uint32_t* stage_occupancy(const DScene& S, uint32_t* s_occ) {
-  if (!kSmem) return S.bits;
-  const int nwords = (S.BG * S.BG * S.BG + 31) >> 5;
-  for (int i = threadIdx.x; i < nwords; i += blockDim.x) s_occ[i] = __ldg(S.bits + i);
+  if (!kSmem) return S.cells;
+  const int P = S.BG + 2, nwords = (P * P * P + 31) >> 5;
+  for (int i = threadIdx.x; i < nwords; i += blockDim.x) s_occ[i] = __ldg(S.cells + i);
   __syncthreads();
   return s_occ;
 }
@@ -24,7 +24,7 @@ VRT_DI const uint32_t* stage_occupancy(const DScene& S, uint32_t* s_occ) {
 
 inline DScene to_dscene(const SceneDev& s) {
   DScene d;
-  d.vox = s.vox; d.cells = s.cells; d.bits = s.bits; d.N = s.N; d.BG = s.BG;
+  d.vox = s.vox; d.cells = s.cells; d.N = s.N; d.BG = s.BG;
   d.rP = recip_pad(s.BG); d.rP2 = recip_pad2(s.BG);
   d.mw = (uint32_t)mask_word(s.BG); d.pad = 0u;
   return d;

@@ -269,7 +269,6 @@ static int scene_alloc(VrtCtx* ctx, int N, VrtScene** out) {
   int r = dev_alloc(ctx, (void**)&s->dev.vox, nv * 4, &s->bytes);
   if (!r) r = dev_alloc(ctx, (void**)&s->dev.bricks, nb * 4, &s->bytes);
   if (!r) r = dev_alloc(ctx, (void**)&s->dev.cells, cell_bytes(s->dev.BG), &s->bytes);
-  if (!r) r = dev_alloc(ctx, (void**)&s->dev.bits, occ_words(s->dev.BG) * 4 + 128, &s->bytes);
   if (r) {
     std::string keep = g_err;
     vrt_scene_destroy(s);
@@ -379,7 +378,6 @@ int vrt_scene_destroy(VrtScene* s) {
   dev_free(c, s->dev.vox, N * N * N * 4, &s->bytes);
   dev_free(c, s->dev.bricks, nb * 4, &s->bytes);
   dev_free(c, s->dev.cells, cell_bytes(s->dev.BG), &s->bytes);
-  dev_free(c, s->dev.bits, occ_words(s->dev.BG) * 4 + 128, &s->bytes);
   const size_t cap = s->light_cap;
   dev_free(c, s->light_words, cap * 8, &s->bytes);
   dev_free(c, s->light_w, cap * 8, &s->bytes);
@@ -1273,7 +1271,7 @@ static int batch_frame_impl(VrtBatch* b, const int* idx, int m, const VrtUniform
     const int p = parity_of(s);
     j.u = u[i];
     sun_frame(j.u.sunDir, j.sunT, j.sunB);
-    j.vox = s->scene->dev.vox; j.cells = s->scene->dev.cells; j.bits = s->scene->dev.bits;
+    j.vox = s->scene->dev.vox; j.cells = s->scene->dev.cells;
     j.N = s->scene->dev.N; j.BG = s->scene->dev.BG;
     j.rP = recip_pad(j.BG); j.rP2 = recip_pad2(j.BG);
     j.mw = (uint32_t)mask_word(j.BG);

@@ -369,7 +369,6 @@ struct DScene {
   // 1 bit per cell (border cells: set), then from word mw on 16 mask words per
   // cell (border cells: full).
   const uint32_t* __restrict__ cells;
-  const uint32_t* __restrict__ bits;    // 1 bit per brick: bricks[bi] != 0
   int N, BG;
   uint32_t rP, rP2;                     // 2^32 / P and 2^32 / P^2 rounded up (dda_walk.cuh)
   uint32_t mw, pad;
@@ -425,10 +424,10 @@ VRT_DI void block_flush_one(unsigned long long* dst, uint32_t v) {
   }
 }
 
-// Brick occupancy bit of brick bi from the bitmap `occ` (shared memory when
-// the kernel staged it, global otherwise).
-VRT_DI bool brick_occupied(const uint32_t* occ, uint32_t bi) {
-  return (occ[bi >> 5] >> (bi & 31u)) & 1u;
+// Occupancy bit of cell ci of the padded brick grid from the bitmap `occ` (shared
+// memory when the kernel staged it, global otherwise).
+VRT_DI bool brick_occupied(const uint32_t* occ, uint32_t ci) {
+  return (occ[ci >> 5] >> (ci & 31u)) & 1u;
 }
 
 // One component of hit.n = -vmask * vec3<f32>(stepDir) (voxel.wgsl:126) with
@@ -443,7 +442,7 @@ VRT_DI float face_normal_component(bool on_axis, int s) {
 
 // trace(): the reference's two-level Amanatides-Woo walk.  Outer loop over
 // 8^3 bricks (at most 3*BGRID+2 steps), inner per-voxel loop (at most 24
-// steps) inside occupied bricks; brick occupancy comes from a 1-bit-per-brick
+// steps) inside occupied bricks; brick occupancy comes from the padded grid's
 // bitmap, voxel occupancy from the 16-word brick mask (read-only path), and
 // the packed voxel is read on a hit.  Counters track iterations entered.
 template <bool kCount>
@@ -489,15 +488,17 @@ VRT_DI DHit trace(const DScene& S, const uint32_t* occ, F3 roW, F3 rd, float max
   const F3 tDeltaB = absInv * 8.0f;
   F3 tMaxB = ((f3((float)bx, (float)by, (float)bz) + stepGE) * 8.0f - ro) * invRd;
 
-  const int P = BG + 2;                                       // the padded grid's side
-  const uint32_t* __restrict__ mask0 = S.cells + (S.mw + 16u * (uint32_t)(1 + P + P * P));   // brick (0, 0, 0)
+  // from here on in cells of the padded grid, where bricks lie at 1 .. BG
+  bx++; by++; bz++;
+  const uint32_t P = (uint32_t)BG + 2u;
+  const uint32_t* __restrict__ masks = S.cells + S.mw;
   const int outerMax = 3 * BG + 2;
   for (int iter = 0; iter < outerMax; iter++) {
     if (t > tExit) break;
     if (kCount) cnt.outer++;
-    const uint32_t bi = (uint32_t)bx + (uint32_t)by * (uint32_t)BG + (uint32_t)bz * (uint32_t)(BG * BG);
-    if (brick_occupied(occ, bi)) {
-      const int mnx = bx * kBrick, mny = by * kBrick, mnz = bz * kBrick;
+    const uint32_t ci = (uint32_t)bx + (uint32_t)by * P + (uint32_t)bz * (P * P);
+    if (brick_occupied(occ, ci)) {
+      const int mnx = bx * kBrick - kBrick, mny = by * kBrick - kBrick, mnz = bz * kBrick - kBrick;
       const F3 p = ro + rd * (t + 1e-4f);
       int vx = iclamp_(ifloor_(p.x), mnx, mnx + 7);
       int vy = iclamp_(ifloor_(p.y), mny, mny + 7);
@@ -505,7 +506,7 @@ VRT_DI DHit trace(const DScene& S, const uint32_t* occ, F3 roW, F3 rd, float max
       F3 tMaxV = ((f3((float)vx, (float)vy, (float)vz) + stepGE) - ro) * invRd;
       float tCur = t;
       int vax = ax;
-      const uint32_t* __restrict__ bm = mask0 + (uint32_t)(bx + P * (by + P * bz)) * 16u;
+      const uint32_t* __restrict__ bm = masks + (size_t)ci * 16u;
       for (int j = 0; j < 3 * kBrick; j++) {
         if (kCount) cnt.inner++;
         const uint32_t bit = (uint32_t)((vx - mnx) + (vy - mny) * 8 + (vz - mnz) * 64);
@@ -539,7 +540,7 @@ VRT_DI DHit trace(const DScene& S, const uint32_t* occ, F3 roW, F3 rd, float max
     } else {
       t = tMaxB.z; tMaxB.z = tMaxB.z + tDeltaB.z; bz += sz; ax = 2;
     }
-    if (bx < 0 || by < 0 || bz < 0 || bx >= BG || by >= BG || bz >= BG) break;
+    if (bx < 1 || by < 1 || bz < 1 || bx > BG || by > BG || bz > BG) break;
   }
   return hit;
 }

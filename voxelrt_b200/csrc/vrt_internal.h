@@ -12,17 +12,23 @@ namespace vrt {
 void sun_frame(const float w[4], float tang[4], float bitan[4]);
 
 // Device-resident scene: packed voxels, per-brick words and masks, plus the
-// 1-bit-per-brick occupancy bitmap the per-thread traversal stages in shared
-// memory and the padded one the queue tracer walks (dda_walk.cuh).
+// occupancy bitmap that the per-thread traversal stages in shared memory and the
+// queue tracer walks (dda_walk.cuh), over the padded brick grid like the masks.
 struct SceneDev {
   uint32_t* vox = nullptr;     // N^3
   uint32_t* bricks = nullptr;  // BG^3
   uint32_t* cells = nullptr;   // the padded bitmap and, from word mask_word(BG) on, the padded masks
-  uint32_t* bits = nullptr;    // ceil(BG^3 / 32)
   int N = 0, BG = 0;
 };
 
-inline size_t occ_words(int BG) { return ((size_t)BG * BG * BG + 31) / 32; }
+// Multiprocessors of the current device.
+inline int wf_sm_count() {
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms > 0 ? sms : 1;
+}
+
 // Largest brick grid side of the queue tracer's narrow form (dda_walk.cuh).
 constexpr int kNarrowBG = 128;
 // Words of the padded bitmap: one bit per cell of the (BG + 2)^3 grid, a border of one cell on
@@ -114,7 +120,6 @@ struct JobHost {
   float sunT[4], sunB[4];   // sun_frame(u.sunDir)
   const uint32_t* vox;
   const uint32_t* cells;
-  const uint32_t* bits;
   int N, BG;
   uint32_t rP, rP2;         // recip_pad(BG), recip_pad2(BG)
   uint32_t mw, spad;        // mask_word(BG)
@@ -256,7 +261,7 @@ cudaError_t launch_wavefront(const SceneDev& s, const VrtUniforms& u, float fcla
 
 cudaError_t launch_build_bricks(const SceneDev& s, int bx0, int by0, int bz0, int bx1, int by1, int bz1,
                                 cudaStream_t st);
-// Both occupancy bitmaps (plain and padded) from the brick words.
+// The padded occupancy bitmap from the brick words.
 cudaError_t launch_build_bits(const SceneDev& s, cudaStream_t st);
 cudaError_t launch_fill_box(const SceneDev& s, int x0, int y0, int z0, int x1, int y1, int z1, uint32_t value,
                             cudaStream_t st);

@@ -979,13 +979,6 @@ inline WfDev wf_view(const WavefrontBufs& w) {
   return d;
 }
 
-inline int wf_sm_count() {
-  int dev = 0, sms = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  return sms > 0 ? sms : 1;
-}
-
 // ---------------------------------------------------------------------------
 // host: post-wave cache work of one job -- inference over its queries, the
 // resolve of its cache-terminated paths, then its training steps.  Every
