@@ -305,3 +305,28 @@ def test_ray_batch_lines_match_oracle(vrt, orc, ctx, grid, n):
     for f in ("mat", "voxel", "face", "steps", "bytes"):
         assert np.array_equal(got[f], want[f]), f
     sc.close()
+
+
+@pytest.mark.parametrize("variant", range(9))
+def test_tracer_variants_leave_the_image(vrt, ctx, variant):
+    """Every shape of the tracer that a tuning can name, for a session and for a batch, against the megakernel."""
+    W, H = 160, 90
+    vox, spawn = vrt.generate_scene(vrt.VRT_SCENE_FULL, 128, 2)
+    sc = vrt.Scene(ctx, vox, 128)
+    u = vrt.make_uniforms(vrt.camera_spline(spawn, 4), None, vrt.Lighting(), 9, 4, 0, W, H)
+    mega = vrt.Session(ctx, sc, W, H, keep_radiance_f32=True, path_kernel="megakernel")
+    wave = vrt.Session(ctx, sc, W, H, keep_radiance_f32=True)
+    view = vrt.Session(ctx, sc, W, H, keep_radiance_f32=True, path_kernel="batch_only")
+    batch = vrt.Batch(ctx, [view])
+    for t in (wave, batch):
+        t.set_tuning(trace_variant=variant, tail_wave=0)
+    mega.frame(u)
+    wave.frame(u)
+    batch.frame([u])
+    a = mega.stats()
+    for s, st in ((wave, wave.stats()), (view, batch.stats())):
+        assert s.radiance_f32().tobytes() == mega.radiance_f32().tobytes()
+        assert (st.rays, st.dda_outer, st.dda_inner, st.voxel_reads) == (a.rays, a.dda_outer, a.dda_inner, a.voxel_reads)
+    batch.close()
+    for o in (mega, wave, view, sc):
+        o.close()

@@ -159,3 +159,30 @@ def test_noalloc_odd_values(vrt, orc, W, H, share, value):
         nan = np.isnan(want.view(np.float16))
         assert np.array_equal(nan, np.isnan(got.view(np.float16)))
         assert np.array_equal(got[~nan], want[~nan])
+
+
+# The same rows of one image on both sides of the line between tiles of 16 and of 32 rows (two waves of the taller, three
+# on a multiprocessor): cut off below the rows that reach the cut within the three steps, both give the same pixels.
+@pytest.mark.parametrize("acc_f32", [False, True])
+def test_noalloc_tile_heights_agree(vrt, acc_f32):
+    import torch
+    from voxelrt_b200._lib import lib
+
+    line = 6 * torch.cuda.get_device_properties(0).multi_processor_count
+    W = 1184
+    H = -(-line // (W // 32)) * 32                       # the first height with `line` tiles of 32 x 32
+    r = np.random.default_rng(5)
+    gb = np.zeros((H, W, 4), np.float32)
+    np.put_along_axis(gb, r.integers(0, 3, (H // 8, W // 8, 1)).repeat(8, 0).repeat(8, 1), 1.0, axis=2)
+    gb[..., 3] = np.where(r.random((H, W)) < 0.1, -1.0, 2.0 + 0.1 * r.random((H, W)))
+    acc = np.zeros((H, W, 4), np.float32)
+    acc[..., :3] = np.exp(r.normal(size=(H, W, 3)))
+    acc[..., 3] = r.integers(0, 65, (H, W))
+    src = acc if acc_f32 else acc.astype(np.float16).view(np.uint16)
+    out = []
+    for h in (H, H - 32):
+        got, _, _ = _run_noalloc(lib, torch, torch.device("cuda:0"), np.ascontiguousarray(src[:h]), acc_f32,
+                                 np.ascontiguousarray(gb[:h]), W, h)
+        out.append(got.reshape(h, W, 4))
+    keep = H - 32 - 2 * (1 + 2 + 4)
+    assert np.array_equal(out[0][:keep], out[1][:keep])

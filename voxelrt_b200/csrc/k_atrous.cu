@@ -17,7 +17,7 @@ namespace vrt {
 // Tiles of 32 rows read less halo; 16 rows make twice the blocks.  Measured at
 // 16 / 32 rows: 320x180 32 / 33 us, 800x450 52 / 56, 960x540 69 / 68, 1283x721
 // 104 / 107, 1920x1080 201 / 197: the line is at two full waves of 32-row tiles
-// (3 on each of 148 SMs).  8 rows: no better at any size.
+// (3 on each SM).  8 rows: no better at any size.
 template <int S, int R, bool kSrcF32>
 __global__ void __launch_bounds__(8 * R, 96 / R) k_atrous(int W, int H, const void* src, const float4* gbuf,
                                                           uint2* __restrict__ dst) {
@@ -40,7 +40,7 @@ static cudaError_t run_tiles(int W, int H, const void* src, const void* gbuf, vo
 template <int S, bool kSrcF32>
 static cudaError_t run(int W, int H, const void* src, const void* gbuf, void* dst, cudaStream_t st) {
   const long tiles = (long)((W + 31) / 32) * ((H + 31) / 32);
-  return tiles < 888 ? run_tiles<S, 16, kSrcF32>(W, H, src, gbuf, dst, st)
+  return tiles < 6 * wf_sm_count() ? run_tiles<S, 16, kSrcF32>(W, H, src, gbuf, dst, st)
                      : run_tiles<S, 32, kSrcF32>(W, H, src, gbuf, dst, st);
 }
 
