@@ -113,14 +113,16 @@ typedef struct VrtTuning {
                                  1: (4,4,9), 2: (3,4,8), 3: (4,3,9), 4: (2,4,9),
                                  5: (8,1,9), 6: (4,3,10), 7: (3,6,9), 8: (3,6,8) */
   int atrous_tile_rows;       /* 0, 8 or 16: accepted and returned; the a-trous
-                                 pass picks its tiles by the image's size      */
+                                 pass picks its tiles by the image's size (a
+                                 batch always takes 32 rows)                   */
   int tail_wave;              /* first wave whose remaining paths each finish on
                                  a thread or two of one launch, not in launches
                                  per wave; 0 = never, -1 = automatic
                                  (wave 2 for a cache-assisted session, or for a
                                  batch whose every job is cache-assisted; else by
-                                 pixels and bounces); the image is the same either
-                                 way                                           */
+                                 pixels and bounces); in a frame with the radiance
+                                 cache a wave of 1 counts as 2; the image is the
+                                 same either way                               */
 } VrtTuning;
 
 /* One traced ray (vrt_trace_rays).  face: 0..5 = +x,-x,+y,-y,+z,-z normal,

@@ -2,8 +2,9 @@
 //
 // A batch frame renders one frame for each of n sessions (different scenes,
 // sizes, bounce counts, cameras).  The sessions' pixels are laid out back to
-// back in one global index space; every kernel finds the job of a pixel by a
-// binary search over the jobs' first pixels.  The wavefront path tracer runs
+// back in one global index space; a warp of consecutive pixels finds its job
+// with one load per 32 jobs over the jobs' first pixels, a path from a list by a
+// binary search over them.  The wavefront path tracer runs
 // over all jobs at once -- one persistent trace launch per wave serves rays
 // of every scene -- followed by one temporal, three a-trous and one present
 // launch over all jobs.  Per-pixel arithmetic is the single-session code
@@ -41,8 +42,9 @@ __global__ void __launch_bounds__(256) k_b_temporal(MultiJob J, uint32_t P) {
 
 // atrous.wgsl:26-83 iteration `it` (step 1 << it) of every job whose denoise
 // flag is set; chain accum -> dA -> dB -> dA (main.js:503-507).  A CTA computes
-// one 32 x 32 tile of one job (atrous_tile.cuh).  tiles: m + 1 prefix counts of
-// the jobs' tiles, in which CTA b finds its job.
+// one 32 x 32 tile of one job (atrous_tile.cuh), whatever the views' sizes: the
+// jobs' tiles fill the GPU together, as those of one large image.  tiles: m + 1
+// prefix counts of the jobs' tiles, in which CTA b finds its job.
 constexpr int kBatchRows = 32;   // tile rows
 template <int S>
 __global__ void __launch_bounds__(8 * kBatchRows, 96 / kBatchRows) k_b_atrous(MultiJob J,

@@ -600,7 +600,8 @@ __global__ void __launch_bounds__(256, 2) k_mlp_infer(const __grid_constant__ Ml
 // Bound by the chain of eight tensor-core phases per 256 samples, two warps per
 // scheduler; taking the ReLU's derivative from the stored activations instead
 // of building 192 mask bits per sample cut the instructions 5.3 -> 3.8 M and
-// the time 28.7 -> 25.7 us for 65,536 samples (983 K: a call 312 -> 271 us).
+// the time 28.7 -> 25.7 us for 65,536 samples (983 K: a call 312 -> 271 us);
+// storing them so that every positive one stays positive (store_row_hidden) costs 0.4 M and half a us.
 __global__ void __launch_bounds__(256, 1) k_mlp_grad(const __grid_constant__ MlpTaskSet ts) {
   frame_begin();
   using namespace mlp;

@@ -416,8 +416,8 @@ int vrt_trace_rays(VrtScene* s, const float* o, const float* d, const float* tma
   cudaStream_t st = s->ctx->stream;
   const size_t bo = (size_t)n * 12, bt = (size_t)n * 4, bh = (size_t)n * sizeof(VrtHit);
   // Small batches through pinned memory that the kernel reads and writes itself: one launch and one
-  // wait, where an allocation and four copies took most of the call (64 rays 61 -> 32 us, 5000 rays
-  // 132 -> 72, 16384 rays 239 -> 195).  Past kRayStage the copies themselves decide.  Device pointers,
+  // wait, where an allocation and four copies took most of the call (1 ray 36 -> 25 us, 64 rays 48 -> 32, 1000
+  // 73 -> 51, 5000 127 -> 88, 16384 249 -> 154).  Past kRayStage the copies themselves decide.  Device pointers,
   // which are none of this entry's, are left to the copies to refuse; and a call that finds the staging
   // taken by another thread's copies through memory of its own.
   VrtCtx* c = s->ctx;
@@ -1148,8 +1148,9 @@ static int batch_create_capacity(VrtCtx* ctx, VrtSession* const* sessions, int n
   if (int r = set_dev(ctx)) return r;
   VrtBatch* b = new VrtBatch();
   b->ctx = ctx;
-  // batch default launch shape: the tracer variant that holds its walk in registers for the batch's
-  // job lookups (6 steps per pass, 4 blocks per SM; the 8 x 5 shape spills there), refill at 16 idle lanes
+  // batch default launch shape: the tracer variant with 64 registers, which spills least with the batch's job
+  // lookups beside the walk (3 rounds of 4 steps, 8 blocks per SM: 1.418 ms for sixteen 480x270 views, the
+  // other variants 1.423 to 1.72), refill at 16 idle lanes
   b->tune.trace_variant = 2;
   b->tune.refill_min = 16;
   if (sessions) b->sessions.assign(sessions, sessions + n);

@@ -387,7 +387,7 @@ struct DCount {
 
 // Block-reduced traversal counters: stats[0..4] += rays, brick iterations,
 // voxel iterations, voxel reads, pixels of the block (the frame counters'
-// first five slots); one atomic per counter per block of 256 threads, since
+// first five slots); one atomic per counter per block, since
 // every block adds to the same counters.  All threads of the block call it.
 VRT_DI void block_flush_stats(unsigned long long* stats, const DCount& c, uint32_t pix) {
   __shared__ uint32_t s_part[8][5];

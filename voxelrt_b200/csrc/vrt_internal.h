@@ -47,7 +47,7 @@ inline uint32_t recip_pad2(int BG) { return recip_up((uint32_t)(BG + 2) * (uint3
 // Per-frame counters written by the path kernel (u64 each).
 enum StatSlot {
   kStatRays = 0, kStatOuter, kStatInner, kStatVReads, kStatPixels, kStatCacheQueries, kStatCacheSamples,
-  kStatTraceSlots,   // lane step slots of the queue tracer: 32 x steps per pass x passes, per warp
+  kStatTraceSlots,   // lane step slots of the tracer and of the tail: 32 x steps per pass x passes, per warp
   kStatCount = 8
 };
 static_assert(kStatRays == 0 && kStatOuter == 1 && kStatInner == 2 && kStatVReads == 3 && kStatPixels == 4,

@@ -403,7 +403,7 @@ VRT_DI bool shade_vertex(const Uni& u, const WfDev& b, uint32_t g, uint32_t k, F
   return want_shadow || want_bounce;
 }
 
-// Block-aggregated appends: each thread of a block of 256 adds nf entries to
+// Block-aggregated appends: each thread of a block of up to 256 adds nf entries to
 // the list counted by c_front, nb to the list counted by c_back and, if act,
 // one to the list counted by c_act; one atomicAdd per counter per block, since
 // every block of the grid appends to the same counters.  Returns the thread's
@@ -1080,7 +1080,8 @@ cudaError_t wf_launch_trace(const J& jobs, int blocks_per_sm, int sms, const WfD
 // of 128 threads and 56 registers per SM, refill at 12 idle lanes): 1 step
 // 1.251 ms, 3 0.987, 4 0.955, 5 0.949, 6 0.952.  8 blocks (64 registers, no
 // spills) 0.971 at 4 steps; 10 (48 registers, spilling) 1.05 at 3.  Refill at 8
-// / 10 / 12 / 14 idle lanes: 0.959 / 0.950 / 0.949 / 0.953.  Fetching the next
+// / 10 / 12 / 14 idle lanes: 0.959 / 0.950 / 0.949 / 0.953 (later, from another
+// view: 1.004 / 0.994 / 0.994 / 0.995, 16: 1.002).  Fetching the next
 // cell's word before the checks that may end a level's walk: 0.990 against
 // 0.971 (it costs a register that spills).
 template <class J, bool kVarMaxT = false>
@@ -1142,9 +1143,8 @@ cudaError_t wf_run_waves(const J& jobs, uint32_t P, int waves, const WavefrontBu
     if (tm && (e = cudaEventRecord(trace_ev[2 * w], st)) != cudaSuccess) return e;
     const int impl = w == 0 ? (int)P : 0;
     const int tb = tune.trace_blocks_per_sm;
-    // the coherent primary rays refill later: the 1080p primary wave took 299 / 290 / 285 / 277 / 271 us at
-    // 8 / 12 / 16 / 24 / 32 idle lanes (32: only whole warps refill), while the later waves are fastest at 8
-    // (490 / 426 / 143 us against 530 / 479 / 153 at 24)
+    // the coherent primary rays refill later, in whole warps: the four waves of a 1080p frame trace in 1.008 /
+    // 1.003 / 0.998 / 0.994 ms with the primary wave's refill at 12 / 16 / 24 / 32 idle lanes, the others' at 12
     const int rf = w == 0 ? std::max(refill, kPrimaryRefill) : refill;
     e = wf_dispatch_trace<J, kVarMaxT>(tune.trace_variant, jobs, tb, sms, b, w, impl, rf, stats, st);
     if (e != cudaSuccess) return e;
