@@ -113,8 +113,7 @@ typedef struct VrtTuning {
                                  1: (4,4,9), 2: (3,4,8), 3: (4,3,9), 4: (2,4,9),
                                  5: (8,1,9), 6: (4,3,10), 7: (3,6,9), 8: (3,6,8) */
   int atrous_tile_rows;       /* 0, 8 or 16: accepted and returned; the a-trous
-                                 pass picks its tiles by the image's size (a
-                                 batch always takes 32 rows)                   */
+                                 pass has tiles of one shape                   */
   int tail_wave;              /* first wave whose remaining paths each finish on
                                  a thread or two of one launch, not in launches
                                  per wave; 0 = never, -1 = automatic

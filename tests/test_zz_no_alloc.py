@@ -161,8 +161,7 @@ def test_noalloc_odd_values(vrt, orc, W, H, share, value):
         assert np.array_equal(got[~nan], want[~nan])
 
 
-# The same rows of one image on both sides of the line between tiles of 16 and of 32 rows (two waves of the taller, three
-# on a multiprocessor): cut off below the rows that reach the cut within the three steps, both give the same pixels.
+# The same rows of one image at two heights: above the rows that reach the cut within the three steps, the same pixels.
 @pytest.mark.parametrize("acc_f32", [False, True])
 def test_noalloc_tile_heights_agree(vrt, acc_f32):
     import torch
@@ -170,7 +169,7 @@ def test_noalloc_tile_heights_agree(vrt, acc_f32):
 
     line = 6 * torch.cuda.get_device_properties(0).multi_processor_count
     W = 1184
-    H = -(-line // (W // 32)) * 32                       # the first height with `line` tiles of 32 x 32
+    H = -(-line // (W // 32)) * 32
     r = np.random.default_rng(5)
     gb = np.zeros((H, W, 4), np.float32)
     np.put_along_axis(gb, r.integers(0, 3, (H // 8, W // 8, 1)).repeat(8, 0).repeat(8, 1), 1.0, axis=2)

@@ -1,5 +1,5 @@
 // atrous_tile.cuh -- one a-trous iteration (atrous.wgsl:26-83) over a tile of
-// 32 x R output pixels (R = 32, or 16 for small images), shared by the single-image kernel (k_atrous.cu) and
+// 32 x 16 output pixels, shared by the single-image kernel (k_atrous.cu) and
 // the batched one (k_batch.cu): 5x5 B3-spline taps at the step, weights
 // normal^32 * exp(-(|dt| / (0.05 t + 0.01) + |dL| / sigmaL)),
 // sigmaL = max(0.08, 2/sqrt(max(history,1))); sky, out-of-image taps and taps of
@@ -14,13 +14,14 @@
 //    per pair, so that a tap of both pixels is a few loads straight into
 //    register pairs.  Taps at odd distances (step 1 only) take halves of two
 //    neighbouring pairs.
-//  * A thread of 8 R computes two pairs, `step` rows apart, whose taps share four
-//    rows of five: 30 tap loads per pair where one pair alone takes 50.
+//  * Each of the 256 threads computes one pair.  (Two pairs, `step` rows apart,
+//    whose taps share four rows of five, take 30 tap loads per pair instead of 50, but half
+//    the threads stage the tile and walk the taps: three iterations 27 against 15.6 us at 128x72,
+//    28.4 / 20.7 at 320x180, 51 / 38 at 800x450, 172.4 / 172.1 at 1920x1080.)
 //  * Normals along an axis (every G-buffer of a voxel world) are staged as one
 //    code: the power of the dot product is then exactly 1 for equal codes and
 //    0 otherwise, a compare and a select instead of ten multiplications.  A
-//    tile with any other normal is computed as two halves with the normals
-//    staged in full (one pair per thread).
+//    tile with any other normal is staged again with the normals in full.
 //  * No branches per tap: a tap that the definition skips (outside the image,
 //    sky, a zero normal weight) adds a product with a weight of 0.  That
 //    changes no bit while every staged colour is finite and not negative (nor
@@ -37,19 +38,16 @@
 
 namespace vrt {
 
-constexpr int kAtrousTile = 32;   // tile width
+constexpr int kAtrousW = 32, kAtrousH = 16;               // a tile
+constexpr int kAtrousThreads = kAtrousW * kAtrousH / 2;   // a pair each
+constexpr int kAtrousBlocks = 3;                          // an SM
 
-template <int S, int R>
+template <int S>
 struct AtrousGeom {
-  static constexpr int threads = 8 * R;
-  static constexpr int HX = 2 * S;                        // halo
-  static constexpr int EW = (kAtrousTile + 2 * HX) / 2;   // pairs per row
-  static constexpr int EH = R + 2 * HX;
-  static constexpr int NE = EW * EH;
-  static constexpr int HH = R / 2 + 2 * HX;               // rows of a half tile
-  static constexpr int HE = EW * HH;
-  // a tile, or a half tile with full normals; 30 / 38 / 54 KB at steps 1 / 2 / 4 with 32 rows
-  static constexpr int smem = NE * 48 > HE * 64 ? NE * 48 : HE * 64;
+  static constexpr int HX = 2 * S;                     // halo
+  static constexpr int EW = (kAtrousW + 2 * HX) / 2;   // pairs per row
+  static constexpr int NE = EW * (kAtrousH + 2 * HX);
+  static constexpr int smem = NE * 64;                 // with the normals in full; 23 / 30 / 48 KB at steps 1 / 2 / 4
 };
 
 VRT_DI float2 f2(float x, float y) { return make_float2(x, y); }
@@ -158,15 +156,14 @@ struct AtrousImage {
 
 enum : int { kTileOdd = 1, kTileFullNormals = 2 };   // what staged values ask for
 
-// Stages rows [0, rows) of the tile at (x0, y0) (the halo's corner); returns
-// kTile flags.
-template <int S, int R, bool kUnit>
-VRT_DI int stage_tile(float4* sm, const AtrousImage& I, int x0, int y0, int rows) {
-  using G = AtrousGeom<S, R>;
-  const int ne = G::EW * rows;
+// Stages the tile at (x0, y0) (the halo's corner); returns kTile flags.
+template <int S, bool kUnit>
+VRT_DI int stage_tile(float4* sm, const AtrousImage& I, int x0, int y0) {
+  using G = AtrousGeom<S>;
+  constexpr int ne = G::NE;
   int flags = 0;
 #pragma unroll 2
-  for (int e = threadIdx.x; e < ne; e += G::threads) {
+  for (int e = threadIdx.x; e < ne; e += kAtrousThreads) {
     const int qy = y0 + e / G::EW, qx = x0 + 2 * (e % G::EW);
     float4 g[2], c[2];
 #pragma unroll
@@ -209,41 +206,27 @@ VRT_DI int stage_tile(float4* sm, const AtrousImage& I, int x0, int y0, int rows
   return flags;
 }
 
-// The alpha (history length) of kPairs pairs: pixels px, px + 1 of rows y + q S;
-// 1 outside the image.
-template <int S, int kPairs>
-VRT_DI void load_alpha(const AtrousImage& I, int px, int y, float (&alpha)[kPairs][2]) {
-#pragma unroll
-  for (int q = 0; q < kPairs; q++)
-#pragma unroll
-    for (int k = 0; k < 2; k++)
-      alpha[q][k] = px + k < I.W && y + q * S < I.H ? load_px(I.src, I.src_f32, (size_t)(y + q * S) * I.W + (px + k)).w
-                                                    : 1.0f;
-}
-
-// kPairs pairs of this thread: pixels px, px + 1 of image rows y + q S, staged
-// in rows ly + q S (the halo's corner is row 0) at pair column pc.  kOdd: the
-// staged tile holds a value that asks for it.
-template <int S, int R, bool kUnit, int kPairs, bool kOdd>
-VRT_DI void filter_pairs(const float4* sm, const AtrousImage& I, int ne, int pc, int ly, int px, int y,
-                         const float (&alpha)[kPairs][2]) {
-  using G = AtrousGeom<S, R>;
-  CentrePair c[kPairs];
+// This thread's pair: pixels px, px + 1 of image row y, staged at pair column pc of row ly (the halo's corner is
+// row 0).  alpha: their history lengths.  kOdd: the staged tile holds a value that asks for it.
+template <int S, bool kUnit, bool kOdd>
+VRT_DI void filter_pair(const float4* sm, const AtrousImage& I, int pc, int ly, int px, int y, const float (&alpha)[2]) {
+  using G = AtrousGeom<S>;
+  constexpr int ne = G::NE;
+  CentrePair c;
   bool live = false;
-#pragma unroll
-  for (int q = 0; q < kPairs; q++) {
-    const TapPair p = load_pair<kUnit>(sm, ne, (ly + q * S + G::HX) * G::EW + pc + G::HX / 2);
-    c[q].x = p.x; c[q].y = p.y; c[q].z = p.z; c[q].w = p.w; c[q].l = p.l;
+  {
+    const TapPair p = load_pair<kUnit>(sm, ne, (ly + G::HX) * G::EW + pc + G::HX / 2);
+    c.x = p.x; c.y = p.y; c.z = p.z; c.w = p.w; c.l = p.l;
     if (kUnit) {   // a pixel without a normal matches no tap
-      if (c[q].x.x == 0.0f) c[q].x.x = 8.0f;
-      if (c[q].x.y == 0.0f) c[q].x.y = 8.0f;
+      if (c.x.x == 0.0f) c.x.x = 8.0f;
+      if (c.x.y == 0.0f) c.x.y = 8.0f;
     }
     const float cr[2] = {p.r.x, p.r.y}, cg[2] = {p.g.x, p.g.y}, cb[2] = {p.b.x, p.b.y}, gw[2] = {p.w.x, p.w.y};
     float invD[2], invS[2], sr[2], sg[2], sb[2];
 #pragma unroll
     for (int k = 0; k < 2; k++) {
       live = live || !(gw[k] < 0.0f);   // in the image and not sky
-      const float history = fmax_(alpha[q][k], 1.0f);
+      const float history = fmax_(alpha[k], 1.0f);
       const float sigmaL = fmax_(0.08f, 2.0f / __fsqrt_rn(history));
       invD[k] = 1.0f / (0.05f * gw[k] + 0.01f);
       invS[k] = 1.0f / sigmaL;
@@ -251,18 +234,17 @@ VRT_DI void filter_pairs(const float4* sm, const AtrousImage& I, int ne, int pc,
       sg[k] = (cg[k] * 0.375f) * 0.375f;
       sb[k] = (cb[k] * 0.375f) * 0.375f;
     }
-    c[q].invD = f2(invD[0], invD[1]);
-    c[q].invS = f2(invS[0], invS[1]);
-    c[q].sr = f2(sr[0], sr[1]);
-    c[q].sg = f2(sg[0], sg[1]);
-    c[q].sb = f2(sb[0], sb[1]);
-    c[q].ws = f2(0.140625f, 0.140625f);
+    c.invD = f2(invD[0], invD[1]);
+    c.invS = f2(invS[0], invS[1]);
+    c.sr = f2(sr[0], sr[1]);
+    c.sg = f2(sg[0], sg[1]);
+    c.sb = f2(sb[0], sb[1]);
+    c.ws = f2(0.140625f, 0.140625f);
   }
   if (live) {
 #pragma unroll 1
-    for (int j = 0; j < 4 + kPairs; j++) {   // tap rows (j - 2) S of the first pair, (j - 3) S of the second
-      const float w0 = j == 2 ? 0.375f : ((j == 1 || j == 3) ? 0.25f : 0.0625f);
-      const float w1 = j == 3 ? 0.375f : ((j == 2 || j == 4) ? 0.25f : 0.0625f);
+    for (int j = 0; j < 5; j++) {   // tap rows (j - 2) S
+      const float wy = j == 2 ? 0.375f : ((j == 1 || j == 3) ? 0.25f : 0.0625f);
       const int e = (ly + j * S) * G::EW + pc;
       TapPair prev;
 #pragma unroll
@@ -279,61 +261,50 @@ VRT_DI void filter_pairs(const float4* sm, const AtrousImage& I, int ne, int pc,
         } else {
           tp = prev;
         }
-        const float wx = b3_weight(dx);
-        if (j < 5 && (dx != 0 || j != 2)) tap_pair<kUnit, kOdd>(c[0], tp, -(wx * w0));
-        if (kPairs > 1 && j > 0 && (dx != 0 || j != 3)) tap_pair<kUnit, kOdd>(c[kPairs - 1], tp, -(wx * w1));
+        if (dx != 0 || j != 2) tap_pair<kUnit, kOdd>(c, tp, -(b3_weight(dx) * wy));
       }
     }
   }
 #pragma unroll
-  for (int q = 0; q < kPairs; q++) {
-#pragma unroll
-    for (int k = 0; k < 2; k++) {
-      if (px + k >= I.W || y + q * S >= I.H) continue;
-      const size_t i = (size_t)(y + q * S) * I.W + (px + k);
-      float4 v;
-      if ((k ? c[q].w.y : c[q].w.x) < 0.0f) {
-        v = load_px(I.src, I.src_f32, i);   // sky passes through
-      } else {
-        v.w = alpha[q][k];
-        const float den = fmax_(k ? c[q].ws.y : c[q].ws.x, 1e-6f);
-        v.x = (k ? c[q].sr.y : c[q].sr.x) / den;
-        v.y = (k ? c[q].sg.y : c[q].sg.x) / den;
-        v.z = (k ? c[q].sb.y : c[q].sb.x) / den;
-      }
-      I.dst[i] = pack_h4(v.x, v.y, v.z, v.w);
+  for (int k = 0; k < 2; k++) {
+    if (px + k >= I.W || y >= I.H) continue;
+    const size_t i = (size_t)y * I.W + (px + k);
+    float4 v;
+    if ((k ? c.w.y : c.w.x) < 0.0f) {
+      v = load_px(I.src, I.src_f32, i);   // sky passes through
+    } else {
+      v.w = alpha[k];
+      const float den = fmax_(k ? c.ws.y : c.ws.x, 1e-6f);
+      v.x = (k ? c.sr.y : c.sr.x) / den;
+      v.y = (k ? c.sg.y : c.sg.x) / den;
+      v.z = (k ? c.sb.y : c.sb.x) / den;
     }
+    I.dst[i] = pack_h4(v.x, v.y, v.z, v.w);
   }
 }
 
-// The tile at (x0, y0) (multiples of 32 and R); all 8 R threads of the block
-// call it.  sm: AtrousGeom<S, R>::smem bytes.
-template <int S, int R>
+// The tile at (x0, y0) (multiples of 32 and 16); all kAtrousThreads threads of
+// the block call it.  sm: AtrousGeom<S>::smem bytes.
+template <int S>
 VRT_DI void atrous_tile(float4* sm, const AtrousImage& I, int x0, int y0) {
-  using G = AtrousGeom<S, R>;
-  const int t = threadIdx.x, pc = t & 15, rs = t >> 4;
-  // rows ya and ya + S of the tile; their alphas arrive while the tile is staged
-  const int ya = (rs / S) * (2 * S) + rs % S;
-  float alpha[2][2];
-  load_alpha<S, 2>(I, x0 + 2 * pc, y0 + ya, alpha);
-  const int flags = stage_tile<S, R, true>(sm, I, x0 - G::HX, y0 - G::HX, G::EH);
-  const bool odd = __syncthreads_or(flags & kTileOdd) != 0;
+  using G = AtrousGeom<S>;
+  const int pc = threadIdx.x & 15, ly = threadIdx.x >> 4, px = x0 + 2 * pc, y = y0 + ly;
+  float alpha[2];   // arrives while the tile is staged; 1 outside the image
+#pragma unroll
+  for (int k = 0; k < 2; k++)
+    alpha[k] = px + k < I.W && y < I.H ? load_px(I.src, I.src_f32, (size_t)y * I.W + (px + k)).w : 1.0f;
+  int flags = stage_tile<S, true>(sm, I, x0 - G::HX, y0 - G::HX);
+  bool odd = __syncthreads_or(flags & kTileOdd) != 0;
   const bool full = __syncthreads_or(flags & kTileFullNormals) != 0;
   if (!full) {
-    if (!odd) filter_pairs<S, R, true, 2, false>(sm, I, G::NE, pc, ya, x0 + 2 * pc, y0 + ya, alpha);
-    else filter_pairs<S, R, true, 2, true>(sm, I, G::NE, pc, ya, x0 + 2 * pc, y0 + ya, alpha);
+    if (!odd) filter_pair<S, true, false>(sm, I, pc, ly, px, y, alpha);
+    else filter_pair<S, true, true>(sm, I, pc, ly, px, y, alpha);
     return;
   }
-  for (int half = 0; half < 2; half++) {   // R / 2 rows, one pair per thread
-    const int yh = y0 + (R / 2) * half;
-    const int f = stage_tile<S, R, false>(sm, I, x0 - G::HX, yh - G::HX, G::HH);
-    const bool oddh = __syncthreads_or(f & kTileOdd) != 0;
-    float a1[1][2];
-    load_alpha<S, 1>(I, x0 + 2 * pc, yh + rs, a1);
-    if (!oddh) filter_pairs<S, R, false, 1, false>(sm, I, G::HE, pc, rs, x0 + 2 * pc, yh + rs, a1);
-    else filter_pairs<S, R, false, 1, true>(sm, I, G::HE, pc, rs, x0 + 2 * pc, yh + rs, a1);
-    __syncthreads();   // the half's taps are read before the next half is staged
-  }
+  flags = stage_tile<S, false>(sm, I, x0 - G::HX, y0 - G::HX);
+  odd = __syncthreads_or(flags & kTileOdd) != 0;
+  if (!odd) filter_pair<S, false, false>(sm, I, pc, ly, px, y, alpha);
+  else filter_pair<S, false, true>(sm, I, pc, ly, px, y, alpha);
 }
 
 }  // namespace vrt

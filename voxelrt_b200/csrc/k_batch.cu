@@ -42,37 +42,32 @@ __global__ void __launch_bounds__(256) k_b_temporal(MultiJob J, uint32_t P) {
 
 // atrous.wgsl:26-83 iteration `it` (step 1 << it) of every job whose denoise
 // flag is set; chain accum -> dA -> dB -> dA (main.js:503-507).  A CTA computes
-// one 32 x 32 tile of one job (atrous_tile.cuh), whatever the views' sizes: the
-// jobs' tiles fill the GPU together, as those of one large image.  tiles: m + 1
-// prefix counts of the jobs' tiles, in which CTA b finds its job.
-constexpr int kBatchRows = 32;   // tile rows
+// one tile of one job (atrous_tile.cuh).  tiles: m + 1 prefix counts of the jobs'
+// tiles, in which CTA b finds its job.
 template <int S>
-__global__ void __launch_bounds__(8 * kBatchRows, 96 / kBatchRows) k_b_atrous(MultiJob J,
-                                                                             const uint32_t* __restrict__ tiles) {
+__global__ void __launch_bounds__(kAtrousThreads, kAtrousBlocks) k_b_atrous(MultiJob J, const uint32_t* __restrict__ tiles) {
   frame_begin();
   extern __shared__ float4 sm[];
   const uint32_t b = blockIdx.x;
   const int lo = last_at_or_before(tiles, J.n, b);
   const JobDev& jd = J.jobs[lo];
   if ((jd.u.params0[2] & 2u) == 0u) return;
-  const int tb = (int)(b - __ldg(tiles + lo)), tw = (jd.W + kAtrousTile - 1) / kAtrousTile;
+  const int tb = (int)(b - __ldg(tiles + lo)), tw = (jd.W + kAtrousW - 1) / kAtrousW;
   const void* src = S == 1 ? jd.acc_cur : (S == 2 ? (const void*)jd.den0 : (const void*)jd.den1);
   uint2* dst = S == 2 ? jd.den1 : jd.den0;
-  const int x0 = (tb % tw) * kAtrousTile, y0 = (tb / tw) * kBatchRows;
+  const int x0 = (tb % tw) * kAtrousW, y0 = (tb / tw) * kAtrousH;
   // one copy of the filter for each type of history, as for a single view
-  if (S == 1 && jd.acc_f32 != 0)
-    atrous_tile<S, kBatchRows>(sm, AtrousImage{jd.W, jd.H, src, true, jd.out.gbuf, dst}, x0, y0);
-  else
-    atrous_tile<S, kBatchRows>(sm, AtrousImage{jd.W, jd.H, src, false, jd.out.gbuf, dst}, x0, y0);
+  if (S == 1 && jd.acc_f32 != 0) atrous_tile<S>(sm, AtrousImage{jd.W, jd.H, src, true, jd.out.gbuf, dst}, x0, y0);
+  else atrous_tile<S>(sm, AtrousImage{jd.W, jd.H, src, false, jd.out.gbuf, dst}, x0, y0);
 }
 
 template <int S>
 static cudaError_t launch_b_atrous(const MultiJob& J, const AtrousTiles& at, cudaStream_t st) {
-  using G = AtrousGeom<S, kBatchRows>;
+  using G = AtrousGeom<S>;
   const cudaError_t e =
       cudaFuncSetAttribute(k_b_atrous<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, G::smem);
   if (e != cudaSuccess) return e;
-  launch_after(k_b_atrous<S>, at.n, G::threads, G::smem, st, J, at.first);
+  launch_after(k_b_atrous<S>, at.n, kAtrousThreads, G::smem, st, J, at.first);
   return cudaGetLastError();
 }
 

@@ -1289,12 +1289,12 @@ static int batch_frame_impl(VrtBatch* b, const int* idx, int m, const VrtUniform
   }
   const uint32_t P = first;
   if (P > b->P) return fail(VRT_ERR_INVALID, "batch frame of %u pixels exceeds the pool's %u", P, b->P);
-  // a-trous tile table: prefix counts of each job's 32 x 32 tiles
+  // a-trous tile table: prefix counts of each job's tiles
   uint32_t* tiles = b->h_firsts + n;
   tiles[0] = 0u;
   for (int i = 0; i < m; i++) {
     const VrtSession* s = ss[(size_t)i];
-    tiles[i + 1] = tiles[i] + (uint32_t)((s->W + 31) / 32) * (uint32_t)((s->H + 31) / 32);
+    tiles[i + 1] = tiles[i] + atrous_tiles(s->W, s->H);
   }
   const AtrousTiles at{b->d_firsts + n, tiles[m]};
   CUDA_TRY(cudaMemcpyAsync(b->d_jobs, b->h_jobs, (size_t)m * sizeof(JobHost), cudaMemcpyHostToDevice, st));

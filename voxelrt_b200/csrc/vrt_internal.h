@@ -108,7 +108,7 @@ struct WavefrontTuning {
   int shade_blocks_per_sm = 32;
   int trace_variant = 0;        // shape of the tracer (wf_dispatch_trace): (transition rounds per
                                 // warp-bookkeeping pass, steps per round, min blocks/SM)
-  int atrous_rows = 0;          // kept from the caller's tuning; the a-trous tiles go by the image's size
+  int atrous_rows = 0;          // kept from the caller's tuning; the a-trous tiles have one shape
   int tail_wave = -1;           // first wave whose paths finish one thread each (k_wf_tail); 0 = never;
                                 // -1 = automatic (auto_tail in wavefront_core.cuh)
 };
@@ -141,8 +141,10 @@ struct JobHost {
   CacheDev cache;
 };
 
-// The batch a-trous tile table: the prefix counts of the jobs' 32 x 32 output tiles (m + 1 entries in
-// device memory) and their total.
+// Tiles of 32 x 16 pixels of a W x H image (atrous_tile.cuh).
+inline uint32_t atrous_tiles(int W, int H) { return (uint32_t)((W + 31) / 32) * (uint32_t)((H + 15) / 16); }
+// The batch a-trous tile table: the prefix counts of the jobs' tiles (m + 1 entries in device memory) and their
+// total.
 struct AtrousTiles {
   const uint32_t* first;
   uint32_t n;
