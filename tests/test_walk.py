@@ -330,3 +330,26 @@ def test_tracer_variants_leave_the_image(vrt, ctx, variant):
     batch.close()
     for o in (mega, wave, view, sc):
         o.close()
+
+
+@pytest.mark.parametrize("n", [8, 24, 104])
+def test_edits_keep_the_bitmap(vrt, ctx, n):
+    """A world after boxes of voxels were set and cleared, bricks at its edges among them, answers rays as a world
+    uploaded with those voxels does, and as one uploaded with its bricks and masks."""
+    r = np.random.default_rng(n)
+    sc = vrt.Scene(ctx, np.zeros(n ** 3, np.uint32), n)
+    o, d, t = _odd_rays(4000, n / 16.0, n)
+    for k in range(24):
+        lo = r.integers(0, n, 3)
+        hi = np.minimum(lo + r.integers(0, 20, 3), n - 1)
+        if k % 6 == 5:                       # whole bricks, the world's first or last
+            lo = np.zeros(3, int) if k % 12 == 5 else np.full(3, n - 8)
+            hi = lo + 7
+        sc.edit_box(*map(int, lo), *map(int, hi), 0 if k % 3 == 2 else int(r.integers(1, 1 << 32)))
+        if k % 4 == 3:
+            v, b, m = sc.read()
+            want = sc.trace_rays(o, d, t).tobytes()
+            for other in (vrt.Scene(ctx, v, n), vrt.Scene(ctx, v, n, b, m)):
+                assert other.trace_rays(o, d, t).tobytes() == want
+                other.close()
+    sc.close()

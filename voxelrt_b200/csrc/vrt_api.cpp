@@ -275,7 +275,7 @@ static int scene_alloc(VrtCtx* ctx, int N, VrtScene** out) {
     g_err = keep;
     return r;
   }
-  // full masks everywhere; building or uploading the bricks overwrites all but the border
+  // full masks and set bits everywhere; building or uploading the bricks overwrites all but the border
   const cudaError_t e = cudaMemsetAsync(s->dev.cells, 0xff, cell_bytes(s->dev.BG), ctx->stream);
   if (e != cudaSuccess) {
     vrt_scene_destroy(s);
@@ -310,7 +310,6 @@ int vrt_scene_upload(VrtCtx* ctx, const uint32_t* voxels, int N, VrtScene** out)
   cudaStream_t st = ctx->stream;
   cudaError_t e = cudaMemcpyAsync(s->dev.vox, voxels, nv * 4, cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess) e = launch_build_bricks(s->dev, 0, 0, 0, s->dev.BG - 1, s->dev.BG - 1, s->dev.BG - 1, st);
-  if (e == cudaSuccess) e = launch_build_bits(s->dev, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) {
     vrt_scene_destroy(s);
@@ -353,7 +352,6 @@ int vrt_scene_edit_box(VrtScene* s, int x0, int y0, int z0, int x1, int y1, int 
   cudaStream_t st = s->ctx->stream;
   CUDA_TRY(launch_fill_box(s->dev, x0, y0, z0, x1, y1, z1, value, st));
   CUDA_TRY(launch_build_bricks(s->dev, x0 / 8, y0 / 8, z0 / 8, x1 / 8, y1 / 8, z1 / 8, st));
-  CUDA_TRY(launch_build_bits(s->dev, st));
   return VRT_OK;
 }
 
@@ -2307,7 +2305,6 @@ int vrt_session_restore(VrtSession* s, const void* host, uint64_t bytes) {
   CUDA_TRY(h2d(s->scene->dev.vox, N * N * N * 4));
   const int BG = s->scene->dev.BG;
   CUDA_TRY(launch_build_bricks(s->scene->dev, 0, 0, 0, BG - 1, BG - 1, BG - 1, st));
-  CUDA_TRY(launch_build_bits(s->scene->dev, st));
   s->scene->lights_built = false;
   for (int i = 0; i < 2; i++) CUDA_TRY(h2d(s->accum[i], P * acc_bpp(s)));
   for (int i = 0; i < 2; i++) CUDA_TRY(h2d(s->gbuf[i], P * 16));

@@ -263,7 +263,7 @@ cudaError_t launch_wavefront(const SceneDev& s, const VrtUniforms& u, float fcla
 
 cudaError_t launch_build_bricks(const SceneDev& s, int bx0, int by0, int bz0, int bx1, int by1, int bz1,
                                 cudaStream_t st);
-// The padded occupancy bitmap from the brick words.
+// The whole padded occupancy bitmap from the brick words (launch_build_bricks sets the bits of its bricks).
 cudaError_t launch_build_bits(const SceneDev& s, cudaStream_t st);
 cudaError_t launch_fill_box(const SceneDev& s, int x0, int y0, int z0, int x1, int y1, int z1, uint32_t value,
                             cudaStream_t st);
