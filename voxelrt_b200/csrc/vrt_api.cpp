@@ -400,11 +400,17 @@ int vrt_trace_rays_device(VrtScene* s, const float* o, const float* d, const flo
 
 constexpr int kRayStage = 16384;   // rays of the staged path (1.2 MB of pinned memory per context)
 
-// Whether the host itself can read and write p (the runtime knows it as no device allocation).
-static bool host_memory(const void* p) {
-  cudaPointerAttributes at;
-  return cudaPointerGetAttributes(&at, p) == cudaSuccess && at.type != cudaMemoryTypeDevice;
+// What the runtime knows p as; a pointer that it cannot tell counts as unregistered, and leaves no error behind.
+static cudaPointerAttributes pointer_kind(const void* p) {
+  cudaPointerAttributes at = {};
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    cudaGetLastError();
+    at = {};
+  }
+  return at;
 }
+// Whether the host itself can read and write p.
+static bool host_memory(const void* p) { return pointer_kind(p).type != cudaMemoryTypeDevice; }
 
 int vrt_trace_rays(VrtScene* s, const float* o, const float* d, const float* tmax, int n, VrtHit* out) {
   if (!s || n < 0) return fail(VRT_ERR_INVALID, "bad argument");
@@ -2071,8 +2077,7 @@ int vrt_mlp_gradient_device(VrtMlp* m, const float* d_q9, const float* d_y3, int
   // array (misaligned, on the host, on another device) takes a copy, which accepts or refuses it.
   bool direct = false;
   if (d_grad && ((uintptr_t)d_grad & 3u) == 0u) {
-    cudaPointerAttributes at;
-    CUDA_TRY(cudaPointerGetAttributes(&at, d_grad));
+    const cudaPointerAttributes at = pointer_kind(d_grad);
     direct = at.type == cudaMemoryTypeDevice && at.device == m->ctx->device;
   }
   if (int r = mlp_grad_impl(m, d_q9, d_y3, n, extent, direct ? d_grad : m->grad, loss_out, false)) return r;
