@@ -217,7 +217,10 @@ __device__ __forceinline__ void store_row_relu(uint8_t* tile, int row, int C, co
 // stored as 0, since the backward pass takes the ReLU's derivative from here.  The added
 // half of bf16's least value (2^-134) sees to that: it lifts every positive h over
 // the tie and leaves 0 on it (rounded to even, 0), and above 2^-109 it is lost
-// in the sum.
+// in the sum; below that a value may round up that would have rounded down.
+// (Lifting only the positive values that would be 0, found by the least pattern
+// of the row: bit for bit the rounding without the sum, but a call of 983 K
+// samples 247 -> 261 us.)
 __device__ __forceinline__ void store_row_hidden(uint8_t* tile, int row, const float* v) {
   const float2 half = make_float2(0x1p-134f, 0x1p-134f);
   const __nv_bfloat162 zero = __floats2bfloat162_rn(0.0f, 0.0f);
